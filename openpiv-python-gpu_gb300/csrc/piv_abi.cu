@@ -124,6 +124,7 @@ struct IterState {
   uint8_t* near_tie = nullptr;  // per window: near tie of the correlation peak
   void* s2n = nullptr;
   uint8_t* field_mask = nullptr;
+  void* smooth_tables = nullptr;  // constants of this pass's smoothing
   // Correlation launch variant (0 = default; set by piv_plan_autotune or
   // piv_plan_set_variant), the pass's arguments of the last run, and the
   // autotuner's per-variant times (ms, -1 = not timed).
@@ -388,6 +389,10 @@ int piv_plan_create(const piv_config* cfg, piv_plan** out) {
     if (k < cfg->n_iters - 1) {
       if ((rc = plan_alloc_t(p, &s.u_out, cnt))) break;
       if ((rc = plan_alloc_t(p, &s.v_out, cnt))) break;
+      if (s.mn >= 2) {
+        if ((rc = plan_alloc(p, &s.smooth_tables, smooth_tables_bytes(s.g.m, s.g.n)))) break;
+        if ((rc = smooth_tables_build(s.g.m, s.g.n, s.smooth_tables, nullptr))) break;
+      }
     } else {
       s.u_out = s.u_rep;
       s.v_out = s.v_rep;
@@ -457,6 +462,11 @@ int piv_plan_create(const piv_config* cfg, piv_plan** out) {
     rc = plan_alloc_t(p, &p->outliers, cnt);
     if (rc == PIV_OK) rc = plan_alloc_t(p, &p->u_final, cnt);
     if (rc == PIV_OK) rc = plan_alloc_t(p, &p->v_final, cnt);
+  }
+  // The smoothing tables are complete before a run on any stream reads them.
+  if (rc == PIV_OK && cfg->n_iters > 1) {
+    const cudaError_t e = cudaStreamSynchronize(nullptr);
+    if (e != cudaSuccess) rc = set_cuda_error(e, "plan tables");
   }
   if (rc != PIV_OK) {
     piv_plan_destroy(p);
@@ -718,7 +728,7 @@ static int run_post(piv_plan* p, int k, RunCtx& x, cudaStream_t s) {
   mark(p, x, k * PIV_STAGES + 4, s);
   if (k != n_it - 1) {
     PIV_TRY(smoothn(st.g.m, st.g.n, n_pairs, st.u_rep, st.v_rep, st.u_out, st.v_out, st.field_mask,
-                    it.smoothing_par, st.smooth_p, p->smooth_scratch, s, st.smooth_flags));
+                    it.smoothing_par, st.smooth_p, p->smooth_scratch, s, st.smooth_flags, st.smooth_tables));
     mark(p, x, k * PIV_STAGES + 5, s);
   }
   return PIV_OK;

@@ -190,7 +190,12 @@ size_t smoothn_scratch_bytes(int m, int n, int n_pairs);
 // flags (device [n_pairs], may be NULL) receives the PIV_SMOOTH_* bits of each pair.
 int smoothn(int m, int n, int n_pairs, const double* u_in, const double* v_in, double* u_out, double* v_out,
             const uint8_t* field_mask, double s, double* p_out, void* scratch, cudaStream_t stream,
-            int* flags = nullptr);
+            int* flags = nullptr, const void* tables = nullptr);
+// The constant tables of an m x n field (cosine matrices, lambda^2), which a
+// plan builds once and hands to every smoothn; without them smoothn builds
+// what it needs in its scratch.
+size_t smooth_tables_bytes(int m, int n);
+int smooth_tables_build(int m, int n, void* tables, cudaStream_t stream);
 
 // Final scaling u * scaling_par / dt (gpu_process.py:847-849).
 int scale_fields(int count, const double* u, const double* v, double scaling, double dt, int fp32, double* uo,

@@ -9,8 +9,13 @@
 // finite-difference gradient is below 1e-5 (the stopping test of the
 // reference's L-BFGS-B call, gpu_smoothn.py:191-193).
 //
-// The orthonormal DCT-II/III pairs are float64 matrix products with cosine
-// matrices built on the device; the GCV search runs in one CTA per pair.
+// The orthonormal DCT-II/III pairs are matrix products with cosine matrices
+// built on the device. The GCV search and the weighted iteration of one pair
+// run on one CTA or, when the pairs leave SMs idle, on a cluster of up to
+// eight (cluster_size): float64 has 1/64 of the float32 rate here, so a
+// search on one SM is bound by that SM's float64 pipe. The sums are formed by
+// kVT virtual threads in the same order whatever the cluster size, so the
+// results do not depend on it, bit for bit.
 #include <math.h>
 
 #include <mutex>
@@ -21,25 +26,32 @@
 
 namespace piv {
 
+// Constant tables of an m x n field.
+struct SmoothTables {
+  double* cm;    // [m][m] DCT-II matrix (lines too long for the staged kernels)
+  double* cn;    // [n][n]
+  float* cmf;    // [2][m][m] cm as hi/lo floats
+  float* cnf;    // [2][n][n]
+  float2* cm2;   // weighted path: [m][m] cm as (hi, lo)
+  float2* cn2;   // [n][n]
+  float2* cnt2;  // [n][n] the transpose of cn2
+  double* lam2;  // [mn] lambda^2
+  float* lam2f;  // [mn] lambda^2 in float32 (the GCV scan's fast score)
+};
+
 struct SmoothScratch {
   double* fd;    // [pairs][2][mn] DCT coefficients of u and v
   double* tmp;   // [pairs][2][mn]
   double* f2;    // [pairs][mn] fd_u^2 + fd_v^2
-  double* cm;    // [m][m]
-  double* cn;    // [n][n]
-  double* lam2;  // [mn]
-  double* p;     // [pairs]
+  double* s;     // [pairs] 10^p
   float* f2f;    // [pairs][mn] f2 in float32 (the GCV search's fast score)
-  float* lam2f;  // [mn] lam2 in float32
-  float* cmf;    // [2][m][m] cm as hi/lo floats (the DCT lines' double-float products)
-  float* cnf;    // [2][n][n]
+  SmoothTables t;
 };
 
 static size_t align_up(size_t v) { return (v + 255) / 256 * 256; }
 
-// Per-pair block of the weighted path: f, z, t, fd, tmp (2 mn doubles each),
-// w (mn doubles), the column-nearest table (mn ints) and the hi/lo float
-// split of a DCT input (2 mn floats).
+// Per-pair block of the weighted path: f, z, z', fd, tmp (2 mn doubles each),
+// w (mn doubles), the column-nearest table (mn ints) and 2 mn spare floats.
 static size_t weighted_pair_bytes(size_t mn) { return align_up(11 * mn * 8 + mn * 4 + 2 * mn * 4); }
 // The DCT matrices of the weighted path as hi/lo float pairs (2 (m^2 + n^2) floats).
 static size_t weighted_matrix_bytes(int m, int n) { return align_up(2 * ((size_t)m * m + (size_t)n * n) * 4); }
@@ -67,49 +79,223 @@ static SmoothScratch carve(void* base, int m, int n, int n_pairs) {
   s.fd = (double*)p; p += align_up(2 * mn * n_pairs * 8);
   s.tmp = (double*)p; p += align_up(2 * mn * n_pairs * 8);
   s.f2 = (double*)p; p += align_up(mn * n_pairs * 8);
-  s.cm = (double*)p; p += align_up((size_t)m * m * 8);
-  s.cn = (double*)p; p += align_up((size_t)n * n * 8);
-  s.lam2 = (double*)p; p += align_up(mn * 8);
-  s.p = (double*)p; p += align_up((size_t)n_pairs * 8);
+  s.t.cm = (double*)p; p += align_up((size_t)m * m * 8);
+  s.t.cn = (double*)p; p += align_up((size_t)n * n * 8);
+  s.t.lam2 = (double*)p; p += align_up(mn * 8);
+  s.s = (double*)p; p += align_up((size_t)n_pairs * 8);
   s.f2f = (float*)p; p += align_up(mn * n_pairs * 4);
-  s.lam2f = (float*)p; p += align_up(mn * 4);
-  s.cmf = (float*)p; p += align_up((size_t)m * m * 8);
-  s.cnf = (float*)p;
+  s.t.lam2f = (float*)p; p += align_up(mn * 4);
+  s.t.cmf = (float*)p; p += align_up((size_t)m * m * 8);
+  s.t.cnf = (float*)p;
+  s.t.cm2 = s.t.cn2 = s.t.cnt2 = nullptr;
   return s;
 }
 
-// Orthonormal DCT-II matrix C[k][i] = s_k cos(pi (2i+1) k / (2 len)).
-__global__ void k_dct_matrix(int len, double* c) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= len * len) return;
-  const int k = t / len, i = t % len;
-  const double sk = k == 0 ? sqrt(1.0 / len) : sqrt(2.0 / len);
-  c[t] = sk * cospi((double)((2 * i + 1) * k) / (2.0 * len));
+// The constant tables, one thread per entry: the orthonormal DCT-II matrices
+// C[k][i] = s_k cos(pi (2i+1) k / (2 len)) and lambda^2 with lambda =
+// 2 (2 - (cos(pi i/m) + cos(pi j/n))); NULL tables are left out. One launch
+// where five small ones (two matrices, their splits, lambda^2) took 33 us of a
+// 127 x 127 smoothing.
+__global__ void k_smooth_tables(int m, int n, SmoothTables t) {
+  const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long mm = (long long)m * m, nn = (long long)n * n, mn = (long long)m * n;
+  if (id < mm + nn) {
+    const bool rows = id >= mm;  // the matrix of the transform along the rows
+    const int len = rows ? n : m;
+    const long long e = rows ? id - mm : id;
+    const int k = (int)(e / len), i = (int)(e % len);
+    const double sk = k == 0 ? sqrt(1.0 / len) : sqrt(2.0 / len);
+    const double c = sk * cospi((double)((2 * i + 1) * k) / (2.0 * len));
+    double* cd = rows ? t.cn : t.cm;
+    float* cf = rows ? t.cnf : t.cmf;
+    const long long ll = rows ? nn : mm;
+    const float h = (float)c, l = (float)(c - (double)h);
+    if (cd) cd[e] = c;
+    if (cf) {
+      cf[e] = h;
+      cf[ll + e] = l;
+    }
+    float2* c2 = rows ? t.cn2 : t.cm2;
+    if (c2) c2[e] = make_float2(h, l);
+    if (rows && t.cnt2) t.cnt2[(long long)i * n + k] = make_float2(h, l);
+  } else if (id < mm + nn + mn) {
+    const long long e = id - mm - nn;
+    const int i = (int)(e / n), j = (int)(e % n);
+    const double l = 2.0 * (2.0 - (cos(M_PI * i / m) + cos(M_PI * j / n)));
+    t.lam2[e] = l * l;
+    if (t.lam2f) t.lam2f[e] = (float)(l * l);
+  }
 }
 
-// lambda^2 with lambda = 2 (2 - (cos(pi i/m) + cos(pi j/n))).
-__global__ void k_lambda2(int m, int n, double* lam2, float* lam2f = nullptr) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= m * n) return;
-  const int i = t / n, j = t % n;
-  const double l = 2.0 * (2.0 - (cos(M_PI * i / m) + cos(M_PI * j / n)));
-  lam2[t] = l * l;
-  if (lam2f) lam2f[t] = (float)(l * l);
+static int check(const char* what) {
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? PIV_OK : set_cuda_error(e, what);
 }
+
+#define PIV_RC(expr)               \
+  do {                             \
+    const int rc_ = (expr);        \
+    if (rc_ != PIV_OK) return rc_; \
+  } while (0)
+
+static int build_tables(int m, int n, const SmoothTables& t, cudaStream_t stream) {
+  const long long total = (long long)m * m + (long long)n * n + (long long)m * n;
+  k_smooth_tables<<<(unsigned)((total + 127) / 128), 128, 0, stream>>>(m, n, t);
+  return check("k_smooth_tables");
+}
+
+// Tables that a plan keeps (every table, whichever path its runs take).
+size_t smooth_tables_bytes(int m, int n) {
+  const size_t mm = (size_t)m * m * 8, nn = (size_t)n * n * 8, mn = (size_t)m * n;
+  return 3 * align_up(mm) + 4 * align_up(nn) + align_up(mn * 8) + align_up(mn * 4);
+}
+
+static SmoothTables kept_tables(const void* base, int m, int n) {
+  const size_t mm = (size_t)m * m * 8, nn = (size_t)n * n * 8, mn = (size_t)m * n;
+  char* p = (char*)const_cast<void*>(base);
+  SmoothTables t;
+  t.cm = (double*)p; p += align_up(mm);
+  t.cn = (double*)p; p += align_up(nn);
+  t.cmf = (float*)p; p += align_up(mm);
+  t.cnf = (float*)p; p += align_up(nn);
+  t.cm2 = (float2*)p; p += align_up(mm);
+  t.cn2 = (float2*)p; p += align_up(nn);
+  t.cnt2 = (float2*)p; p += align_up(nn);
+  t.lam2 = (double*)p; p += align_up(mn * 8);
+  t.lam2f = (float*)p;
+  return t;
+}
+
+int smooth_tables_build(int m, int n, void* base, cudaStream_t stream) {
+  return build_tables(m, n, kept_tables(base, m, n), stream);
+}
+
+// ---------------------------------------------------------------------------
+// Clusters of CTAs that share one pair's sums.
+// ---------------------------------------------------------------------------
+static constexpr int kVT = 512;         // virtual threads of a pair's sums
+static constexpr int kVW = kVT / 32;    // virtual warps
+
+PIV_D unsigned cluster_rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// Barrier of every thread of the cluster; orders shared and global memory.
+PIV_D void cluster_barrier(int c) {
+  if (c == 1) {
+    __syncthreads();
+  } else {
+    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+  }
+}
+// Stores v at *p (this CTA's shared memory) of CTA `rank` of the cluster.
+PIV_D void st_cluster(double* p, unsigned rank, double v) {
+  asm volatile(
+      "{\n.reg .u32 a;\nmapa.shared::cluster.u32 a, %0, %1;\nst.shared::cluster.f64 [a], %2;\n}\n" ::"r"(
+          (unsigned)__cvta_generic_to_shared(p)),
+      "r"(rank), "d"(v)
+      : "memory");
+}
+
+// CTAs per pair: the largest power of two up to 8 (the portable cluster size)
+// that keeps every CTA on an SM of its own (with more pairs than that the
+// float64 pipes are busy anyway). Measured: one pair's two GCV searches of a
+// three-pass 1024 x 1024 run 396 -> 157 us with 8 CTAs, those of 64 pairs
+// 230 -> 86 us with 2.
+static int cluster_size(int n_pairs) {
+  int c = 1;
+  while (c < 8 && (long long)n_pairs * c * 2 <= sm_count()) c *= 2;
+  return c;
+}
+
+template <typename... P, typename... A>
+static int launch_cluster(void (*kernel)(P...), int n_pairs, int c, int threads, cudaStream_t stream, const char* what,
+                          A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)n_pairs * (unsigned)c);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)c;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  return e == cudaSuccess ? PIV_OK : set_cuda_error(e, what);
+}
+
+// Sums over the warp of K values per lane, the sum of x[l] left in lane l: the
+// xor tree (16, 8, 4, 2, 1) of a full warp sum per value, but each level
+// halves the values a lane still carries (31 additions for up to 32 values
+// instead of 5 per value; the additions pair the same lanes, so the sums are
+// the same bit for bit).
+template <int K, typename T>
+PIV_D double warp_sums(const T (&x)[K]) {
+  static_assert(K <= 32, "one value per lane");
+  const int lane = threadIdx.x & 31;
+  double v[16];
+  {
+    const bool up = lane & 16;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const T lo = i < K ? x[i] : (T)0, hi = i + 16 < K ? x[i + 16] : (T)0;
+      const T other = __shfl_xor_sync(~0u, up ? lo : hi, 16);
+      v[i] = (double)(up ? hi : lo) + (double)other;
+    }
+  }
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < o; ++i) {
+      const double other = __shfl_xor_sync(~0u, up ? v[i] : v[i + o], o);
+      v[i] = (up ? v[i + o] : v[i]) + other;
+    }
+  }
+  return v[0];
+}
+
+// warp_sums of four values: two levels that halve the values, then the tree;
+// the sum of x[k] is in the lanes whose bits 4 and 3 are k's bits 1 and 0.
+PIV_D double warp_sums4(double x0, double x1, double x2, double x3) {
+  const int lane = threadIdx.x & 31;
+  const bool u16 = lane & 16, u8 = lane & 8;
+  double a = (u16 ? x2 : x0) + __shfl_xor_sync(~0u, u16 ? x0 : x2, 16);
+  double b = (u16 ? x3 : x1) + __shfl_xor_sync(~0u, u16 ? x1 : x3, 16);
+  double v = (u8 ? b : a) + __shfl_xor_sync(~0u, u8 ? a : b, 8);
+  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(~0u, v, o);
+  return v;
+}
+
+// Fields of a DCT pass: component c of pair k at (c ? v : u) + k * stride.
+struct DctIo {
+  double* u;
+  double* v;
+  long long stride;
+  PIV_D double* field(long long f) const { return ((f & 1) ? v : u) + (f >> 1) * stride; }
+};
+// The factor 1 / (1 + s lambda^2) on the inputs of the inverse row pass (lam2
+// NULL: none); s of pair k at s[k].
+struct DctGamma {
+  const double* lam2;
+  const double* s;
+};
 
 // out[b][i][l] = sum_j in[b][i][j] * c[l][j]       (transform along rows, mode 0)
 // out[b][i][l] = sum_j in[b][i][j] * c[j][l]       (inverse along rows, mode 1)
 // out[b][k][j] = sum_i c[k][i] * in[b][i][j]       (transform along columns, mode 2)
 // out[b][k][j] = sum_i c[i][k] * in[b][i][j]       (inverse along columns, mode 3)
-__global__ void k_dct_apply(int m, int n, int batch, int mode, const double* __restrict__ c,
-                            const double* __restrict__ in, double* __restrict__ out) {
+// Lines beyond the staged kernels' shared memory (kDctLongLen) only.
+__global__ void k_dct_apply(int m, int n, int batch, int mode, const double* __restrict__ c, DctIo in, DctIo out) {
   const long long mn = (long long)m * n;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= mn * batch) return;
-  const int b = (int)(t / mn);
+  const long long b = t / mn;
   const int e = (int)(t % mn);
   const int r = e / n, col = e % n;
-  const double* x = in + b * mn;
+  const double* x = in.field(b);
   double acc = 0.0;
   if (mode == 0) {
     for (int j = 0; j < n; ++j) acc = fma(x[r * n + j], c[col * n + j], acc);
@@ -120,24 +306,7 @@ __global__ void k_dct_apply(int m, int n, int batch, int mode, const double* __r
   } else {
     for (int i = 0; i < m; ++i) acc = fma(c[i * m + r], x[i * n + col], acc);
   }
-  out[t] = acc;
-}
-
-// The orthonormal DCT-II matrix has C[k][L-1-i] = (-1)^k C[k][i], so along a
-// line of length L the forward transform needs only the sums x[i] + x[L-1-i]
-// (even k) or differences (odd k) of the first L/2 positions, and the inverse
-// gives x[i] and x[L-1-i] from one pass over the even and the odd k: half the
-// float64 multiply-adds of the plain product. One CTA takes 32 lines staged
-// in shared memory as [position][line]; `cols` selects lines along the
-// columns of the [m][n] fields (stride n) instead of along the rows.
-// Lines up to 90 long keep the staging under the default 48 KB of shared memory.
-// x -> (hi, lo) float pairs: hi = (float)x, lo = (float)(x - hi).
-__global__ void k_split_f64(int count, const double* __restrict__ x, float* __restrict__ hi, float* __restrict__ lo) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= count) return;
-  const float h = (float)x[t];
-  hi[t] = h;
-  lo[t] = (float)(x[t] - (double)h);
+  out.field(b)[e] = acc;
 }
 
 // Dot product of two hi/lo float vectors in float32 with error-free
@@ -161,75 +330,142 @@ struct DfAcc {
   }
 };
 
+// 1/d for d >= 1 from the float32 reciprocal and two Newton steps in float64:
+// within an ulp or two of the rounded quotient, at a fraction of the cost of
+// a float64 division (float64 throughput on this GPU is low).
+PIV_D double rcp_fast(double d) {
+  double r = (double)__frcp_rn((float)d);
+  double e = fma(-d, r, 1.0);
+  r = fma(r, e, r);
+  e = fma(-d, r, 1.0);
+  return fma(r, e, r);
+}
+
 static constexpr int kDctLines = 32, kDctThreads = 256, kDctMaxLen = 90;
+static constexpr int kDctLongLen = 860;  // 33 doubles per position: 227 KB
 
 // DCT-II (or, INV, DCT-III) of kDctLines lines per CTA with the symmetric
-// split of the cosine matrix (half the products). The products are
-// double-float (DfAcc: hi/lo float pairs with error-free transformations,
-// within ~1e-13 of float64); cf holds the matrix as [2][L][L] hi/lo floats.
-template <bool INV>
+// split of the cosine matrix: C[k][L-1-i] = (-1)^k C[k][i], so the forward
+// transform needs only the sums x[i] + x[L-1-i] (even k) or differences (odd
+// k) of the first L/2 positions, and the inverse gives x[i] and x[L-1-i] from
+// one pass over the even and the odd k: half the products. The lines are
+// staged in shared memory as [position][line]; `cols` selects lines along the
+// columns of the [m][n] fields instead of along the rows. blockIdx.y takes a
+// share of the outputs, so that a few lines still fill the SMs (one pair of
+// 63 x 63 has 126 lines, 4 CTAs).
+// DF: double-float products (DfAcc: hi/lo float pairs with error-free
+// transformations, within ~1e-13 of float64) with cf the matrix as [2][L][L]
+// hi/lo floats; else float64 products with cd, which the float64 pipe bounds.
+template <bool INV, bool DF>
 __global__ void __launch_bounds__(kDctThreads) k_dct_lines(int m, int n, int batch, int cols, const float* __restrict__ cf,
-                                                           const double* __restrict__ in, double* __restrict__ out) {
+                                                           const double* __restrict__ cd, DctIo in, DctIo out,
+                                                           DctGamma gam) {
   extern __shared__ double dsm[];
   const int L = cols ? m : n;
-  const long long mn = (long long)m * n;
   const long long n_lines = (long long)batch * (cols ? n : m);
   const long long l0 = (long long)blockIdx.x * kDctLines;
   constexpr int S = kDctLines + 1;           // odd stride: conflict-free rows of 32 lines
   double* xs = dsm;                          // [L][S] doubles
   const int h = L / 2, hc = (L + 1) / 2;
-  float* fs = reinterpret_cast<float*>(dsm + L * S);  // 4 hc S floats after xs
+  float* fs = reinterpret_cast<float*>(dsm + L * S);  // DF: 4 hc S floats after xs
   const float* ch = cf;
   const float* cl = cf + (size_t)L * L;
-  auto addr = [&](long long line, int e) -> long long {
-    if (cols) {
-      const long long f = line / n, col = line % n;
-      return f * mn + (long long)e * n + col;
-    }
-    return line * n + e;
-  };
+  // Field and first element of a line, and the step between its elements.
+  const int per = cols ? n : m;  // lines per field
+  const int step = cols ? n : 1;
   // Load: coalesced along the line for rows, across lines for columns.
   for (int idx = threadIdx.x; idx < kDctLines * L; idx += kDctThreads) {
     int e, l;
     if (cols) { e = idx / kDctLines; l = idx % kDctLines; }
     else { l = idx / L; e = idx % L; }
     const long long line = l0 + l;
-    xs[e * S + l] = line < n_lines ? in[addr(line, e)] : 0.0;
+    double x = 0.0;
+    if (line < n_lines) {
+      const long long f = line / per;
+      const int q = (int)(line % per), at = (cols ? q : q * n) + e * step;
+      x = in.field(f)[at];
+      if (INV && gam.lam2) x = rcp_fast(1.0 + gam.s[f >> 1] * gam.lam2[at]) * x;
+    }
+    xs[e * S + l] = x;
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = kDctThreads / 32;
+  const int split_n = gridDim.y, share = blockIdx.y;
+  const long long my_line = l0 + lane;
+  const bool mine = my_line < n_lines;
+  double* dst = nullptr;  // this lane's output line
+  if (mine) {
+    const int q = (int)(my_line % per);
+    dst = out.field(my_line / per) + (cols ? q : (long long)q * n);
+  }
   auto split = [](double x, float& hi, float& lo) {
     hi = (float)x;
     lo = (float)(x - (double)hi);
   };
+  // Outputs go back through the staging buffer where one CTA holds all of
+  // them (coalesced stores); a share of them is stored directly.
+  auto put = [&](int e, double v) {
+    if (split_n == 1) xs[e * S + lane] = v;
+    else if (mine) dst[(long long)e * step] = v;
+  };
   if (!INV) {
-    // Sums and differences of mirrored inputs, as hi/lo floats.
+    // Sums and differences of mirrored inputs.
     float* esh = fs;
     float* esl = fs + hc * S;
     float* osh = fs + 2 * hc * S;
     float* osl = fs + 3 * hc * S;
     for (int i = warp; i < h; i += nw) {
       const double a = xs[i * S + lane], b = xs[(L - 1 - i) * S + lane];
-      split(a + b, esh[i * S + lane], esl[i * S + lane]);
-      split(a - b, osh[i * S + lane], osl[i * S + lane]);
+      if (DF) {
+        split(a + b, esh[i * S + lane], esl[i * S + lane]);
+        split(a - b, osh[i * S + lane], osl[i * S + lane]);
+      } else {
+        xs[i * S + lane] = a + b;
+        xs[(L - 1 - i) * S + lane] = a - b;
+      }
     }
     float mid_h = 0.f, mid_l = 0.f;
-    if (L & 1) split(xs[h * S + lane], mid_h, mid_l);
-    __syncthreads();
-    // y[k] into xs (the inputs are no longer needed).
-    for (int k = warp; k < L; k += nw) {
-      const float* sh = (k & 1) ? osh : esh;
-      const float* sl = (k & 1) ? osl : esl;
-      const float* ckh = ch + (long long)k * L;
-      const float* ckl = cl + (long long)k * L;
-      DfAcc acc;
-      if (L & 1) acc.add(ckh[h], ckl[h], mid_h, mid_l);
-      for (int i = 0; i < h; ++i) acc.add(ckh[i], ckl[i], sh[i * S + lane], sl[i * S + lane]);
-      float rh, rl;
-      acc.result(rh, rl);
-      xs[k * S + lane] = (double)rh + (double)rl;
+    double mid = 0.0;
+    if (L & 1) {
+      mid = xs[h * S + lane];
+      split(mid, mid_h, mid_l);
     }
-  } else {
+    __syncthreads();
+    if (DF) {
+      // y[k] (into xs: the inputs are no longer needed).
+      for (int k = share * nw + warp; k < L; k += nw * split_n) {
+        const float* sh = (k & 1) ? osh : esh;
+        const float* sl = (k & 1) ? osl : esl;
+        const float* ckh = ch + (long long)k * L;
+        const float* ckl = cl + (long long)k * L;
+        DfAcc acc;
+        if (L & 1) acc.add(ckh[h], ckl[h], mid_h, mid_l);
+        for (int i = 0; i < h; ++i) acc.add(ckh[i], ckl[i], sh[i * S + lane], sl[i * S + lane]);
+        float rh, rl;
+        acc.result(rh, rl);
+        put(k, (double)rh + (double)rl);
+      }
+    } else {
+      // Two outputs of one parity per turn share the loaded sums.
+      for (int g = share * nw + warp; 4 * g < L; g += nw * split_n)
+        for (int par = 0; par < 2; ++par) {
+          const int k0 = 4 * g + par, k1 = k0 + 2;
+          if (k0 >= L) continue;
+          const double* c0 = cd + (long long)k0 * L;
+          const double* c1 = cd + (long long)min(k1, L - 1) * L;
+          double a0 = (L & 1) ? c0[h] * mid : 0.0, a1 = (L & 1) ? c1[h] * mid : 0.0;
+          const double* x = par ? xs + (L - 1) * S + lane : xs + lane;
+          const int xstep = par ? -S : S;
+#pragma unroll 4
+          for (int i = 0; i < h; ++i, x += xstep) {
+            a0 = fma(c0[i], *x, a0);
+            a1 = fma(c1[i], *x, a1);
+          }
+          if (mine) dst[(long long)k0 * step] = a0;
+          if (mine && k1 < L) dst[(long long)k1 * step] = a1;
+        }
+    }
+  } else if (DF) {
     // The inputs as hi/lo floats.
     float* xh = fs;
     float* xl = fs + L * S;
@@ -238,7 +474,7 @@ __global__ void __launch_bounds__(kDctThreads) k_dct_lines(int m, int n, int bat
       split(xs[q], xh[q], xl[q]);
     }
     __syncthreads();
-    for (int i = warp; i < hc; i += nw) {
+    for (int i = share * nw + warp; i < hc; i += nw * split_n) {
       DfAcc ev, od;
       for (int k = 0; k < L; k += 2) ev.add(ch[(long long)k * L + i], cl[(long long)k * L + i], xh[k * S + lane], xl[k * S + lane]);
       for (int k = 1; k < L; k += 2) od.add(ch[(long long)k * L + i], cl[(long long)k * L + i], xh[k * S + lane], xl[k * S + lane]);
@@ -246,49 +482,101 @@ __global__ void __launch_bounds__(kDctThreads) k_dct_lines(int m, int n, int bat
       ev.result(eh, el);
       od.result(oh, ol);
       const double e = (double)eh + (double)el, o = (double)oh + (double)ol;
-      xs[i * S + lane] = e + o;                          // x[i]
-      if (L - 1 - i != i) xs[(L - 1 - i) * S + lane] = e - o;  // x[L-1-i]
+      put(i, e + o);                          // x[i]
+      if (L - 1 - i != i) put(L - 1 - i, e - o);  // x[L-1-i]
+    }
+  } else {
+    for (int g = share * nw + warp; 2 * g < hc; g += nw * split_n) {
+      const int i0 = 2 * g, i1 = min(i0 + 1, hc - 1);
+      double e0 = 0.0, e1 = 0.0, o0 = 0.0, o1 = 0.0;
+#pragma unroll 2
+      for (int k = 0; k < L; k += 2) {
+        const double x = xs[k * S + lane];
+        const double* c = cd + (long long)k * L;
+        e0 = fma(c[i0], x, e0);
+        e1 = fma(c[i1], x, e1);
+        if (k + 1 < L) {
+          const double y = xs[(k + 1) * S + lane];
+          o0 = fma(c[L + i0], y, o0);
+          o1 = fma(c[L + i1], y, o1);
+        }
+      }
+      if (!mine) continue;
+      dst[(long long)i0 * step] = e0 + o0;
+      if (L - 1 - i0 != i0) dst[(long long)(L - 1 - i0) * step] = e0 - o0;
+      if (i1 == i0) continue;
+      dst[(long long)i1 * step] = e1 + o1;
+      if (L - 1 - i1 != i1) dst[(long long)(L - 1 - i1) * step] = e1 - o1;
     }
   }
+  if (!DF || split_n > 1) return;
   __syncthreads();
   for (int idx = threadIdx.x; idx < kDctLines * L; idx += kDctThreads) {
     int e, l;
     if (cols) { e = idx / kDctLines; l = idx % kDctLines; }
     else { l = idx / L; e = idx % L; }
     const long long line = l0 + l;
-    if (line < n_lines) out[addr(line, e)] = xs[e * S + l];
+    if (line >= n_lines) continue;
+    const int q = (int)(line % per);
+    out.field(line / per)[(cols ? q : q * n) + e * step] = xs[e * S + l];
   }
+}
+
+__global__ void k_apply_gamma(long long mn, int n_pairs, DctGamma gam, double* __restrict__ fd) {
+  const int pair = blockIdx.y;
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= 2 * mn) return;
+  const long long e = t % mn;
+  double* f = fd + (long long)pair * 2 * mn + t;
+  *f = rcp_fast(1.0 + gam.s[pair] * gam.lam2[e]) * *f;
 }
 
 // One DCT pass over `batch` fields: forward (DCT-II) or inverse (DCT-III)
-// along rows (cols = 0, matrix c of size n) or columns (cols = 1, size m).
-static void dct_pass(int m, int n, int batch, bool inverse, int cols, const double* c, const float* cf,
-                     const double* in, double* out, cudaStream_t stream) {
+// along rows (cols = 0, tables of size n) or columns (cols = 1, size m). Lines
+// of up to kDctMaxLen positions take the double-float products, longer ones
+// the float64 products (the double-float error grows with the length), both
+// staged with the symmetric split. Measured: 63 x 63, one pair, 18 -> 11 us
+// per pass by the shares; 253 x 253, one pair, 70 us per pass by plain float64
+// dot products, 55 us so (31 us of it at the float64 rate).
+template <bool INV>
+static int dct_pass(int m, int n, int batch, int cols, const SmoothTables& t, DctIo in, DctIo out, DctGamma gam,
+                    cudaStream_t stream) {
   const int L = cols ? m : n;
   const long long n_lines = (long long)batch * (cols ? n : m);
-  if (L > kDctMaxLen) {
+  if (L > kDctLongLen) {
+    if (gam.lam2) {
+      const long long mn = (long long)m * n;
+      k_apply_gamma<<<dim3((unsigned)((2 * mn + 255) / 256), (unsigned)(batch / 2)), 256, 0, stream>>>(mn, batch / 2,
+                                                                                                     gam, in.u);
+    }
     const long long tot = (long long)m * n * batch;
-    const int mode = cols ? (inverse ? 3 : 2) : (inverse ? 1 : 0);
-    k_dct_apply<<<(unsigned)((tot + 255) / 256), 256, 0, stream>>>(m, n, batch, mode, c, in, out);
-    return;
+    const int mode = cols ? (INV ? 3 : 2) : (INV ? 1 : 0);
+    k_dct_apply<<<(unsigned)((tot + 255) / 256), 256, 0, stream>>>(m, n, batch, mode, cols ? t.cm : t.cn, in, out);
+    return check("k_dct_apply");
   }
-  const size_t smem = (size_t)(L + 2 * ((L + 1) / 2)) * (kDctLines + 1) * sizeof(double);
-  const unsigned grid = (unsigned)((n_lines + kDctLines - 1) / kDctLines);
-  if (inverse) k_dct_lines<true><<<grid, kDctThreads, smem, stream>>>(m, n, batch, cols, cf, in, out);
-  else k_dct_lines<false><<<grid, kDctThreads, smem, stream>>>(m, n, batch, cols, cf, in, out);
+  const bool df = L <= kDctMaxLen;
+  const float* cf = cols ? t.cmf : t.cnf;
+  const double* cd = cols ? t.cm : t.cn;
+  const long long blocks = (n_lines + kDctLines - 1) / kDctLines;
+  // Shares of the outputs: as many as the SMs take, each warp of a share
+  // with at least one output.
+  const int turns = df ? (INV ? (L + 1) / 2 : L) : (L + 3) / 4;
+  int shares = (turns + kDctThreads / 32 - 1) / (kDctThreads / 32);
+  const long long room = blocks < sm_count() ? sm_count() / blocks : 1;
+  if (shares > room) shares = (int)room;
+  const dim3 grid((unsigned)blocks, (unsigned)shares);
+  if (df) {
+    const size_t smem = (size_t)(L + 2 * ((L + 1) / 2)) * (kDctLines + 1) * sizeof(double);
+    k_dct_lines<INV, true><<<grid, kDctThreads, smem, stream>>>(m, n, batch, cols, cf, cd, in, out, gam);
+  } else {
+    const size_t smem = (size_t)L * (kDctLines + 1) * sizeof(double);
+    cudaError_t e = cudaFuncSetAttribute(k_dct_lines<INV, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         kDctLongLen * (kDctLines + 1) * (int)sizeof(double));
+    if (e != cudaSuccess) return set_cuda_error(e, "cudaFuncSetAttribute(k_dct_lines)");
+    k_dct_lines<INV, false><<<grid, kDctThreads, smem, stream>>>(m, n, batch, cols, cf, cd, in, out, gam);
+  }
+  return check("k_dct_lines");
 }
-
-__global__ void k_f2(long long mn, int n_pairs, const double* __restrict__ fd, double* __restrict__ f2,
-                     float* __restrict__ f2f) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= mn * n_pairs) return;
-  const long long pair = t / mn, e = t % mn;
-  const double a = fd[(2 * pair) * mn + e], b = fd[(2 * pair + 1) * mn + e];
-  f2[t] = a * a + b * b;
-  f2f[t] = (float)(a * a + b * b);
-}
-
-static constexpr int kGcvThreads = 512;
 
 // Flags of SmoothnGPU's log messages (gpu_smoothn.py:218-222, 429-439): with
 // GCV, the smoothing parameter within 0.1 (in log10) of its lower or else its
@@ -303,182 +591,199 @@ PIV_D int smooth_flags(bool is_auto, double p, double pmin, double pmax, bool la
   return f;
 }
 
-// 1/d for d >= 1 from the float32 reciprocal and two Newton steps in float64:
-// within an ulp or two of the rounded quotient, at a fraction of the cost of
-// a float64 division (float64 throughput on this GPU is low).
-PIV_D double rcp_fast(double d) {
-  double r = (double)__frcp_rn((float)d);
-  double e = fma(-d, r, 1.0);
-  r = fma(r, e, r);
-  e = fma(-d, r, 1.0);
-  return fma(r, e, r);
-}
-
-// One CTA per pair. Every thread takes part in the sums of each score; the
-// search itself (scan bookkeeping and the L-BFGS-B steps: scalar float64
-// work) runs in warp 0 alone, which announces each next point as s = 10^p in
-// shared memory. Float64 runs at a small fraction of the float32 rate on this
-// GPU, so the search is not repeated by all 16 warps. The fast score (float32
-// terms, float64 sums: 1 - gamma = s l / (1 + s l) formed without
+// The GCV search of one pair, by the c CTAs of a cluster. The sums of each
+// score are formed by the kVT virtual threads (each CTA runs kVT / c of them);
+// the warps' partial sums go to every CTA of the cluster through distributed
+// shared memory, and warp 0 of every CTA adds them in warp order and runs the
+// search (scan bookkeeping and the L-BFGS-B steps: scalar float64 work) for
+// itself, so one cluster barrier per evaluation suffices. The fast score
+// (float32 terms, float64 sums: 1 - gamma = s l / (1 + s l) formed without
 // cancellation, each term within a few float32 ulps, the score within ~1e-9)
-// only ranks the scan points; the L-BFGS-B evaluations, whose difference
-// quotients divide score differences by 1e-8, use the float64 score.
-__global__ void __launch_bounds__(kGcvThreads)
-k_gcv(int m, int n, int n_pairs, const double* __restrict__ f2, const double* __restrict__ lam2,
-      const float* __restrict__ f2f, const float* __restrict__ lam2f, double pmin, double pmax,
-      double* __restrict__ p_out, int* __restrict__ flags) {
-  __shared__ double red[64];
-  __shared__ double sh_s;  // 10^p of the next score
-  __shared__ int sh_go;    // warp 0's decision for the next step
-  const int pair = blockIdx.x;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+// only ranks the scan points, all ten in one pass over the field; the
+// L-BFGS-B evaluations, whose difference quotients divide score differences
+// by 1e-8, use the float64 score, the point and its neighbour together.
+// Bound by the float64 pipe and by the latency of the search's steps. One
+// score at a time on one CTA, with the scan in ten passes, took 396 us for
+// the 31 x 31 and 63 x 63 fields of one 1024 x 1024 pair; this takes 157 us.
+__global__ void __launch_bounds__(kVT)
+k_gcv(int m, int n, int c, const double* __restrict__ fd, double* __restrict__ f2, float* __restrict__ f2f,
+      const double* __restrict__ lam2, const float* __restrict__ lam2f, double pmin, double pmax,
+      double* __restrict__ p_out, double* __restrict__ s_out, int* __restrict__ flags) {
+  __shared__ double part[2][kVW][20];  // by parity of the evaluation: the virtual warps' partial sums
+  __shared__ double sh_s[10];          // 10^p of the next scores
+  __shared__ int sh_go;                // warp 0's decision for the next step
+  const int pair = blockIdx.x / c;
+  const int rank = c > 1 ? (int)cluster_rank() : 0;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int vt = rank * blockDim.x + threadIdx.x, vw = vt >> 5;
   const bool w0 = warp == 0;
   const long long mn = (long long)m * n;
-  const double* f2p = f2 + pair * mn;
-  const float* f2fp = f2f + pair * mn;
+  const double* fu = fd + 2 * pair * mn;
+  double* f2p = f2 + pair * mn;
+  float* f2fp = f2f + pair * mn;
   const double n_finite = (double)mn;
-  // Combines the per-warp sums in red[] (valid in warp 0).
-  auto combine = [&](double& trss, double& ttr) {
-    trss = 0.0;
-    ttr = 0.0;
-    for (int k = 0; k < nw; ++k) { trss += red[k]; ttr += red[32 + k]; }
-  };
-  // Scores at the announced point (all threads, after a barrier that follows
-  // the announcement); the value is valid in warp 0.
-  auto score_fast = [&]() -> double {
-    const float s = (float)sh_s;
-    float rss = 0.f, tr = 0.f;
-    for (long long e = threadIdx.x; e < mn; e += blockDim.x) {
-      const float sl = s * lam2f[e];
-      const float d = sl * __frcp_rn(1.0f + sl);  // 1 - gamma
-      rss = fmaf(f2fp[e] * d, d, rss);
-      tr += d;
-    }
-    double drss = rss, dtr = tr;
-    for (int o = 16; o > 0; o >>= 1) {
-      drss += __shfl_xor_sync(~0u, drss, o);
-      dtr += __shfl_xor_sync(~0u, dtr, o);
-    }
-    if (lane == 0) { red[warp] = drss; red[32 + warp] = dtr; }
-    __syncthreads();
-    double f = 0.0;
-    if (w0) {
-      double trss, ttr;
-      combine(trss, ttr);
-      const double q = ttr / (double)mn;
-      f = trss / n_finite / (q * q) / 2;
-    }
-    return f;
-  };
-  auto score = [&]() -> double {
-    const double s = sh_s;
-    double rss = 0.0, tr = 0.0;
-    for (long long e = threadIdx.x; e < mn; e += blockDim.x) {
-      const double gm = rcp_fast(1.0 + s * lam2[e]);
-      const double d = gm - 1.0;
-      rss += f2p[e] * d * d;
-      tr += gm;
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      rss += __shfl_xor_sync(~0u, rss, o);
-      tr += __shfl_xor_sync(~0u, tr, o);
-    }
-    if (lane == 0) { red[warp] = rss; red[32 + warp] = tr; }
-    __syncthreads();
-    double f = 0.0;
-    if (w0) {
-      double trss, ttr;
-      combine(trss, ttr);
-      const double q = 1.0 - ttr / (double)mn;
-      f = trss / n_finite / (q * q) / 2;
-    }
-    return f;
-  };
-  // Announces p (thread 0) and whether the search goes on, and makes both
-  // visible; the barrier also orders the previous score's reads of red[]
-  // before the next score's writes.
-  auto announce = [&](double p, bool go) {
-    if (threadIdx.x == 0) {
-      sh_s = pow(10.0, p);
-      sh_go = go;
-    }
-    __syncthreads();
+  // fd_u^2 + fd_v^2; each virtual thread reads only what it wrote.
+  for (long long e = vt; e < mn; e += kVT) {
+    const double a = fu[e], b = fu[mn + e];
+    const double q = a * a + b * b;
+    f2p[e] = q;
+    f2fp[e] = (float)q;
+  }
+  int par = 0;
+  auto publish = [&](int count, int slot, bool holds, double v) {
+    if (holds && slot < count)
+      for (int r = 0; r < c; ++r) {
+        if (c == 1) part[par][vw][slot] = v;
+        else st_cluster(&part[par][vw][slot], (unsigned)r, v);
+      }
+    cluster_barrier(c);
   };
   // 10-point scan (gpu_smoothn.py:182-188), ranked with the fast score; when
   // other points score within 1e-6 of the best, those points are scored
   // again in float64 and the first minimum among them is kept (np.argmin).
-  double fast[10];
-  double best_f = INFINITY;
-  for (int k = 0; k < 10; ++k) {
-    const double pk = ((double)k * (1.0 / 9.0)) * (pmax - pmin) + pmin;
-    announce(pk, true);
-    fast[k] = score_fast();
-    if (fast[k] < best_f) best_f = fast[k];
-  }
-  unsigned near_best = 0;  // scan points within 1e-6 of the best fast score (warp 0)
-  for (int k = 0; k < 10; ++k)
-    if (fast[k] <= best_f + 1e-6 * fabs(best_f)) near_best |= 1u << k;
-  if (threadIdx.x == 0) sh_go = __popc(near_best) > 1 ? (int)near_best : 0;
+  auto scan_point = [&](int k) { return ((double)k * (1.0 / 9.0)) * (pmax - pmin) + pmin; };
+  if (threadIdx.x < 10) sh_s[threadIdx.x] = pow(10.0, scan_point(threadIdx.x));
   __syncthreads();
-  const unsigned rescore = (unsigned)sh_go;
+  {
+    float acc[20], s[10];
+#pragma unroll
+    for (int k = 0; k < 10; ++k) {
+      s[k] = (float)sh_s[k];
+      acc[k] = acc[10 + k] = 0.f;
+    }
+    for (long long e = vt; e < mn; e += kVT) {
+      const float l = lam2f[e], f = f2fp[e];
+#pragma unroll
+      for (int k = 0; k < 10; ++k) {
+        const float sl = s[k] * l;
+        const float d = sl * __frcp_rn(1.0f + sl);  // 1 - gamma
+        acc[k] = fmaf(f * d, d, acc[k]);
+        acc[10 + k] += d;
+      }
+    }
+    publish(20, lane, true, warp_sums(acc));
+  }
   double p0 = pmin;
+  unsigned rescore = 0;  // scan points within 1e-6 of the best fast score, when there are several
+  if (w0) {
+    const int q = lane < 10 ? lane : 0;
+    double trss = 0.0, ttr = 0.0;
+    for (int k = 0; k < kVW; ++k) {
+      trss += part[par][k][q];
+      ttr += part[par][k][10 + q];
+    }
+    const double w = ttr / (double)mn;
+    const double f = trss / n_finite / (w * w) / 2;
+    double best_f = INFINITY;
+    double fast[10];
+#pragma unroll
+    for (int k = 0; k < 10; ++k) {
+      fast[k] = __shfl_sync(~0u, f, k);
+      if (fast[k] < best_f) best_f = fast[k];
+    }
+    unsigned near_best = 0;
+#pragma unroll
+    for (int k = 9; k >= 0; --k) {
+      if (fast[k] <= best_f + 1e-6 * fabs(best_f)) near_best |= 1u << k;
+      if (fast[k] == best_f) p0 = scan_point(k);
+    }
+    if (lane == 0) sh_go = __popc(near_best) > 1 ? (int)near_best : 0;
+  }
+  par ^= 1;
+  // Announces two points (warp 0) and whether the search goes on, and makes
+  // both visible to the CTA.
+  auto announce = [&](double pa, double pb, bool go) {
+    if (w0) {
+      if (lane < 2) sh_s[lane] = pow(10.0, lane ? pb : pa);
+      if (lane == 0) sh_go = go;
+    }
+    __syncthreads();
+  };
+  // Float64 scores at the two announced points (valid in warp 0).
+  auto score2 = [&](double& fa, double& fb) {
+    const double sa = sh_s[0], sb = sh_s[1];
+    double ra = 0.0, ta = 0.0, rb = 0.0, tb = 0.0;
+    for (long long e = vt; e < mn; e += kVT) {
+      const double l = lam2[e], f = f2p[e];
+      const double ga = rcp_fast(1.0 + sa * l), gb = rcp_fast(1.0 + sb * l);
+      const double da = ga - 1.0, db = gb - 1.0;
+      ra += f * da * da;
+      ta += ga;
+      rb += f * db * db;
+      tb += gb;
+    }
+    publish(4, lane >> 3, (lane & 7) == 0, warp_sums4(ra, ta, rb, tb));
+    if (w0) {
+      double t = 0.0;
+      for (int k = 0; k < kVW; ++k) t += part[par][k][lane & 3];
+      const double trss = __shfl_sync(~0u, t, (lane & 1) * 2), ttr = __shfl_sync(~0u, t, (lane & 1) * 2 + 1);
+      const double q = 1.0 - ttr / (double)mn;
+      const double f = trss / n_finite / (q * q) / 2;
+      fa = __shfl_sync(~0u, f, 0);
+      fb = __shfl_sync(~0u, f, 1);
+    }
+    par ^= 1;
+  };
+  __syncthreads();
+  rescore = (unsigned)sh_go;
   if (rescore) {
     double best64 = INFINITY;
-    for (int k = 0; k < 10; ++k) {
-      if (!((rescore >> k) & 1u)) continue;
-      const double pk = ((double)k * (1.0 / 9.0)) * (pmax - pmin) + pmin;
-      announce(pk, true);
-      const double fk = score();
-      if (fk < best64) { best64 = fk; p0 = pk; }
+    p0 = pmin;
+    while (rescore) {
+      const int ka = __ffs(rescore) - 1;
+      rescore &= rescore - 1;
+      const int kb = rescore ? __ffs(rescore) - 1 : ka;
+      rescore &= rescore - 1;
+      const double pa = scan_point(ka), pb = scan_point(kb);
+      __syncthreads();  // every read of sh_go and sh_s is done
+      announce(pa, pb, true);
+      double fa = 0.0, fb = 0.0;
+      score2(fa, fb);
+      if (fa < best64) { best64 = fa; p0 = pa; }
+      if (fb < best64) { best64 = fb; p0 = pb; }
     }
-  } else {
-    for (int k = 9; k >= 0; --k)
-      if (fast[k] == best_f) p0 = ((double)k * (1.0 / 9.0)) * (pmax - pmin) + pmin;
   }
   // L-BFGS-B from the scan point (gpu_smoothn.py:191-193), its scalar state
-  // in warp 0; every evaluation is the float64 score at the point and at its
-  // forward-difference neighbour.
+  // in warp 0.
   Lb1 lb;
-  lb_init(lb, p0, pmin, pmax);
+  lb.done = false;
+  if (w0) lb_init(lb, p0, pmin, pmax);
   for (int ev = 0; ev < kLbMaxEvals; ++ev) {
-    const double xt = lb.xt, xs = lb_fd_point(xt, pmin, pmax);
-    announce(xt, !lb.done);
+    double xt = 0.0, xs = 0.0;
+    if (w0) {
+      xt = lb.xt;
+      xs = lb_fd_point(xt, pmin, pmax);
+    }
+    __syncthreads();  // every read of sh_go and sh_s is done
+    announce(xt, xs, !lb.done);
     if (!sh_go) break;
-    const double f = score();
-    announce(xs, true);
-    const double fh = score();
+    double f = 0.0, fh = 0.0;
+    score2(f, fh);
     if (w0) lb_feed(lb, f, (fh - f) / (xs - xt));
   }
-  const double p = lb.x;
-  if (threadIdx.x == 0) {
-    p_out[pair] = p;
+  if (rank == 0 && threadIdx.x == 0) {
+    const double p = lb.x;
+    s_out[pair] = pow(10.0, p);
+    if (p_out) p_out[pair] = p;
     if (flags) flags[pair] = smooth_flags(true, p, pmin, pmax, false);
   }
 }
 
-// fd *= gamma(p) for both fields of each pair. Grid: x over the 2 mn
-// coefficients of a pair, y over pairs; s = 10^p is formed once per CTA.
-__global__ void k_apply_gamma(long long mn, int n_pairs, const double* __restrict__ lam2,
-                              const double* __restrict__ p, double fixed_p, double* __restrict__ fd) {
-  __shared__ double s_sh;
-  const int pair = blockIdx.y;
-  if (threadIdx.x == 0) s_sh = pow(10.0, p ? p[pair] : fixed_p);
-  __syncthreads();
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 2 * mn) return;
-  const long long e = t % mn;
-  double* f = fd + (long long)pair * 2 * mn + t;
-  *f = rcp_fast(1.0 + s_sh * lam2[e]) * *f;
-}
-
-__global__ void k_fill(int count, double value, double* out) {
+// A given parameter: s = 10^p of every pair (and p itself).
+__global__ void k_fill_s(int count, double p, double* s, double* p_out) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < count) out[t] = value;
+  if (t >= count) return;
+  s[t] = pow(10.0, p);
+  if (p_out) p_out[t] = p;
 }
 
-static int check(const char* what) {
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? PIV_OK : set_cuda_error(e, what);
+// Bounds of p = log10(s) for order 2 (gpu_smoothn.py:320-338), on the host.
+static void gcv_bounds(int m, int n, double* pmin, double* pmax) {
+  const double h_min = 1e-3, h_max = 1.0 - h_min;
+  const int rank = (m != 1) + (n != 1);
+  const double a_max = pow(h_max, 2.0 / rank), a_min = pow(h_min, 2.0 / rank);
+  *pmin = log10((pow((1.0 + sqrt(1.0 + 8.0 * a_max)) / 4.0 / a_max, 2.0) - 1.0) / 16.0);
+  *pmax = log10((pow((1.0 + sqrt(1.0 + 8.0 * a_min)) / 4.0 / a_min, 2.0) - 1.0) / 16.0);
 }
 
 // ---------------------------------------------------------------------------
@@ -494,305 +799,395 @@ static int check(const char* what) {
 // the GCV search runs at iterations 1, 2, 4, 8, ... (gpu_smoothn.py:176-193),
 // with the w_mean <= 0.9 score refitting the field for every candidate s
 // (gpu_smoothn.py:359-368). Output zero inside the mask (gpu_smoothn.py:224-225).
-// One CTA per pair does the whole iteration; float64 throughout.
+// Float64 throughout but for the DCTs' double-float products (DfAcc).
+//
+// A cluster of c CTAs runs each pair (cluster_size). CTA r owns the rows [r
+// R, (r + 1) R) of the 2 m rows of the two fields: it transforms its rows and
+// forms its rows of the column passes, whose inputs (all rows) come through
+// global memory (L2) with one cluster barrier in between; the forward column
+// pass leaves the rows that the inverse row pass of the same CTA starts from.
+// The sums run over virtual threads as in k_gcv, so the result does not
+// depend on c. Bound by the DCTs' dot products and the barriers between
+// passes: one pair of 63 x 63 around a masked disc takes 0.90 ms with 8 CTAs.
+// On one CTA, with strided matrix reads and 10^p formed by every thread, it
+// took 6.4 ms.
 // ---------------------------------------------------------------------------
 static constexpr int kSwThreads = 512;
 
-PIV_D double cta_sum(double v, double* red) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(~0u, v, o);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
-  __syncthreads();
-  if (l == 0) red[w] = v;
-  __syncthreads();
-  double t = l < nw ? red[l] : 0.0;
-  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(~0u, t, o);
-  return t;
-}
-
-struct DfMats {
-  const float *cmh, *cml, *cnh, *cnl;  // [m][m], [n][n] hi and lo parts
+struct SwShared {
+  double red[2][4][kVW];
+  double sums[4];
+  double s[2];
+  int go;
 };
 
-// 2-D orthonormal DCT-II (inv = false) or DCT-III of one m x n field inside the
-// CTA, in the double-float arithmetic of DfAcc. xs: 2 mn floats (the input's
-// hi/lo split); tmp: 2 mn floats (the row pass); in and out may not overlap
-// tmp or xs.
-PIV_D void cta_dct2(const double* in, float* xs, float* tmp, double* out, int m, int n, const DfMats& M, bool inv) {
-  const int mn = m * n;
-  for (int e = threadIdx.x; e < mn; e += blockDim.x) {
-    const double x = in[e];
-    const float h = (float)x;
-    xs[e] = h;
-    xs[mn + e] = (float)(x - (double)h);
+struct SwCtx {
+  int m, n, mn, c, rank, par;
+  int e0, e1;  // this CTA's rows as flat elements of the two fields
+  const double* lam2;
+  const float2 *cm, *cn, *cnt;  // DCT matrices as (hi, lo): [m][m], [n][n] and its transpose
+  double *f, *z, *zo, *fd, *tmp, *w;
+  double n_finite, w_mean;
+  SwShared* sh;
+};
+
+// Row pass over this CTA's rows, in the double-float arithmetic of DfAcc: the
+// inputs load(e) are split into xs (this CTA's rows of it), the results go to
+// out as (hi, lo). out may be the array that load reads.
+template <class Load>
+PIV_D void sw_row_pass(const SwCtx& x, bool inv, Load load, float2* xs, float2* out) {
+  for (int e = x.e0 + threadIdx.x; e < x.e1; e += kSwThreads) {
+    const double v = load(e);
+    const float h = (float)v;
+    xs[e] = make_float2(h, (float)(v - (double)h));
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < mn; e += blockDim.x) {
-    const int i = e / n, l = e % n;
+  const float2* mat = inv ? x.cn : x.cnt;
+  const int n = x.n;
+  for (int e = x.e0 + threadIdx.x; e < x.e1; e += kSwThreads) {
+    const int l = e % n;
+    const float2* xr = xs + (e - l);
+    const float2* mc = mat + l;
     DfAcc acc;
+#pragma unroll 8
     for (int j = 0; j < n; ++j) {
-      const int ci = inv ? j * n + l : l * n + j;
-      acc.add(xs[i * n + j], xs[mn + i * n + j], M.cnh[ci], M.cnl[ci]);
+      const float2 a = xr[j], b = __ldg(mc + (long long)j * n);
+      acc.add(a.x, a.y, b.x, b.y);
     }
-    acc.result(tmp[e], tmp[mn + e]);
+    float2 r;
+    acc.result(r.x, r.y);
+    out[e] = r;
   }
-  __syncthreads();
-  for (int e = threadIdx.x; e < mn; e += blockDim.x) {
-    const int k = e / n, j = e % n;
+}
+
+// Column pass: this CTA's rows of the result from all rows of `in`.
+template <class Store>
+PIV_D void sw_col_pass(const SwCtx& x, bool inv, const float2* in, Store store) {
+  const int m = x.m, n = x.n, mn = x.mn;
+  for (int e = x.e0 + threadIdx.x; e < x.e1; e += kSwThreads) {
+    const int fi = e >= mn ? 1 : 0, q = e - fi * mn, k = q / n, j = q - k * n;
+    const float2* col = in + fi * mn + j;
+    const float2* mr = inv ? x.cm + k : x.cm + k * m;
+    const int ms = inv ? m : 1;
     DfAcc acc;
+#pragma unroll 8
     for (int i = 0; i < m; ++i) {
-      const int ci = inv ? i * m + k : k * m + i;
-      acc.add(M.cmh[ci], M.cml[ci], tmp[i * n + j], tmp[mn + i * n + j]);
+      const float2 a = __ldg(mr + i * ms), b = col[i * n];
+      acc.add(a.x, a.y, b.x, b.y);
     }
     float h, l;
     acc.result(h, l);
-    out[e] = (double)h + (double)l;
+    store(e, (double)h + (double)l);
   }
-  __syncthreads();
 }
 
-struct SwCtx {
-  int m, n, mn;
-  const double* lam2;
-  DfMats mats;
-  double *f, *z, *t, *fd, *tmp, *w;
-  float* xs;  // 2 mn floats: hi/lo split of a DCT input
-  double n_finite, w_mean;
-  double* red;
-};
+// Sums over the pair's virtual threads of up to four values, into sh->sums
+// (every thread of the cluster calls it; it ends with a barrier).
+PIV_D void sw_sums(SwCtx& x, double a, double b, double c, double d) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int vtn = kVT / x.c;
+  if ((int)threadIdx.x < vtn) {
+    const double v = warp_sums4(a, b, c, d);
+    const int vw = (x.rank * vtn + threadIdx.x) >> 5;
+    if ((lane & 7) == 0)
+      for (int r = 0; r < x.c; ++r) {
+        if (x.c == 1) x.sh->red[x.par][lane >> 3][vw] = v;
+        else st_cluster(&x.sh->red[x.par][lane >> 3][vw], (unsigned)r, v);
+      }
+  }
+  cluster_barrier(x.c);
+  if (warp < 2) {
+    const int q = warp * 2 + (lane >> 4);
+    double t = x.sh->red[x.par][q][lane & 15];
+    for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(~0u, t, o);
+    if ((lane & 15) == 0) x.sh->sums[q] = t;
+  }
+  __syncthreads();
+  x.par ^= 1;
+}
 
-// GCV score at p (gpu_smoothn.py:353-372). fd: DCT of both fields.
-PIV_D double sw_gcv(const SwCtx& c, double p) {
-  const double s = pow(10.0, p);
-  double rss = 0.0, tr = 0.0;
-  if (c.w_mean > 0.9) {
-    for (int e = threadIdx.x; e < c.mn; e += blockDim.x) {
-      const double gm = rcp_fast(1.0 + s * c.lam2[e]);
-      const double d = gm - 1.0;
-      rss += (c.fd[e] * c.fd[e] + c.fd[c.mn + e] * c.fd[c.mn + e]) * d * d;
-      tr += gm;
+// GCV scores at the two announced points (gpu_smoothn.py:353-372; s in
+// sh->s); valid in warp 0. fd: DCT of both fields.
+PIV_D void sw_score2(SwCtx& x, double& fa, double& fb) {
+  const int mn = x.mn, vtn = kVT / x.c;
+  const int vt = (int)threadIdx.x < vtn ? x.rank * vtn + (int)threadIdx.x : 0x7fffffff;
+  const double s[2] = {x.sh->s[0], x.sh->s[1]};
+  double rss[2] = {0.0, 0.0}, tr[2] = {0.0, 0.0};
+  if (x.w_mean > 0.9) {
+    for (int e = vt; e < mn; e += kVT) {
+      const double l = x.lam2[e], fu = x.fd[e], fv = x.fd[mn + e];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const double gm = rcp_fast(1.0 + s[k] * l);
+        const double d = gm - 1.0;
+        rss[k] += (fu * fu + fv * fv) * d * d;
+        tr[k] += gm;
+      }
     }
   } else {
-    for (int e = threadIdx.x; e < c.mn; e += blockDim.x) tr += rcp_fast(1.0 + s * c.lam2[e]);
-    for (int fi = 0; fi < 2; ++fi) {
-      // f_hat = IDCT2(gamma fd); t holds gamma fd, z is kept.
-      for (int e = threadIdx.x; e < c.mn; e += blockDim.x)
-        c.t[fi * c.mn + e] = c.fd[fi * c.mn + e] * rcp_fast(1.0 + s * c.lam2[e]);
-      __syncthreads();
-      cta_dct2(c.t + fi * c.mn, c.xs, reinterpret_cast<float*>(c.tmp), c.tmp + c.mn, c.m, c.n, c.mats, true);
-      for (int e = threadIdx.x; e < c.mn; e += blockDim.x) {
-        const double fv = c.f[fi * c.mn + e];
-        if (isfinite(fv) || c.w[e] > 0) {
-          const double d = fv - c.tmp[c.mn + e];
-          rss += c.w[e] * d * d;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      for (int e = vt; e < mn; e += kVT) tr[k] += rcp_fast(1.0 + s[k] * x.lam2[e]);
+      // f_hat = IDCT2(gamma fd), into the spare z buffer.
+      sw_row_pass(x, true, [&](int e) { return x.fd[e] * rcp_fast(1.0 + s[k] * x.lam2[e >= mn ? e - mn : e]); },
+                  reinterpret_cast<float2*>(x.zo), reinterpret_cast<float2*>(x.tmp));
+      cluster_barrier(x.c);
+      sw_col_pass(x, true, reinterpret_cast<const float2*>(x.tmp), [&](int e, double v) { x.zo[e] = v; });
+      cluster_barrier(x.c);
+      for (int fi = 0; fi < 2; ++fi)
+        for (int e = vt; e < mn; e += kVT) {
+          const double fv = x.f[fi * mn + e];
+          if (isfinite(fv) || x.w[e] > 0) {
+            const double d = fv - x.zo[fi * mn + e];
+            rss[k] += x.w[e] * d * d;
+          }
         }
-      }
-      __syncthreads();
+      cluster_barrier(x.c);  // the next refit rewrites the buffers
     }
   }
-  rss = cta_sum(rss, c.red);
-  tr = cta_sum(tr, c.red);
-  const double q = 1.0 - tr / (double)c.mn;
-  return rss / c.n_finite / (q * q) / 2.0;
+  sw_sums(x, rss[0], tr[0], rss[1], tr[1]);
+  if (threadIdx.x < 32) {
+    const int k = threadIdx.x & 1;
+    const double q = 1.0 - x.sh->sums[2 * k + 1] / (double)mn;
+    const double f = x.sh->sums[2 * k] / x.n_finite / (q * q) / 2.0;
+    fa = __shfl_sync(~0u, f, 0);
+    fb = __shfl_sync(~0u, f, 1);
+  }
+}
+
+// Announces 10^pa and 10^pb (warp 0) and whether the search goes on.
+PIV_D void sw_announce(SwCtx& x, double pa, double pb, bool go) {
+  __syncthreads();  // every read of the previous announcement is done
+  if (threadIdx.x < 2) x.sh->s[threadIdx.x] = pow(10.0, threadIdx.x ? pb : pa);
+  if (threadIdx.x == 0) x.sh->go = go;
+  __syncthreads();
 }
 
 // The search of k_gcv: the 10-point scan on the first call (float64 scores,
 // np.argmin's first minimum), then L-BFGS-B from the start point
-// (gpu_smoothn.py:179-193). Every thread runs the same scalar steps on the
-// same scores (sw_gcv returns the CTA's sums to every thread).
-PIV_D double sw_search(const SwCtx& c, double p, bool have_p, double pmin, double pmax) {
+// (gpu_smoothn.py:179-193), its scalar steps in warp 0 of every CTA.
+PIV_D double sw_search(SwCtx& x, double p, bool have_p, double pmin, double pmax) {
+  const bool w0 = threadIdx.x < 32;
+  auto scan_point = [&](int k) { return ((double)k * (1.0 / 9.0)) * (pmax - pmin) + pmin; };
   if (!have_p) {
     double best_f = INFINITY;
-    for (int k = 0; k < 10; ++k) {
-      const double pk = ((double)k * (1.0 / 9.0)) * (pmax - pmin) + pmin;
-      const double fk = sw_gcv(c, pk);
-      if (k == 0 || fk < best_f) { best_f = fk; p = pk; }
+    for (int k = 0; k < 10; k += 2) {
+      const double pa = scan_point(k), pb = scan_point(k + 1);
+      sw_announce(x, pa, pb, true);
+      double fa = 0.0, fb = 0.0;
+      sw_score2(x, fa, fb);
+      if (k == 0 || fa < best_f) { best_f = fa; p = pa; }
+      if (fb < best_f) { best_f = fb; p = pb; }
     }
   }
   Lb1 lb;
-  lb_init(lb, p, pmin, pmax);
-  for (int ev = 0; ev < kLbMaxEvals && !lb.done; ++ev) {
-    const double x = lb.xt, xs = lb_fd_point(x, pmin, pmax);
-    const double f = sw_gcv(c, x);
-    const double fh = sw_gcv(c, xs);
-    lb_feed(lb, f, (fh - f) / (xs - x));
+  lb.done = false;
+  if (w0) lb_init(lb, p, pmin, pmax);
+  for (int ev = 0; ev < kLbMaxEvals; ++ev) {
+    double xt = 0.0, xs = 0.0;
+    if (w0) {
+      xt = lb.xt;
+      xs = lb_fd_point(xt, pmin, pmax);
+    }
+    sw_announce(x, xt, xs, !lb.done);
+    if (!x.sh->go) break;
+    double f = 0.0, fh = 0.0;
+    sw_score2(x, f, fh);
+    if (w0) lb_feed(lb, f, (fh - f) / (xs - xt));
   }
-  return lb.x;
+  return w0 ? lb.x : p;
 }
 
 __global__ void __launch_bounds__(kSwThreads)
-k_smoothn_weighted(int m, int n, const double* u_in, const double* v_in, double* u_out, double* v_out,
-                   const uint8_t* __restrict__ mask,
-                   double fixed_p, int is_auto, double pmin, double pmax, DfMats mats,
-                   const double* __restrict__ lam2, unsigned char* scratch, size_t pair_bytes, double* p_out,
-                   int* flags) {
-  __shared__ double red[32];
-  __shared__ int s_flag;
-  const int pair = blockIdx.x, mn = m * n, tid = threadIdx.x, nt = blockDim.x;
+k_smoothn_weighted(int m, int n, int c, const double* u_in, const double* v_in, double* u_out, double* v_out,
+                   const uint8_t* __restrict__ mask, double fixed_p, int is_auto, double pmin, double pmax,
+                   const float2* cm2, const float2* cn2, const float2* cnt2, const double* __restrict__ lam2,
+                   unsigned char* scratch, size_t pair_bytes, double* p_out, int* flags) {
+  __shared__ SwShared sh;
+  const int pair = blockIdx.x / c, mn = m * n, tid = threadIdx.x;
   double* base = reinterpret_cast<double*>(scratch + pair_bytes * pair);
-  SwCtx c;
-  c.m = m; c.n = n; c.mn = mn; c.mats = mats; c.lam2 = lam2;
-  c.f = base; c.z = base + 2 * mn; c.t = base + 4 * mn; c.fd = base + 6 * mn; c.tmp = base + 8 * mn;
-  c.w = base + 10 * mn; c.red = red;
+  SwCtx x;
+  x.m = m; x.n = n; x.mn = mn; x.c = c; x.rank = c > 1 ? (int)cluster_rank() : 0; x.par = 0;
+  x.cm = cm2; x.cn = cn2; x.cnt = cnt2; x.lam2 = lam2;
+  x.f = base; x.z = base + 2 * mn; x.zo = base + 4 * mn; x.fd = base + 6 * mn; x.tmp = base + 8 * mn;
+  x.w = base + 10 * mn; x.sh = &sh;
   int* near = reinterpret_cast<int*>(base + 11 * mn);
-  c.xs = reinterpret_cast<float*>(near + mn);
-  float* tmpf = reinterpret_cast<float*>(c.tmp);
+  const int rows = (2 * m + c - 1) / c;
+  x.e0 = min(x.rank * rows, 2 * m) * n;
+  x.e1 = min((x.rank + 1) * rows, 2 * m) * n;
+  const int vtn = kVT / c;
+  const int vt = tid < vtn ? x.rank * vtn + tid : 0x7fffffff;
+  const int gt = x.rank * kSwThreads + tid, gn = c * kSwThreads;  // thread of the cluster
   const long long off = (long long)pair * mn;
   // Fields, finite mask and weights.
   double nf = 0.0, ws = 0.0;
-  for (int e = tid; e < mn; e += nt) {
+  for (int e = vt; e < mn; e += kVT) {
     const double a = u_in[off + e], b = v_in[off + e];
     const bool fin = isfinite(a) && isfinite(b);
-    c.f[e] = a;
-    c.f[mn + e] = b;
+    x.f[e] = a;
+    x.f[mn + e] = b;
     const double wv = (fin && !(mask && mask[e])) ? 1.0 : 0.0;
-    c.w[e] = wv;
+    x.w[e] = wv;
     nf += fin ? 1.0 : 0.0;
     ws += wv;
   }
-  nf = cta_sum(nf, red);
-  ws = cta_sum(ws, red);
-  c.n_finite = nf;
-  c.w_mean = ws / (double)mn;
+  sw_sums(x, nf, ws, 0.0, 0.0);
+  nf = sh.sums[0];
+  ws = sh.sums[1];
+  x.n_finite = nf;
+  x.w_mean = ws / (double)mn;
   const bool weighted = ws != (double)mn;
   // Nearest finite neighbour of the missing points: first the nearest finite
   // row in every column (ties: the lower row), then the nearest column.
   if (nf < (double)mn && nf > 0) {
-    for (int col = tid; col < n; col += nt) {
+    for (int col = gt; col < n; col += gn) {
       int last = -1;
       for (int y = 0; y < m; ++y) {
-        if (isfinite(c.f[y * n + col]) && isfinite(c.f[mn + y * n + col])) last = y;
+        if (isfinite(x.f[y * n + col]) && isfinite(x.f[mn + y * n + col])) last = y;
         near[y * n + col] = last;
       }
       int next = -1;
       for (int y = m - 1; y >= 0; --y) {
-        if (isfinite(c.f[y * n + col]) && isfinite(c.f[mn + y * n + col])) next = y;
+        if (isfinite(x.f[y * n + col]) && isfinite(x.f[mn + y * n + col])) next = y;
         const int up = near[y * n + col];
         int r = up;
         if (up < 0 || (next >= 0 && next - y < y - up)) r = next;
         near[y * n + col] = r;
       }
     }
-    __syncthreads();
-    for (int e = tid; e < mn; e += nt) {
-      if (isfinite(c.f[e]) && isfinite(c.f[mn + e])) continue;
-      const int y = e / n, x = e % n;
+    cluster_barrier(c);
+    for (int e = gt; e < mn; e += gn) {
+      if (isfinite(x.f[e]) && isfinite(x.f[mn + e])) continue;
+      const int y = e / n, xx = e % n;
       long long best = -1;
       int br = 0, bc = 0;
       for (int col = 0; col < n; ++col) {
         const int r = near[y * n + col];
         if (r < 0) continue;
-        const long long d = (long long)(col - x) * (col - x) + (long long)(r - y) * (r - y);
+        const long long d = (long long)(col - xx) * (col - xx) + (long long)(r - y) * (r - y);
         if (best < 0 || d < best) { best = d; br = r; bc = col; }
       }
-      c.t[e] = c.f[br * n + bc];
-      c.t[mn + e] = c.f[mn + br * n + bc];
+      x.zo[e] = x.f[br * n + bc];
+      x.zo[mn + e] = x.f[mn + br * n + bc];
     }
-    __syncthreads();
-    for (int e = tid; e < mn; e += nt) {
-      if (isfinite(c.f[e]) && isfinite(c.f[mn + e])) continue;
-      c.f[e] = c.t[e];
-      c.f[mn + e] = c.t[mn + e];
+    cluster_barrier(c);
+    for (int e = gt; e < mn; e += gn) {
+      if (isfinite(x.f[e]) && isfinite(x.f[mn + e])) continue;
+      x.f[e] = x.zo[e];
+      x.f[mn + e] = x.zo[mn + e];
     }
-    __syncthreads();
+    cluster_barrier(c);
   }
   // Start: the low DCT coefficients of f (one trailing block cleared), or 0.
   const int n0 = (m + 9) / 10 + 1, n1 = (n + 9) / 10 + 1;
-  for (int fi = 0; fi < 2; ++fi) {
-    if (weighted) {
-      cta_dct2(c.f + fi * mn, c.xs, tmpf, c.t + fi * mn, m, n, mats, false);
-      for (int e = tid; e < mn; e += nt)
-        if (e / n >= n0 && e % n >= n1) c.t[fi * mn + e] = 0.0;
-      __syncthreads();
-      cta_dct2(c.t + fi * mn, c.xs, tmpf, c.z + fi * mn, m, n, mats, true);
-    } else {
-      for (int e = tid; e < mn; e += nt) c.z[fi * mn + e] = 0.0;
-    }
+  if (weighted) {
+    sw_row_pass(x, false, [&](int e) { return x.f[e]; }, reinterpret_cast<float2*>(x.zo),
+                reinterpret_cast<float2*>(x.tmp));
+    cluster_barrier(c);
+    sw_col_pass(x, false, reinterpret_cast<const float2*>(x.tmp), [&](int e, double v) {
+      const int q = e >= mn ? e - mn : e;
+      x.z[e] = (q / n >= n0 && q % n >= n1) ? 0.0 : v;
+    });
+    sw_row_pass(x, true, [&](int e) { return x.z[e]; }, reinterpret_cast<float2*>(x.zo),
+                reinterpret_cast<float2*>(x.fd));
+    cluster_barrier(c);
+    sw_col_pass(x, true, reinterpret_cast<const float2*>(x.fd), [&](int e, double v) { x.z[e] = v; });
+  } else {
+    for (int e = x.e0 + tid; e < x.e1; e += kSwThreads) x.z[e] = 0.0;
   }
-  __syncthreads();
   const double rf = weighted ? 1.75 : 1.0;
   double p = fixed_p;
   bool have_p = !is_auto;
+  if (have_p) sw_announce(x, p, p, true);
   int k_last = 0;  // index of the last iteration run
   for (int k = 0; k < 100; ++k) {
     k_last = k;
-    for (int e = tid; e < 2 * mn; e += nt) {
-      const double wv = c.w[e % mn];
-      c.t[e] = wv * (c.f[e] - c.z[e]) + c.z[e];
-    }
-    __syncthreads();
-    for (int fi = 0; fi < 2; ++fi) cta_dct2(c.t + fi * mn, c.xs, tmpf, c.fd + fi * mn, m, n, mats, false);
+    sw_row_pass(x, false,
+                [&](int e) {
+                  const double wv = x.w[e >= mn ? e - mn : e];
+                  return wv * (x.f[e] - x.z[e]) + x.z[e];
+                },
+                reinterpret_cast<float2*>(x.zo), reinterpret_cast<float2*>(x.tmp));
+    cluster_barrier(c);
+    sw_col_pass(x, false, reinterpret_cast<const float2*>(x.tmp), [&](int e, double v) { x.fd[e] = v; });
     if (is_auto && ((k + 1) & k) == 0) {
-      p = sw_search(c, p, have_p, pmin, pmax);
+      cluster_barrier(c);  // the scores read every row of fd
+      p = sw_search(x, p, have_p, pmin, pmax);
       have_p = true;
+      sw_announce(x, p, p, true);
+      cluster_barrier(c);  // fd is rewritten below
     }
-    const double s = pow(10.0, p);
+    const double s = sh.s[0];
+    // The inverse row pass takes the rows of fd that this CTA just wrote and
+    // leaves its (hi, lo) results in their place.
+    sw_row_pass(x, true, [&](int e) { return x.fd[e] * rcp_fast(1.0 + s * lam2[e >= mn ? e - mn : e]); },
+                reinterpret_cast<float2*>(x.zo), reinterpret_cast<float2*>(x.fd));
+    cluster_barrier(c);
+    sw_col_pass(x, true, reinterpret_cast<const float2*>(x.fd),
+                [&](int e, double v) { x.zo[e] = rf * v + (1.0 - rf) * x.z[e]; });
+    cluster_barrier(c);
     double num = 0.0, den = 0.0;
-    for (int fi = 0; fi < 2; ++fi) {
-      for (int e = tid; e < mn; e += nt) c.t[fi * mn + e] = c.fd[fi * mn + e] * rcp_fast(1.0 + s * lam2[e]);
-      __syncthreads();
-      cta_dct2(c.t + fi * mn, c.xs, tmpf, c.tmp + mn, m, n, mats, true);
-      for (int e = tid; e < mn; e += nt) {
-        const double z0 = c.z[fi * mn + e];
-        const double z1 = rf * c.tmp[mn + e] + (1.0 - rf) * z0;
-        c.z[fi * mn + e] = z1;
+    for (int fi = 0; fi < 2; ++fi)
+      for (int e = vt; e < mn; e += kVT) {
+        const double z0 = x.z[fi * mn + e], z1 = x.zo[fi * mn + e];
         num += (z0 - z1) * (z0 - z1);
         den += z1 * z1;
       }
-      __syncthreads();
+    sw_sums(x, num, den, 0.0, 0.0);
+    double* t = x.z;
+    x.z = x.zo;
+    x.zo = t;
+    if (tid == 0) {
+      const double tol = weighted ? sqrt(sh.sums[0]) / (sqrt(sh.sums[1]) + 1e-6) : 0.0;
+      sh.go = tol > 1e-3 || isnan(tol);
     }
-    num = cta_sum(num, red);
-    den = cta_sum(den, red);
-    const double tol = weighted ? sqrt(num) / (sqrt(den) + 1e-6) : 0.0;
-    if (tid == 0) s_flag = tol <= 1e-3;
     __syncthreads();
-    if (s_flag) break;
+    if (!sh.go) break;
   }
-  for (int e = tid; e < mn; e += nt) {
-    const bool in_mask = mask && mask[e];
-    u_out[off + e] = in_mask ? 0.0 : c.z[e];
-    v_out[off + e] = in_mask ? 0.0 : c.z[mn + e];
+  for (int e = x.e0 + tid; e < x.e1; e += kSwThreads) {
+    const int fi = e >= mn ? 1 : 0, q = e - fi * mn;
+    (fi ? v_out : u_out)[off + q] = (mask && mask[q]) ? 0.0 : x.z[e];
   }
-  if (tid == 0 && p_out) p_out[pair] = p;
-  if (tid == 0 && flags) flags[pair] = smooth_flags(is_auto != 0, p, pmin, pmax, k_last == 99);
+  if (x.rank == 0 && tid == 0) {
+    if (p_out) p_out[pair] = p;
+    if (flags) flags[pair] = smooth_flags(is_auto != 0, p, pmin, pmax, k_last == 99);
+  }
 }
 
 static int smoothn_weighted(int m, int n, int n_pairs, const double* u_in, const double* v_in, double* u_out,
                             double* v_out, const uint8_t* field_mask, double s, double* p_out, void* scratch,
-                            cudaStream_t stream, int* flags) {
+                            cudaStream_t stream, int* flags, const void* tables) {
   const size_t mn = (size_t)m * n;
+  // Scratch: room of m^2 and n^2 doubles, lambda^2, n_pairs doubles, the
+  // matrices as float pairs, then the pairs' blocks.
   char* p = (char*)scratch;
-  double* cm = (double*)p; p += align_up((size_t)m * m * 8);
-  double* cn = (double*)p; p += align_up((size_t)n * n * 8);
+  p += align_up((size_t)m * m * 8);
+  float2* cnt2 = (float2*)p; p += align_up((size_t)n * n * 8);
   double* lam2 = (double*)p; p += align_up(mn * 8);
   p += align_up((size_t)n_pairs * 8);
-  float* mf = (float*)p; p += weighted_matrix_bytes(m, n);
-  const DfMats mats{mf, mf + m * m, mf + 2 * m * m, mf + 2 * m * m + n * n};
-  const int bs = 256;
-  k_dct_matrix<<<(m * m + bs - 1) / bs, bs, 0, stream>>>(m, cm);
-  k_dct_matrix<<<(n * n + bs - 1) / bs, bs, 0, stream>>>(n, cn);
-  k_split_f64<<<(m * m + bs - 1) / bs, bs, 0, stream>>>(m * m, cm, const_cast<float*>(mats.cmh),
-                                                         const_cast<float*>(mats.cml));
-  k_split_f64<<<(n * n + bs - 1) / bs, bs, 0, stream>>>(n * n, cn, const_cast<float*>(mats.cnh),
-                                                         const_cast<float*>(mats.cnl));
-  k_lambda2<<<(unsigned)((mn + bs - 1) / bs), bs, 0, stream>>>(m, n, lam2);
+  float2* cm2 = (float2*)p;
+  float2* cn2 = cm2 + (size_t)m * m;
+  p += weighted_matrix_bytes(m, n);
+  SmoothTables t{};
+  if (tables) {
+    t = kept_tables(tables, m, n);
+  } else {
+    t.cm2 = cm2; t.cn2 = cn2; t.cnt2 = cnt2; t.lam2 = lam2;
+    const int rc = build_tables(m, n, t, stream);
+    if (rc) return rc;
+  }
   const bool is_auto = !(s > 0);
   double pmin = 0, pmax = 0;
-  if (is_auto) {
-    const double h_min = 1e-3, h_max = 1.0 - h_min;
-    const int rank = (m != 1) + (n != 1);
-    const double a_max = pow(h_max, 2.0 / rank), a_min = pow(h_min, 2.0 / rank);
-    pmin = log10((pow((1.0 + sqrt(1.0 + 8.0 * a_max)) / 4.0 / a_max, 2.0) - 1.0) / 16.0);
-    pmax = log10((pow((1.0 + sqrt(1.0 + 8.0 * a_min)) / 4.0 / a_min, 2.0) - 1.0) / 16.0);
-  }
-  k_smoothn_weighted<<<n_pairs, kSwThreads, 0, stream>>>(m, n, u_in, v_in, u_out, v_out, field_mask,
-                                                          is_auto ? 0.0 : log10(s), is_auto ? 1 : 0, pmin, pmax, mats,
-                                                          lam2, (unsigned char*)p, weighted_pair_bytes(mn), p_out,
-                                                          flags);
-  return check("k_smoothn_weighted");
+  if (is_auto) gcv_bounds(m, n, &pmin, &pmax);
+  const int c = cluster_size(n_pairs);
+  return launch_cluster(k_smoothn_weighted, n_pairs, c, kSwThreads, stream, "k_smoothn_weighted", m, n, c, u_in, v_in,
+                        u_out, v_out, field_mask, is_auto ? 0.0 : log10(s), is_auto ? 1 : 0, pmin, pmax, t.cm2, t.cn2,
+                        t.cnt2, t.lam2, (unsigned char*)p, weighted_pair_bytes(mn), p_out, flags);
 }
 
 int smoothn(int m, int n, int n_pairs, const double* u_in, const double* v_in, double* u_out, double* v_out,
-            const uint8_t* field_mask, double s, double* p_out, void* scratch, cudaStream_t stream, int* flags) {
+            const uint8_t* field_mask, double s, double* p_out, void* scratch, cudaStream_t stream, int* flags,
+            const void* tables) {
   const long long mn = (long long)m * n;
   if (n_pairs == 0 || mn == 0) return PIV_OK;
   if (flags && (mn < 2 || (!field_mask && s > 0))) cudaMemsetAsync(flags, 0, sizeof(int) * n_pairs, stream);
@@ -802,62 +1197,35 @@ int smoothn(int m, int n, int n_pairs, const double* u_in, const double* v_in, d
     return check("smoothn copy");
   }
   if (field_mask)
-    return smoothn_weighted(m, n, n_pairs, u_in, v_in, u_out, v_out, field_mask, s, p_out, scratch, stream, flags);
-  SmoothScratch sc = carve(scratch, m, n, n_pairs);
-  const int bs = 256;
-  k_dct_matrix<<<(m * m + bs - 1) / bs, bs, 0, stream>>>(m, sc.cm);
-  k_dct_matrix<<<(n * n + bs - 1) / bs, bs, 0, stream>>>(n, sc.cn);
-  k_split_f64<<<(m * m + bs - 1) / bs, bs, 0, stream>>>(m * m, sc.cm, sc.cmf, sc.cmf + m * m);
-  k_split_f64<<<(n * n + bs - 1) / bs, bs, 0, stream>>>(n * n, sc.cn, sc.cnf, sc.cnf + n * n);
-  k_lambda2<<<(unsigned)((mn + bs - 1) / bs), bs, 0, stream>>>(m, n, sc.lam2, sc.lam2f);
-  // Gather u and v as [pair][field][mn] into tmp.
-  for (int f = 0; f < 2; ++f) {
-    cudaMemcpy2DAsync(sc.tmp + f * mn, 2 * mn * 8, f == 0 ? u_in : v_in, mn * 8, mn * 8, n_pairs,
-                      cudaMemcpyDeviceToDevice, stream);
-  }
-  // Forward DCT-II: rows then columns.
-  dct_pass(m, n, 2 * n_pairs, false, 0, sc.cn, sc.cnf, sc.tmp, sc.fd, stream);
-  dct_pass(m, n, 2 * n_pairs, false, 1, sc.cm, sc.cmf, sc.fd, sc.tmp, stream);
-  int rc = check("smoothn forward dct");
-  if (rc) return rc;
-  // tmp now holds the DCT coefficients.
-  double* pvec = nullptr;
-  double fixed_p = 0.0;
-  const bool gcv = !(s > 0);
-  if (gcv) {
-    // p bounds for order 2 (gpu_smoothn.py:320-338), on the host.
-    const double h_min = 1e-3, h_max = 1.0 - h_min;
-    const int rank = (m != 1) + (n != 1);
-    const double a_max = pow(h_max, 2.0 / rank), a_min = pow(h_min, 2.0 / rank);
-    const double pmin = log10((pow((1.0 + sqrt(1.0 + 8.0 * a_max)) / 4.0 / a_max, 2.0) - 1.0) / 16.0);
-    const double pmax = log10((pow((1.0 + sqrt(1.0 + 8.0 * a_min)) / 4.0 / a_min, 2.0) - 1.0) / 16.0);
-    k_f2<<<(unsigned)((mn * n_pairs + bs - 1) / bs), bs, 0, stream>>>(mn, n_pairs, sc.tmp, sc.f2, sc.f2f);
-    k_gcv<<<n_pairs, kGcvThreads, 0, stream>>>(m, n, n_pairs, sc.f2, sc.lam2, sc.f2f, sc.lam2f, pmin, pmax, sc.p,
-                                               flags);
-    pvec = sc.p;
-    rc = check("k_gcv");
-    if (rc) return rc;
-  } else {
-    fixed_p = log10(s);
-  }
+    return smoothn_weighted(m, n, n_pairs, u_in, v_in, u_out, v_out, field_mask, s, p_out, scratch, stream, flags,
+                            tables);
   if (n_pairs > 65535) return set_error(PIV_E_UNSUPPORTED, "smoothn: more than 65535 pairs in one call");
-  k_apply_gamma<<<dim3((unsigned)((2 * mn + bs - 1) / bs), (unsigned)n_pairs), bs, 0, stream>>>(mn, n_pairs, sc.lam2,
-                                                                                               pvec, fixed_p, sc.tmp);
-  // Inverse DCT (DCT-III): rows then columns.
-  dct_pass(m, n, 2 * n_pairs, true, 0, sc.cn, sc.cnf, sc.tmp, sc.fd, stream);
-  dct_pass(m, n, 2 * n_pairs, true, 1, sc.cm, sc.cmf, sc.fd, sc.tmp, stream);
-  for (int f = 0; f < 2; ++f) {
-    cudaMemcpy2DAsync(f == 0 ? u_out : v_out, mn * 8, sc.tmp + f * mn, 2 * mn * 8, mn * 8, n_pairs,
-                      cudaMemcpyDeviceToDevice, stream);
+  SmoothScratch sc = carve(scratch, m, n, n_pairs);
+  if (tables) {
+    sc.t = kept_tables(tables, m, n);
+  } else {
+    PIV_RC(build_tables(m, n, sc.t, stream));
   }
-  if (p_out) {
-    if (gcv) {
-      cudaMemcpyAsync(p_out, sc.p, n_pairs * 8, cudaMemcpyDeviceToDevice, stream);
-    } else {
-      k_fill<<<(n_pairs + 127) / 128, 128, 0, stream>>>(n_pairs, fixed_p, p_out);
-    }
+  const DctIo in{const_cast<double*>(u_in), const_cast<double*>(v_in), mn}, result{u_out, v_out, mn};
+  const DctIo fd{sc.fd, sc.fd + mn, 2 * mn}, tmp{sc.tmp, sc.tmp + mn, 2 * mn};
+  const DctGamma none{nullptr, nullptr}, gam{sc.t.lam2, sc.s};
+  // Forward DCT-II: rows, then columns.
+  PIV_RC(dct_pass<false>(m, n, 2 * n_pairs, 0, sc.t, in, tmp, none, stream));
+  PIV_RC(dct_pass<false>(m, n, 2 * n_pairs, 1, sc.t, tmp, fd, none, stream));
+  if (!(s > 0)) {
+    double pmin = 0, pmax = 0;
+    gcv_bounds(m, n, &pmin, &pmax);
+    const int c = cluster_size(n_pairs);
+    PIV_RC(launch_cluster(k_gcv, n_pairs, c, kVT / c, stream, "k_gcv", m, n, c, sc.fd, sc.f2, sc.f2f, sc.t.lam2,
+                          sc.t.lam2f, pmin, pmax, p_out, sc.s, flags));
+  } else {
+    k_fill_s<<<(n_pairs + 127) / 128, 128, 0, stream>>>(n_pairs, log10(s), sc.s, p_out);
+    PIV_RC(check("k_fill_s"));
   }
-  return check("smoothn");
+  // Inverse DCT (DCT-III): rows, their inputs scaled by 1 / (1 + s lambda^2),
+  // then columns.
+  PIV_RC(dct_pass<true>(m, n, 2 * n_pairs, 0, sc.t, fd, tmp, gam, stream));
+  return dct_pass<true>(m, n, 2 * n_pairs, 1, sc.t, tmp, result, none, stream);
 }
 
 }  // namespace piv
