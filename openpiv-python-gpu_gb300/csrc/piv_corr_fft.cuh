@@ -250,18 +250,142 @@ PIV_D void window_positive_mean(const Cplx<T>* buf, const T* limit, T* part_v, i
   __syncthreads();
 }
 
+// The small shared-memory arrays of a CTA after the twiddles (RED_BYTES).
+template <class C, typename T = typename C::T>
+struct CorrShared {
+  using L = FftLayout<C>;
+  long long* win_base;  // [WPC] element offset of each window's corner
+  T* part_v;            // [PART]
+  T* win_v;             // 4 * WPC values
+  int* part_i;          // [PART]
+  int* win_i;           // 8 * WPC ints
+  T *means, *pval;      // [2 * WPC] means of a and b (later the second-largest values), [WPC] peak values
+  int *peak, *pi, *pj, *valid;  // [WPC] flat peak index, row, column; window in use
+  PIV_D explicit CorrShared(unsigned char* red) {
+    constexpr int WPC = L::WPC;
+    win_base = reinterpret_cast<long long*>(red);
+    part_v = reinterpret_cast<T*>(red + WPC * sizeof(long long));
+    win_v = part_v + L::PART;
+    part_i = reinterpret_cast<int*>(win_v + 4 * WPC);
+    win_i = part_i + L::PART;
+    means = win_v;
+    pval = win_v + 2 * WPC;
+    peak = win_i;
+    pi = win_i + WPC;
+    pj = win_i + 2 * WPC;
+    valid = win_i + 3 * WPC;
+  }
+};
+
+// Subpixel fit, displacement, near-tie flags and S2N of the windows in slots
+// g0 .. g0 + WPC - 1, from their maps in buf and their peaks in S.
+template <class C, int N = C::N, typename T = typename C::T>
+PIV_D void corr_outputs(const CorrArgs& a, const Cplx<T>* buf, const CorrShared<C>& S, long long g0, long long total) {
+  using L = FftLayout<C>;
+  constexpr int WPC = L::WPC;
+  const int tid = threadIdx.x, ss = a.ss;
+  const bool ties = a.near_tie || a.tie_count;
+  auto win_of = [&](long long slot) -> long long { return a.win_list ? (long long)a.win_list[slot] : slot; };
+  // Subpixel fit and displacement.
+  if (tid < WPC && g0 + tid < total) {
+    const int w = tid;
+    const long long g = win_of(g0 + w);
+    const Cplx<T>* wb = buf + w * L::WIN;
+    const int i = S.pi[w], j = S.pj[w];
+    T isp = (T)i, jsp = (T)j;
+    if (i > 0 && i < N - 1 && j > 0 && j < N - 1) {
+      T c = corr_at<N, T>(wb, i, j, ss);
+      T cd = corr_at<N, T>(wb, i - 1, j, ss), cu = corr_at<N, T>(wb, i + 1, j, ss);
+      T cl = corr_at<N, T>(wb, i, j - 1, ss), cr = corr_at<N, T>(wb, i, j + 1, ss);
+      const T eps = (T)1e-7;
+      const T half = (T)0.5, two = (T)2;
+      if (a.subpixel == PIV_SUBPIXEL_GAUSSIAN) {
+        if (c > 0 && cd > 0 && cu > 0 && cl > 0 && cr > 0) {
+          c = log(c); cd = log(cd); cu = log(cu); cl = log(cl); cr = log(cr);
+          T di = div_rn(mul_rn(half, sub_rn(cd, cu)), add_rn(add_rn(sub_rn(cd, mul_rn(two, c)), cu), eps));
+          T dj = div_rn(mul_rn(half, sub_rn(cl, cr)), add_rn(add_rn(sub_rn(cl, mul_rn(two, c)), cr), eps));
+          isp = add_rn((T)i, di);
+          jsp = add_rn((T)j, dj);
+        }
+      } else if (a.subpixel == PIV_SUBPIXEL_PARABOLIC) {
+        T di = div_rn(mul_rn(half, sub_rn(cd, cu)), add_rn(add_rn(sub_rn(cd, mul_rn(two, c)), cu), eps));
+        T dj = div_rn(mul_rn(half, sub_rn(cl, cr)), add_rn(add_rn(sub_rn(cl, mul_rn(two, c)), cr), eps));
+        isp = add_rn((T)i, di);
+        jsp = add_rn((T)j, dj);
+      } else {
+        T di = div_rn(sub_rn(cu, cd), add_rn(add_rn(add_rn(cd, c), cu), eps));
+        T dj = div_rn(sub_rn(cr, cl), add_rn(add_rn(add_rn(cl, c), cr), eps));
+        isp = add_rn((T)i, di);
+        jsp = add_rn((T)j, dj);
+      }
+    }
+    T* uo = reinterpret_cast<T*>(a.u);
+    T* vo = reinterpret_cast<T*>(a.v);
+    if (S.valid[w]) {
+      uo[g] = sub_rn(jsp, (T)(N / 2));
+      vo[g] = sub_rn(isp, (T)(N / 2));
+    } else {
+      uo[g] = (T)NAN;
+      vo[g] = (T)NAN;
+    }
+    if (a.peak_i) a.peak_i[g] = i;
+    if (a.peak_j) a.peak_j[g] = j;
+    if (ties) {
+      const T best = S.pval[w], gap = best - S.means[w];
+      const bool tie = S.valid[w] && !(gap > (T)a.tie_tol * (best < 0 ? -best : best));
+      if (a.near_tie) a.near_tie[g] = tie ? 1 : 0;
+      if (tie && a.tie_count) atomicAdd(a.tie_count, 1);
+    }
+  }
+
+  // Signal-to-noise ratio.
+  if (a.s2n) {
+    T* p2 = S.win_v + 3 * WPC;  // [WPC]
+    if (a.s2n_method == PIV_S2N_PEAK2PEAK) {
+      int* peak2 = S.win_i + 4 * WPC;
+      window_argmax<C>(buf, ss, a.s2n_size, S.pi, S.pj, S.part_v, S.part_i, p2, peak2);
+      if (tid < WPC) {
+        // The reference reads the second peak value from its masked map: a
+        // value inside the excluded box reads -inf.
+        const int i2 = peak2[tid] / N, j2 = peak2[tid] % N;
+        int di = (i2 - S.pi[tid]) & (N - 1), dj = (j2 - S.pj[tid]) & (N - 1);
+        if (di > N / 2) di -= N;
+        if (dj > N / 2) dj -= N;
+        const bool inside = di >= -a.s2n_size && di <= a.s2n_size && dj >= -a.s2n_size && dj <= a.s2n_size;
+        p2[tid] = inside ? (T)-INFINITY : corr_at<N, T>(buf + tid * L::WIN, i2, j2, ss);
+      }
+    } else {
+      // peak2mean / peak2energy: mean of the positive map values, excluding
+      // values above half the first peak for peak2mean (gpu_process.py:1325-1330).
+      T* limit = S.means;  // the window means are no longer needed
+      if (tid < WPC) limit[tid] = a.s2n_method == PIV_S2N_PEAK2MEAN ? (T)0.5 * S.pval[tid] : (T)NAN;
+      __syncthreads();
+      window_positive_mean<C>(buf, limit, S.part_v, S.part_i, p2);
+    }
+    __syncthreads();
+    if (tid < WPC && g0 + tid < total) {
+      const long long g = win_of(g0 + tid);
+      const T p1 = S.pval[tid], q2 = p2[tid];
+      T s = 0;
+      if (S.valid[tid]) {
+        if (p1 > 0) s = p1 / q2;
+        if (q2 <= 0 && p1 > 0) s = (T)INFINITY;
+      }
+      reinterpret_cast<T*>(a.s2n)[g] = s;
+    }
+  }
+}
+
 template <class C, int N = C::N, typename T = typename C::T>
 __global__ void __launch_bounds__(C::NT) k_corr_fft(CorrArgs a, Cplx<T>* gbuf) {
   using L = FftLayout<C>;
   constexpr int R1 = C::R1, R2 = C::R2, WPC = C::WPC, NT = C::NT, NW = L::NW, LD = L::LD;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Cplx<T>* tw = reinterpret_cast<Cplx<T>*>(smem_raw);
-  unsigned char* red = smem_raw + L::TW_BYTES;
-  long long* win_base = reinterpret_cast<long long*>(red);  // [WPC] element offset of each window's corner
-  T* part_v = reinterpret_cast<T*>(red + WPC * sizeof(long long));
-  T* win_v = part_v + L::PART;         // 4 * WPC values
-  int* part_i = reinterpret_cast<int*>(win_v + 4 * WPC);
-  int* win_i = part_i + L::PART;       // 8 * WPC ints
+  CorrShared<C> S(smem_raw + L::TW_BYTES);
+  long long* win_base = S.win_base;
+  T* part_v = S.part_v;
+  int* part_i = S.part_i;
   Cplx<T>* buf = L::GLOBAL_BUF ? gbuf + (size_t)blockIdx.x * WPC * L::WIN
                                : reinterpret_cast<Cplx<T>*>(smem_raw + L::SMEM_SMALL);
   const int tid = threadIdx.x;
@@ -286,12 +410,9 @@ __global__ void __launch_bounds__(C::NT) k_corr_fft(CorrArgs a, Cplx<T>* gbuf) {
   const int inner0 = (a.ss - a.ws) / 2, inner1 = a.ss - inner0;  // shrink: A's window rows/cols
   const bool normalize = a.normalize || pad != 0;
   const T inv_nn = (T)1 / (T)(N * N);
-  T* means = win_v;       // [2*WPC]: mean_a, mean_b
-  int* peak = win_i;      // [WPC]: flat peak index
-  int* pi = win_i + WPC;  // [WPC]
-  int* pj = win_i + 2 * WPC;
-  T* pval = win_v + 2 * WPC;  // [WPC]
-  int* valid = win_i + 3 * WPC;
+  T* means = S.means;
+  int *peak = S.peak, *pi = S.pi, *pj = S.pj, *valid = S.valid;
+  T* pval = S.pval;
 
   for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
     const long long g0 = (long long)tile * WPC;
@@ -449,94 +570,7 @@ __global__ void __launch_bounds__(C::NT) k_corr_fft(CorrArgs a, Cplx<T>* gbuf) {
     }
     __syncthreads();
 
-    // Subpixel fit and displacement.
-    if (tid < WPC && g0 + tid < total) {
-      const int w = tid;
-      const long long g = win_id(g0 + w);
-      const Cplx<T>* wb = buf + w * L::WIN;
-      const int i = pi[w], j = pj[w];
-      T isp = (T)i, jsp = (T)j;
-      if (i > 0 && i < N - 1 && j > 0 && j < N - 1) {
-        T c = corr_at<N, T>(wb, i, j, ss);
-        T cd = corr_at<N, T>(wb, i - 1, j, ss), cu = corr_at<N, T>(wb, i + 1, j, ss);
-        T cl = corr_at<N, T>(wb, i, j - 1, ss), cr = corr_at<N, T>(wb, i, j + 1, ss);
-        const T eps = (T)1e-7;
-        const T half = (T)0.5, two = (T)2;
-        if (a.subpixel == PIV_SUBPIXEL_GAUSSIAN) {
-          if (c > 0 && cd > 0 && cu > 0 && cl > 0 && cr > 0) {
-            c = log(c); cd = log(cd); cu = log(cu); cl = log(cl); cr = log(cr);
-            T di = div_rn(mul_rn(half, sub_rn(cd, cu)), add_rn(add_rn(sub_rn(cd, mul_rn(two, c)), cu), eps));
-            T dj = div_rn(mul_rn(half, sub_rn(cl, cr)), add_rn(add_rn(sub_rn(cl, mul_rn(two, c)), cr), eps));
-            isp = add_rn((T)i, di);
-            jsp = add_rn((T)j, dj);
-          }
-        } else if (a.subpixel == PIV_SUBPIXEL_PARABOLIC) {
-          T di = div_rn(mul_rn(half, sub_rn(cd, cu)), add_rn(add_rn(sub_rn(cd, mul_rn(two, c)), cu), eps));
-          T dj = div_rn(mul_rn(half, sub_rn(cl, cr)), add_rn(add_rn(sub_rn(cl, mul_rn(two, c)), cr), eps));
-          isp = add_rn((T)i, di);
-          jsp = add_rn((T)j, dj);
-        } else {
-          T di = div_rn(sub_rn(cu, cd), add_rn(add_rn(add_rn(cd, c), cu), eps));
-          T dj = div_rn(sub_rn(cr, cl), add_rn(add_rn(add_rn(cl, c), cr), eps));
-          isp = add_rn((T)i, di);
-          jsp = add_rn((T)j, dj);
-        }
-      }
-      T* uo = reinterpret_cast<T*>(a.u);
-      T* vo = reinterpret_cast<T*>(a.v);
-      if (valid[w]) {
-        uo[g] = sub_rn(jsp, (T)(N / 2));
-        vo[g] = sub_rn(isp, (T)(N / 2));
-      } else {
-        uo[g] = (T)NAN;
-        vo[g] = (T)NAN;
-      }
-      if (a.peak_i) a.peak_i[g] = i;
-      if (a.peak_j) a.peak_j[g] = j;
-      if (ties) {
-        const T best = pval[w], gap = best - second[w];
-        const bool tie = valid[w] && !(gap > (T)a.tie_tol * (best < 0 ? -best : best));
-        if (a.near_tie) a.near_tie[g] = tie ? 1 : 0;
-        if (tie && a.tie_count) atomicAdd(a.tie_count, 1);
-      }
-    }
-
-    // Signal-to-noise ratio.
-    if (a.s2n) {
-      T* p2 = win_v + 3 * WPC;  // [WPC]
-      if (a.s2n_method == PIV_S2N_PEAK2PEAK) {
-        int* peak2 = win_i + 4 * WPC;
-        window_argmax<C>(buf, ss, a.s2n_size, pi, pj, part_v, part_i, p2, peak2);
-        if (tid < WPC) {
-          // The reference reads the second peak value from its masked map: a
-          // value inside the excluded box reads -inf.
-          const int i2 = peak2[tid] / N, j2 = peak2[tid] % N;
-          int di = (i2 - pi[tid]) & (N - 1), dj = (j2 - pj[tid]) & (N - 1);
-          if (di > N / 2) di -= N;
-          if (dj > N / 2) dj -= N;
-          const bool inside = di >= -a.s2n_size && di <= a.s2n_size && dj >= -a.s2n_size && dj <= a.s2n_size;
-          p2[tid] = inside ? (T)-INFINITY : corr_at<N, T>(buf + tid * L::WIN, i2, j2, ss);
-        }
-      } else {
-        // peak2mean / peak2energy: mean of the positive map values, excluding
-        // values above half the first peak for peak2mean (gpu_process.py:1325-1330).
-        T* limit = means;  // the window means are no longer needed
-        if (tid < WPC) limit[tid] = a.s2n_method == PIV_S2N_PEAK2MEAN ? (T)0.5 * pval[tid] : (T)NAN;
-        __syncthreads();
-        window_positive_mean<C>(buf, limit, part_v, part_i, p2);
-      }
-      __syncthreads();
-      if (tid < WPC && g0 + tid < total) {
-        const long long g = win_id(g0 + tid);
-        const T p1 = pval[tid], q2 = p2[tid];
-        T s = 0;
-        if (valid[tid]) {
-          if (p1 > 0) s = p1 / q2;
-          if (q2 <= 0 && p1 > 0) s = (T)INFINITY;
-        }
-        reinterpret_cast<T*>(a.s2n)[g] = s;
-      }
-    }
+    corr_outputs<C>(a, buf, S, g0, total);
   }
 }
 

@@ -1,0 +1,673 @@
+// Plain-form correlation for the common passes: float32, windows of ss = N / 2
+// (n_fft 2, no shrink), N = 32, 64 and 128. The same transforms, product and
+// search as k_corr_fft (piv_corr_fft.cuh), term by term, with fewer sweeps
+// over shared memory:
+//   * only the ss x ss window is stored; the zero pad is never written, and
+//     the forward passes leave its terms out (half the inputs of the first
+//     radix stage along both axes are zero);
+//   * N = 64, 128: the last forward pass along the columns, the conjugate
+//     product and the first inverse pass run on one pair of eight-point groups
+//     (the group of frequencies k2 + R2 k1 and that of the negated
+//     frequencies), in registers;
+//   * N = 32: one warp per window, one line per lane, no block barriers;
+//   * the last inverse pass forms only the real parts, scales them and finds
+//     each line's two largest values on the way;
+//   * the twiddles inside the register DFTs are constants.
+// Shared-memory traffic and instruction issue bound the kernel. Measured (one
+// 1024 x 1024 pair at 50% overlap, 8-bit frames; the general kernel, then
+// this): N = 32 136 -> 64 us, N = 64 139 -> 68 us, N = 128 174 -> 92 us.
+#pragma once
+
+#include "piv_corr_common.cuh"
+#include "piv_corr_fft.cuh"
+
+namespace piv {
+
+// W_32^j = exp(-2 pi i j / 32), j < 16 (every eighth entry of c_tw256_f).
+struct TwPair {
+  float x, y;
+};
+PIV_HD constexpr TwPair tw32(int j) {
+  switch (j) {
+    case 0: return {1.0f, -0.0f};
+    case 1: return {0.9807852506637573f, -0.19509032368659973f};
+    case 2: return {0.9238795042037964f, -0.3826834261417389f};
+    case 3: return {0.8314695954322815f, -0.5555702447891235f};
+    case 4: return {0.7071067690849304f, -0.7071067690849304f};
+    case 5: return {0.5555702447891235f, -0.8314695954322815f};
+    case 6: return {0.3826834261417389f, -0.9238795042037964f};
+    case 7: return {0.19509032368659973f, -0.9807852506637573f};
+    case 8: return {-0.0f, -1.0f};
+    case 9: return {-0.19509032368659973f, -0.9807852506637573f};
+    case 10: return {-0.3826834261417389f, -0.9238795042037964f};
+    case 11: return {-0.5555702447891235f, -0.8314695954322815f};
+    case 12: return {-0.7071067690849304f, -0.7071067690849304f};
+    case 13: return {-0.8314695954322815f, -0.5555702447891235f};
+    case 14: return {-0.9238795042037964f, -0.3826834261417389f};
+    default: return {-0.9807852506637573f, -0.19509032368659973f};
+  }
+}
+
+// a w and the product's terms with the roundings written out (one product of
+// each sum rounded, the other fused), as the compiler contracts the general
+// kernel's expressions: the maps of both kernels are the same bit for bit.
+PIV_D Cplx<float> cmul_k(Cplx<float> a, float wx, float wy) {
+  return cmake<float>(__fmaf_rn(a.x, wx, -__fmul_rn(a.y, wy)), __fmaf_rn(a.y, wx, __fmul_rn(a.x, wy)));
+}
+PIV_D Cplx<float> cmul_k(Cplx<float> a, Cplx<float> w) { return cmul_k(a, w.x, w.y); }
+
+// Radix-2 stages from span LEN up of the R-point register DFT (dft_stage with
+// constant twiddles).
+template <int R, int LEN, bool INV>
+PIV_D void dft_stage_k(Cplx<float> (&y)[R]) {
+#pragma unroll
+  for (int i = 0; i < R; i += LEN) {
+#pragma unroll
+    for (int j = 0; j < LEN / 2; ++j) {
+      const Cplx<float> a = y[i + j];
+      Cplx<float> b = y[i + j + LEN / 2];
+      if (j != 0) {
+        if (LEN >= 4 && j == LEN / 4) {
+          b = INV ? cmake<float>(-b.y, b.x) : cmake<float>(b.y, -b.x);
+        } else {
+          const TwPair w = tw32(j * (32 / LEN));  // constant once unrolled
+          b = cmul_k(b, w.x, INV ? -w.y : w.y);
+        }
+      }
+      y[i + j] = cadd(a, b);
+      y[i + j + LEN / 2] = csub(a, b);
+    }
+  }
+  if constexpr (LEN < R) dft_stage_k<R, 2 * LEN, INV>(y);
+}
+
+template <int R, bool INV>
+PIV_D void dft_k(Cplx<float> (&x)[R]) {
+  Cplx<float> y[R];
+  bitrev_permute<R, float>(y, x, std::make_integer_sequence<int, R>{});
+  dft_stage_k<R, 2, INV>(y);
+#pragma unroll
+  for (int i = 0; i < R; ++i) x[i] = y[i];
+}
+
+// Forward DFT of R points of which only x[R/4 .. 3R/4) are non-zero (the
+// others are not read): of each pair (k, k + R/2) of the first stage one is
+// zero.
+template <int R>
+PIV_D void dft_half(Cplx<float> (&x)[R]) {
+  Cplx<float> y[R];
+#pragma unroll
+  for (int i = 0; i < R; i += 2) {
+    const int k = bitrev<R>(i);  // y[i] = x[k] + x[k + R/2], y[i + 1] = x[k] - x[k + R/2]
+    if (k >= R / 4) {
+      y[i] = x[k];
+      y[i + 1] = x[k];
+    } else {
+      y[i] = x[k + R / 2];
+      y[i + 1] = cmake<float>(-x[k + R / 2].x, -x[k + R / 2].y);
+    }
+  }
+  if constexpr (R > 2) dft_stage_k<R, 4, false>(y);
+#pragma unroll
+  for (int i = 0; i < R; ++i) x[i] = y[i];
+}
+
+// P = conj(A) B at frequency k from Z(k) and Z(-k) of z = a + i b.
+PIV_D Cplx<float> conj_product(Cplx<float> zk, Cplx<float> zm) {
+  const float ar = zk.x + zm.x, ai = zk.y - zm.y;
+  const float br = zk.y + zm.y, bi = zm.x - zk.x;
+  return cmake<float>(__fmul_rn(__fmaf_rn(ar, br, __fmul_rn(ai, bi)), 0.25f),
+                      __fmul_rn(__fmaf_rn(ar, bi, -__fmul_rn(ai, br)), 0.25f));
+}
+
+// Corner of window g (element offset in a frame batch); false when masked.
+PIV_D bool window_corner(const CorrArgs& a, long long g, long long& base) {
+  const int n_wins = a.m * a.n;
+  const int pair = (int)(g / n_wins), k = (int)(g - (long long)pair * n_wins);
+  const int wr = k / a.n, wc = k - wr * a.n;
+  base = pair * ((long long)a.height * a.width) + (long long)(wr * a.spacing + a.y_offset) * a.width +
+         wc * a.spacing + a.x_offset;
+  return !(a.win_mask && a.win_mask[k]);
+}
+
+// Two largest of a line's values in ascending shifted order: v enters with
+// index f.
+struct Top2 {
+  float best, second;
+  int at;
+  PIV_D void init() {
+    best = second = -INFINITY;
+    at = 0x7fffffff;
+  }
+  PIV_D void next(float v, int f) {  // f above every earlier index
+    second = fmaxf(second, fminf(v, best));
+    const bool up = v > best;
+    best = up ? v : best;
+    at = up ? f : at;
+  }
+  PIV_D void merge(const Top2& o) {
+    second = fmaxf(fmaxf(second, o.second), fminf(best, o.best));
+    const bool up = o.best > best || (o.best == best && o.at < at);
+    best = up ? o.best : best;
+    at = up ? o.at : at;
+  }
+};
+
+// ---------------------------------------------------------------------------
+// N = 64 and 128: one window per CTA, lines split as N = 8 R2.
+// ---------------------------------------------------------------------------
+template <int N_, int NT_, int MIN_CTAS_>
+struct HalfCfg {
+  static constexpr int N = N_, NT = NT_, MIN_CTAS = MIN_CTAS_;
+  using Fft = FftCfg<N, float, 8, N / 8, 1, NT>;  // layout and search of the general kernel
+};
+
+template <class H>
+__global__ void __launch_bounds__(H::NT, H::MIN_CTAS) k_corr_fft_half(CorrArgs a) {
+  using C = typename H::Fft;
+  using L = FftLayout<C>;
+  constexpr int N = H::N, NT = H::NT, SS = N / 2, PAD = N / 4, R1 = 8, R2 = N / 8, LD = L::LD, NW = NT / 32;
+  // The window means are summed by the general kernel's threads (NT0 of them,
+  // then its warps in order), so that both give the same bits.
+  constexpr int NT0 = N == 128 ? 1024 : 128, NV = NT0 / NT, PER = SS * SS / NT0, NW0 = NT0 / 32;
+  static_assert(NV >= 1 && NT % 64 == 0, "whole virtual warps per warp");
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Cplx<float>* tw = reinterpret_cast<Cplx<float>*>(smem_raw);
+  CorrShared<C> S(smem_raw + L::TW_BYTES);
+  Cplx<float>* buf = reinterpret_cast<Cplx<float>*>(smem_raw + L::SMEM_SMALL);
+  __shared__ float sum_part[2][NW0];
+  __shared__ Top2 top_part[NW];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  for (int k = tid; k < 256; k += NT) {
+    const float2 w = c_tw256_f[k];
+    tw[k] = cmake<float>(w.x, w.y);
+  }
+  const long long total = a.win_list ? (long long)*a.win_count : (long long)a.n_pairs * a.m * a.n;
+  auto tw_n = [&](int e) { return tw[(e & (N - 1)) * (256 / N)]; };
+
+  for (long long slot = blockIdx.x; slot < total; slot += gridDim.x) {
+    const long long g = a.win_list ? (long long)a.win_list[slot] : slot;
+    long long base;
+    const bool ok = window_corner(a, g, base);
+    // The window's pixels, PER per virtual thread, and the means.
+    float xa[NV][PER], xb[NV][PER];
+    auto load = [&](auto tag) {
+      using P = decltype(tag);
+      const P* fa = reinterpret_cast<const P*>(a.frame_a) + base;
+      const P* fb = reinterpret_cast<const P*>(a.frame_b) + base;
+#pragma unroll
+      for (int v = 0; v < NV; ++v)
+#pragma unroll
+        for (int q = 0; q < PER; ++q) {
+          const int e = tid + v * NT + q * NT0, r = e / SS, c = e % SS;
+          const long long at = (long long)r * a.width + c;
+          xa[v][q] = ok ? (float)__ldg(fa + at) : 0.f;
+          xb[v][q] = ok ? (float)__ldg(fb + at) : 0.f;
+        }
+    };
+    switch (a.pixel_type) {
+      case PIV_PIXEL_U8: load(uint8_t{}); break;
+      case PIV_PIXEL_U16: load(uint16_t{}); break;
+      case PIV_PIXEL_F32: load(float{}); break;
+      default: load(double{}); break;
+    }
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      float sa = 0.f, sb = 0.f;
+#pragma unroll
+      for (int q = 0; q < PER; ++q) {
+        sa += xa[v][q];
+        sb += xb[v][q];
+      }
+      sa = warp_sum(sa);
+      sb = warp_sum(sb);
+      if (lane == 0) {
+        sum_part[0][warp + v * NW] = sa;
+        sum_part[1][warp + v * NW] = sb;
+      }
+    }
+    __syncthreads();
+    if (lane == 0 && warp < 2) {
+      float t = 0.f;
+      for (int q = 0; q < NW0; ++q) t += sum_part[warp][q];
+      S.means[warp] = t / (float)(SS * SS);
+    }
+    __syncthreads();
+    {
+      const float ma = S.means[0], mb = S.means[1];
+#pragma unroll
+      for (int v = 0; v < NV; ++v)
+#pragma unroll
+        for (int q = 0; q < PER; ++q) {
+          const int e = tid + v * NT + q * NT0, r = e / SS, c = e % SS;
+          buf[(PAD + r) * LD + PAD + c] = ok ? cmake<float>(xa[v][q] - ma, xb[v][q] - mb) : cmake<float>(0.f, 0.f);
+        }
+    }
+    __syncthreads();
+
+    // Rows of the window: R2-point DFTs, then eight-point ones. Lanes take
+    // adjacent rows (bank-conflict free), the in-line index is the warp's.
+#pragma unroll 1
+    for (int it0 = 0; it0 < SS * R1; it0 += NT) {
+      const int it = it0 + tid, l = it % SS, n1 = it / SS;
+      Cplx<float>* p = buf + (PAD + l) * LD + n1;
+      Cplx<float> x[R2];
+#pragma unroll
+      for (int k = R2 / 4; k < 3 * R2 / 4; ++k) x[k] = p[k * R1];
+      dft_half<R2>(x);
+      if (n1 != 0) {
+#pragma unroll
+        for (int k = 1; k < R2; ++k) x[k] = cmul_k(x[k], tw_n(n1 * k));
+      }
+#pragma unroll
+      for (int k = 0; k < R2; ++k) p[k * R1] = x[k];
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int it0 = 0; it0 < SS * R2; it0 += NT) {
+      const int it = it0 + tid, l = it % SS, k2 = it / SS;
+      Cplx<float>* p = buf + (PAD + l) * LD + R1 * k2;
+      Cplx<float> x[R1];
+#pragma unroll
+      for (int k = 0; k < R1; ++k) x[k] = p[k];
+      dft_k<R1, false>(x);
+#pragma unroll
+      for (int k = 0; k < R1; ++k) p[k] = x[k];
+    }
+    __syncthreads();
+    // Columns: R2-point DFTs over the window's rows.
+#pragma unroll 1
+    for (int it0 = 0; it0 < N * R1; it0 += NT) {
+      const int it = it0 + tid, l = it % N, n1 = it / N;
+      Cplx<float>* p = buf + n1 * LD + l;
+      Cplx<float> x[R2];
+#pragma unroll
+      for (int k = R2 / 4; k < 3 * R2 / 4; ++k) x[k] = p[k * R1 * LD];
+      dft_half<R2>(x);
+      if (n1 != 0) {
+#pragma unroll
+        for (int k = 1; k < R2; ++k) x[k] = cmul_k(x[k], tw_n(n1 * k));
+      }
+#pragma unroll
+      for (int k = 0; k < R2; ++k) p[k * R1 * LD] = x[k];
+    }
+    __syncthreads();
+    // Column frequencies: position p holds frequency p / 8 + R2 (p % 8). The
+    // group (column c, rows 8 k2 .. 8 k2 + 7) holds the row frequencies k2 +
+    // R2 k1; the negated frequencies form the group (c', rows 8 (R2 - k2) % N
+    // ..), k1 -> 7 - k1 (k2 > 0) or -k1 mod 8 (k2 = 0). One item takes both
+    // groups: eight-point DFTs, product, eight-point inverse DFTs.
+#pragma unroll 1
+    for (int it = tid; it < N * R2 / 2; it += NT) {
+      int c, cm, k2;
+      bool self = false;  // both groups are their own negatives
+      auto negated = [](int q) {
+        const int ca = q >> 3, cb = q & 7;
+        return ca ? 8 * (R2 - ca) + 7 - cb : ((8 - cb) & 7);
+      };
+      if (it < (R2 / 2 - 1) * N) {
+        k2 = 1 + it / N;
+        c = it % N;
+        cm = negated(c);
+      } else {
+        // k2 = 0 and R2 / 2 pair with themselves: half of the columns each.
+        const int j = it - (R2 / 2 - 1) * N, jj = j % (N / 2);
+        k2 = j < N / 2 ? 0 : R2 / 2;
+        constexpr int M = 8 * (R2 / 2 - 1);
+        const int q = jj - M;
+        c = jj < M ? 8 + jj : (q < 3 ? q + 1 : (q == 3 ? 0 : 8 * (R2 / 2) + q - 4));
+        cm = q == 3 ? 4 : negated(c);
+        self = q == 3;
+      }
+      Cplx<float>* pg = buf + 8 * k2 * LD + c;
+      Cplx<float>* ph = buf + 8 * ((R2 - k2) % R2) * LD + cm;
+      Cplx<float> x[R1], y[R1];
+#pragma unroll
+      for (int k = 0; k < R1; ++k) {
+        x[k] = pg[k * LD];
+        y[k] = ph[k * LD];
+      }
+      dft_k<R1, false>(x);
+      dft_k<R1, false>(y);
+      if (!self) {
+        if (k2 == 0) {
+#pragma unroll
+          for (int k = 0; k < R1; ++k) {
+            const Cplx<float> q = conj_product(x[k], y[(8 - k) & 7]);
+            x[k] = q;
+            y[(8 - k) & 7] = cconj(q);
+          }
+        } else {
+#pragma unroll
+          for (int k = 0; k < R1; ++k) {
+            const Cplx<float> q = conj_product(x[k], y[7 - k]);
+            x[k] = q;
+            y[7 - k] = cconj(q);
+          }
+        }
+      } else {
+        Cplx<float> u[R1], w[R1];
+#pragma unroll
+        for (int k = 0; k < R1; ++k) {
+          u[k] = k2 == 0 ? conj_product(x[k], x[(8 - k) & 7]) : conj_product(x[k], x[7 - k]);
+          w[k] = k2 == 0 ? conj_product(y[k], y[(8 - k) & 7]) : conj_product(y[k], y[7 - k]);
+        }
+#pragma unroll
+        for (int k = 0; k < R1; ++k) {
+          x[k] = u[k];
+          y[k] = w[k];
+        }
+      }
+      dft_k<R1, true>(x);
+      dft_k<R1, true>(y);
+#pragma unroll
+      for (int k = 0; k < R1; ++k) {
+        pg[k * LD] = x[k];
+        ph[k * LD] = y[k];
+      }
+    }
+    __syncthreads();
+    // Inverse along the columns (R2-point part), then the rows.
+#pragma unroll 1
+    for (int it0 = 0; it0 < N * R1; it0 += NT) {
+      const int it = it0 + tid, l = it % N, n1 = it / N;
+      Cplx<float>* p = buf + n1 * LD + l;
+      Cplx<float> x[R2];
+#pragma unroll
+      for (int k = 0; k < R2; ++k) x[k] = p[k * R1 * LD];
+      if (n1 != 0) {
+#pragma unroll
+        for (int k = 1; k < R2; ++k) x[k] = cmul_k(x[k], cconj(tw_n(n1 * k)));
+      }
+      dft_k<R2, true>(x);
+#pragma unroll
+      for (int k = 0; k < R2; ++k) p[k * R1 * LD] = x[k];
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int it0 = 0; it0 < N * R2; it0 += NT) {
+      const int it = it0 + tid, l = it % N, k2 = it / N;
+      Cplx<float>* p = buf + l * LD + R1 * k2;
+      Cplx<float> x[R1];
+#pragma unroll
+      for (int k = 0; k < R1; ++k) x[k] = p[k];
+      dft_k<R1, true>(x);
+#pragma unroll
+      for (int k = 0; k < R1; ++k) p[k] = x[k];
+    }
+    __syncthreads();
+    Top2 top;
+    top.init();
+    float sum = 0.f;  // not a number if any value is
+    const float inv_nn = 1.0f / (float)(N * N);
+#pragma unroll 1
+    for (int it0 = 0; it0 < N * R1; it0 += NT) {
+      const int it = it0 + tid, l = it % N, n1 = it / N;
+      Cplx<float>* p = buf + l * LD + n1;
+      Cplx<float> x[R2];
+#pragma unroll
+      for (int k = 0; k < R2; ++k) x[k] = p[k * R1];
+      if (n1 != 0) {
+#pragma unroll
+        for (int k = 1; k < R2; ++k) x[k] = cmul_k(x[k], cconj(tw_n(n1 * k)));
+      }
+      dft_k<R2, true>(x);
+      const int i = l ^ (N / 2);
+      Top2 line;
+      line.init();
+#pragma unroll
+      for (int q = 0; q < R2; ++q) {
+        const int k = q ^ (R2 / 2);  // ascending shifted columns j = n1 + 8 q
+        float v = x[k].x * inv_nn;
+        p[k * R1].x = v;
+        sum += v;
+        if (i == 0 || (q == 0 && n1 == 0)) v = 0.f;  // no window overlap
+        line.next(v, i * N + n1 + R1 * q);
+      }
+      top.merge(line);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      Top2 t;
+      t.best = __shfl_xor_sync(~0u, top.best, o);
+      t.second = __shfl_xor_sync(~0u, top.second, o);
+      t.at = __shfl_xor_sync(~0u, top.at, o);
+      top.merge(t);
+    }
+    if (lane == 0) top_part[warp] = top;
+    const bool bad = __syncthreads_or(is_nan(sum));
+    if (bad) {
+      // Values that are not numbers: the general search's order.
+      window_argmax<C>(buf, SS, -1, nullptr, nullptr, S.part_v, S.part_i, S.pval, S.peak, S.part_v + NW, S.means);
+      if (tid == 0) {
+        S.pi[0] = S.peak[0] / N;
+        S.pj[0] = S.peak[0] % N;
+      }
+    } else if (tid == 0) {
+      Top2 t = top_part[0];
+      for (int w = 1; w < NW; ++w) t.merge(top_part[w]);
+      S.pval[0] = t.best;
+      S.means[0] = t.second;
+      S.peak[0] = t.at;
+      S.pi[0] = t.at / N;
+      S.pj[0] = t.at % N;
+    }
+    if (tid == 0) S.valid[0] = ok ? 1 : 0;
+    if (a.maps || a.s2n) __syncthreads();
+    if (a.maps) {
+      float* mo = reinterpret_cast<float*>(a.maps) + g * N * N;
+      for (int f = tid; f < N * N; f += NT) mo[f] = corr_at<N, float>(buf, f / N, f % N, SS);
+      __syncthreads();
+    }
+    corr_outputs<C>(a, buf, S, slot, total);
+    if (a.s2n) __syncthreads();
+    // The next window's means need two barriers before its pixels replace
+    // this window's map, so the fit above is done by then.
+  }
+}
+
+// ---------------------------------------------------------------------------
+// N = 32: one warp per window, line l in lane l.
+// ---------------------------------------------------------------------------
+static constexpr int kWarpFftWarps = 4, kWarpFftCtas = 4;
+
+__global__ void __launch_bounds__(32 * kWarpFftWarps, kWarpFftCtas) k_corr_fft_warp32(CorrArgs a) {
+  constexpr int N = 32, SS = 16, PAD = 8, LD = N + 1;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  Cplx<float>* buf = reinterpret_cast<Cplx<float>*>(smem_raw) + warp * N * LD;
+  const long long total = a.win_list ? (long long)*a.win_count : (long long)a.n_pairs * a.m * a.n;
+  const float inv_nn = 1.0f / (float)(N * N);
+  const bool ties = a.near_tie || a.tie_count;
+  for (long long slot = (long long)blockIdx.x * kWarpFftWarps + warp; slot < total;
+       slot += (long long)gridDim.x * kWarpFftWarps) {
+    const long long g = a.win_list ? (long long)a.win_list[slot] : slot;
+    long long base;
+    const bool ok = window_corner(a, g, base);
+    // Pixels e = lane + 32 v + 128 q: the sums of the general kernel's 128
+    // threads (pairs e, e + 128), then its four warps in order.
+    float xa[8], xb[8];
+    auto load = [&](auto tag) {
+      using P = decltype(tag);
+      const P* fa = reinterpret_cast<const P*>(a.frame_a) + base;
+      const P* fb = reinterpret_cast<const P*>(a.frame_b) + base;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int e = lane + 32 * q, r = e / SS, c = e % SS;
+        const long long at = (long long)r * a.width + c;
+        xa[q] = ok ? (float)__ldg(fa + at) : 0.f;
+        xb[q] = ok ? (float)__ldg(fb + at) : 0.f;
+      }
+    };
+    switch (a.pixel_type) {
+      case PIV_PIXEL_U8: load(uint8_t{}); break;
+      case PIV_PIXEL_U16: load(uint16_t{}); break;
+      case PIV_PIXEL_F32: load(float{}); break;
+      default: load(double{}); break;
+    }
+    float ta = 0.f, tb = 0.f;
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      ta += warp_sum(xa[v] + xa[v + 4]);
+      tb += warp_sum(xb[v] + xb[v + 4]);
+    }
+    const float ma = ta / (float)(SS * SS), mb = tb / (float)(SS * SS);
+    __syncwarp();  // the previous window's map has been read
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int e = lane + 32 * q, r = e / SS, c = e % SS;
+      buf[(PAD + r) * LD + PAD + c] = ok ? cmake<float>(xa[q] - ma, xb[q] - mb) : cmake<float>(0.f, 0.f);
+    }
+    __syncwarp();
+    Cplx<float> x[N];
+    // Rows of the window (lanes 0 .. 15).
+    if (lane < SS) {
+      Cplx<float>* p = buf + (PAD + lane) * LD;
+#pragma unroll
+      for (int k = PAD; k < PAD + SS; ++k) x[k] = p[k];
+      dft_half<N>(x);
+#pragma unroll
+      for (int k = 0; k < N; ++k) p[k] = x[k];
+    }
+    __syncwarp();
+    // Columns.
+#pragma unroll
+    for (int k = PAD; k < PAD + SS; ++k) x[k] = buf[k * LD + lane];
+    dft_half<N>(x);
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < N; ++k) buf[k * LD + lane] = x[k];
+    __syncwarp();
+    // Product with the column of the negated frequency (read in place), then
+    // the inverse along the columns.
+    const int cm = (N - lane) & (N - 1);
+#pragma unroll
+    for (int k = 0; k < N; ++k) x[k] = conj_product(x[k], buf[((N - k) & (N - 1)) * LD + cm]);
+    dft_k<N, true>(x);
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < N; ++k) buf[k * LD + lane] = x[k];
+    __syncwarp();
+    // Rows: real parts, scaled, with the line's two largest values.
+#pragma unroll
+    for (int k = 0; k < N; ++k) x[k] = buf[lane * LD + k];
+    dft_k<N, true>(x);
+    const int i = lane ^ (N / 2);
+    Top2 top;
+    top.init();
+    float sum = 0.f;
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
+      float v = x[q ^ (N / 2)].x * inv_nn;
+      buf[lane * LD + (q ^ (N / 2))].x = v;
+      sum += v;
+      if (i == 0 || q == 0) v = 0.f;  // no window overlap
+      top.next(v, i * N + q);
+    }
+    const bool bad = __any_sync(~0u, is_nan(sum));
+    __syncwarp();
+    if (bad) {
+      // Values that are not numbers: the general search's order.
+      float bv = -INFINITY, sv = -INFINITY;
+      int bi = 0x7fffffff;
+      for (int f = lane; f < N * N; f += 32) {
+        const float v = corr_at<N, float>(buf, f / N, f % N, SS);
+        if (argmax_better(v, f, bv, bi)) { sv = bv; bv = v; bi = f; }
+        else if (v > sv) sv = v;
+      }
+      warp_argmax2(bv, bi, sv);
+      top.best = bv;
+      top.second = sv;
+      top.at = bi;
+    } else {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        Top2 t;
+        t.best = __shfl_xor_sync(~0u, top.best, o);
+        t.second = __shfl_xor_sync(~0u, top.second, o);
+        t.at = __shfl_xor_sync(~0u, top.at, o);
+        top.merge(t);
+      }
+    }
+    if (a.maps) {
+      float* mo = reinterpret_cast<float*>(a.maps) + g * N * N;
+      for (int f = lane; f < N * N; f += 32) mo[f] = corr_at<N, float>(buf, f / N, f % N, SS);
+    }
+    // Lanes 0 .. 4 fetch the fit's values; lane 0 fits and writes.
+    const int pi = top.at / N, pj = top.at % N;
+    const bool inner = pi > 0 && pi < N - 1 && pj > 0 && pj < N - 1;
+    if (lane == 0) {
+      float isp = (float)pi, jsp = (float)pj;
+      if (inner)
+        subpixel_fit(a.subpixel, pi, pj, corr_at<N, float>(buf, pi, pj, SS), corr_at<N, float>(buf, pi - 1, pj, SS),
+                     corr_at<N, float>(buf, pi + 1, pj, SS), corr_at<N, float>(buf, pi, pj - 1, SS),
+                     corr_at<N, float>(buf, pi, pj + 1, SS), isp, jsp);
+      reinterpret_cast<float*>(a.u)[g] = ok ? sub_rn(jsp, (float)(N / 2)) : NAN;
+      reinterpret_cast<float*>(a.v)[g] = ok ? sub_rn(isp, (float)(N / 2)) : NAN;
+      if (a.peak_i) a.peak_i[g] = pi;
+      if (a.peak_j) a.peak_j[g] = pj;
+      if (ties) {
+        const float gap = top.best - top.second;
+        const bool tie = ok && !(gap > a.tie_tol * fabsf(top.best));
+        if (a.near_tie) a.near_tie[g] = tie ? 1 : 0;
+        if (tie && a.tie_count) atomicAdd(a.tie_count, 1);
+      }
+    }
+  }
+}
+
+template <class H>
+static int launch_corr_fft_half(const CorrArgs& a, cudaStream_t stream) {
+  using L = FftLayout<typename H::Fft>;
+  const long long total = (long long)a.n_pairs * a.m * a.n;
+  if (total == 0) return PIV_OK;
+  static thread_local int configured_dev = -1;
+  static thread_local int per_sm = 1;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (configured_dev != dev) {
+    cudaError_t e = cudaFuncSetAttribute(k_corr_fft_half<H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::SMEM);
+    if (e != cudaSuccess) return set_cuda_error(e, "cudaFuncSetAttribute(k_corr_fft_half)");
+    per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_corr_fft_half<H>, H::NT, L::SMEM);
+    if (per_sm < 1) per_sm = 1;
+    configured_dev = dev;
+  }
+  const long long room = (long long)sm_count() * per_sm;
+  CorrArgs b = a;
+  b.tie_tol = kTieTolF32;
+  k_corr_fft_half<H><<<(unsigned)std::min(total, room), H::NT, L::SMEM, stream>>>(b);
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? PIV_OK : set_cuda_error(e, "k_corr_fft_half launch");
+}
+
+static int launch_corr_fft_warp32(const CorrArgs& a, cudaStream_t stream) {
+  const long long total = (long long)a.n_pairs * a.m * a.n;
+  if (total == 0) return PIV_OK;
+  constexpr int smem = kWarpFftWarps * 32 * 33 * (int)sizeof(Cplx<float>);
+  static_assert(smem <= 48 * 1024, "fits the default shared memory");
+  const long long blocks = (total + kWarpFftWarps - 1) / kWarpFftWarps;
+  const long long room = (long long)sm_count() * kWarpFftCtas;
+  CorrArgs b = a;
+  b.tie_tol = kTieTolF32;
+  k_corr_fft_warp32<<<(unsigned)std::min(blocks, room), 32 * kWarpFftWarps, smem, stream>>>(b);
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? PIV_OK : set_cuda_error(e, "k_corr_fft_warp32 launch");
+}
+
+// Passes that the kernels above take.
+static bool corr_fft_half_supported(const CorrArgs& a) {
+  return a.dtype == PIV_DTYPE_F32 && (a.fft_size == 32 || a.fft_size == 64 || a.fft_size == 128) &&
+         a.fft_size == 2 * a.ss && a.ws == a.ss && !(a.fft_size == 32 && a.s2n);
+}
+
+// Threads per CTA: N = 64 six CTAs of 128 per SM (four or five: 72, 70 us); N
+// = 128, whose map takes most of an SM's shared memory, 512 (256 threads 95
+// us, 1024 with 64 registers each 133 us).
+static int correlate_fft_half(const CorrArgs& a, cudaStream_t stream) {
+  if (a.fft_size == 32) return launch_corr_fft_warp32(a, stream);
+  if (a.fft_size == 64) return launch_corr_fft_half<HalfCfg<64, 128, 6>>(a, stream);
+  return launch_corr_fft_half<HalfCfg<128, 512, 1>>(a, stream);
+}
+
+}  // namespace piv

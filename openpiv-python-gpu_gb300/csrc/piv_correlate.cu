@@ -3,6 +3,7 @@
 #include <algorithm>
 
 #include "piv_corr_fft.cuh"
+#include "piv_corr_fft_half.cuh"
 
 namespace piv {
 
@@ -70,6 +71,7 @@ int correlate_fft(const CorrArgs& a, int variant, cudaStream_t stream) {
   const FftVariant* t = fft_variants(a.fft_size, a.dtype, &n);
   if (!t) return set_error(PIV_E_UNSUPPORTED, "fft_size %d is not supported (8..256)", a.fft_size);
   if (variant < 0 || variant >= n) variant = 0;
+  if (variant == 0 && corr_fft_half_supported(a)) return correlate_fft_half(a, stream);
   return t[variant].launch(a, stream);
 }
 
