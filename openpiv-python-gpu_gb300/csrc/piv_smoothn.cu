@@ -18,6 +18,7 @@
 // results do not depend on it, bit for bit.
 #include <math.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "piv_common.cuh"
@@ -47,6 +48,14 @@ struct SmoothScratch {
   float* f2f;    // [pairs][mn] f2 in float32 (the GCV search's fast score)
   SmoothTables t;
 };
+
+// A square field has one cosine matrix.
+static void share_square(int m, int n, SmoothTables& t) {
+  if (m != n) return;
+  t.cn = t.cm;
+  t.cnf = t.cmf;
+  t.cn2 = t.cm2;
+}
 
 static size_t align_up(size_t v) { return (v + 255) / 256 * 256; }
 
@@ -88,26 +97,37 @@ static SmoothScratch carve(void* base, int m, int n, int n_pairs) {
   s.t.cmf = (float*)p; p += align_up((size_t)m * m * 8);
   s.t.cnf = (float*)p;
   s.t.cm2 = s.t.cn2 = s.t.cnt2 = nullptr;
+  share_square(m, n, s.t);
   return s;
 }
 
-// The constant tables, one thread per entry: the orthonormal DCT-II matrices
-// C[k][i] = s_k cos(pi (2i+1) k / (2 len)) and lambda^2 with lambda =
-// 2 (2 - (cos(pi i/m) + cos(pi j/n))); NULL tables are left out. One launch
-// where five small ones (two matrices, their splits, lambda^2) took 33 us of a
-// 127 x 127 smoothing.
-__global__ void k_smooth_tables(int m, int n, SmoothTables t) {
-  const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long mm = (long long)m * m, nn = (long long)n * n, mn = (long long)m * n;
-  if (id < mm + nn) {
+// The constant tables: the orthonormal DCT-II matrices C[k][i] = s_k cos(pi
+// (2i+1) k / (2 len)), one thread per entry, and lambda^2 with lambda = 2 (2 -
+// (cos(pi i/m) + cos(pi j/n))), kLamRows rows per CTA; NULL tables are left
+// out. sc: s_0 and s_k of the two lengths. One launch where five small ones
+// (two matrices, their splits, lambda^2) took 32 us for 253 x 253, this takes
+// 11 us; bound by the float64 cosines.
+static constexpr int kTabThreads = 128, kLamRows = 16;
+struct TableScale {
+  double m0, mk, n0, nk;
+};
+__global__ void __launch_bounds__(kTabThreads) k_smooth_tables(int m, int n, SmoothTables t, TableScale sc,
+                                                               int mat_blocks, int lam_cols) {
+  __shared__ double row_cos[kLamRows];
+  if ((int)blockIdx.x < mat_blocks) {
+    const long long id = (long long)blockIdx.x * kTabThreads + threadIdx.x;
+    const long long mm = (long long)m * m, nn = (long long)n * n;
+    const bool same = t.cn == t.cm && t.cnf == t.cmf && t.cn2 == t.cm2;  // one matrix for a square field
+    if (id >= mm + (same ? 0 : nn)) return;
     const bool rows = id >= mm;  // the matrix of the transform along the rows
     const int len = rows ? n : m;
     const long long e = rows ? id - mm : id;
     const int k = (int)(e / len), i = (int)(e % len);
-    const double sk = k == 0 ? sqrt(1.0 / len) : sqrt(2.0 / len);
+    const double sk = k == 0 ? (rows ? sc.n0 : sc.m0) : (rows ? sc.nk : sc.mk);
     const double c = sk * cospi((double)((2 * i + 1) * k) / (2.0 * len));
     double* cd = rows ? t.cn : t.cm;
     float* cf = rows ? t.cnf : t.cmf;
+    float2* c2 = rows ? t.cn2 : t.cm2;
     const long long ll = rows ? nn : mm;
     const float h = (float)c, l = (float)(c - (double)h);
     if (cd) cd[e] = c;
@@ -115,15 +135,20 @@ __global__ void k_smooth_tables(int m, int n, SmoothTables t) {
       cf[e] = h;
       cf[ll + e] = l;
     }
-    float2* c2 = rows ? t.cn2 : t.cm2;
     if (c2) c2[e] = make_float2(h, l);
-    if (rows && t.cnt2) t.cnt2[(long long)i * n + k] = make_float2(h, l);
-  } else if (id < mm + nn + mn) {
-    const long long e = id - mm - nn;
-    const int i = (int)(e / n), j = (int)(e % n);
-    const double l = 2.0 * (2.0 - (cos(M_PI * i / m) + cos(M_PI * j / n)));
-    t.lam2[e] = l * l;
-    if (t.lam2f) t.lam2f[e] = (float)(l * l);
+    if ((rows || same) && t.cnt2) t.cnt2[(long long)i * n + k] = make_float2(h, l);
+    return;
+  }
+  const int q = blockIdx.x - mat_blocks, i0 = (q / lam_cols) * kLamRows;
+  const int j = (q % lam_cols) * kTabThreads + threadIdx.x;
+  if (threadIdx.x < kLamRows) row_cos[threadIdx.x] = cos(M_PI * (i0 + (int)threadIdx.x) / m);
+  const double col_cos = cos(M_PI * j / n);
+  __syncthreads();
+  if (j >= n) return;
+  for (int i = i0; i < min(i0 + kLamRows, m); ++i) {
+    const double l = 2.0 * (2.0 - (row_cos[i - i0] + col_cos));
+    t.lam2[(long long)i * n + j] = l * l;
+    if (t.lam2f) t.lam2f[(long long)i * n + j] = (float)(l * l);
   }
 }
 
@@ -139,8 +164,12 @@ static int check(const char* what) {
   } while (0)
 
 static int build_tables(int m, int n, const SmoothTables& t, cudaStream_t stream) {
-  const long long total = (long long)m * m + (long long)n * n + (long long)m * n;
-  k_smooth_tables<<<(unsigned)((total + 127) / 128), 128, 0, stream>>>(m, n, t);
+  const TableScale sc{sqrt(1.0 / m), sqrt(2.0 / m), sqrt(1.0 / n), sqrt(2.0 / n)};
+  const long long entries = (long long)m * m + (long long)n * n;
+  const long long mat = (entries + kTabThreads - 1) / kTabThreads;
+  const long long lam_cols = (n + kTabThreads - 1) / kTabThreads, lam_rows = (m + kLamRows - 1) / kLamRows;
+  k_smooth_tables<<<(unsigned)(mat + lam_cols * lam_rows), kTabThreads, 0, stream>>>(m, n, t, sc, (int)mat,
+                                                                                     (int)lam_cols);
   return check("k_smooth_tables");
 }
 
@@ -163,6 +192,7 @@ static SmoothTables kept_tables(const void* base, int m, int n) {
   t.cnt2 = (float2*)p; p += align_up(nn);
   t.lam2 = (double*)p; p += align_up(mn * 8);
   t.lam2f = (float*)p;
+  share_square(m, n, t);
   return t;
 }
 
@@ -277,10 +307,12 @@ struct DctIo {
   PIV_D double* field(long long f) const { return ((f & 1) ? v : u) + (f >> 1) * stride; }
 };
 // The factor 1 / (1 + s lambda^2) on the inputs of the inverse row pass (lam2
-// NULL: none); s of pair k at s[k].
+// NULL: none): s of pair k is s[k], or `given` for every pair.
 struct DctGamma {
   const double* lam2;
   const double* s;
+  double given;
+  PIV_D double of(long long pair) const { return s ? s[pair] : given; }
 };
 
 // out[b][i][l] = sum_j in[b][i][j] * c[l][j]       (transform along rows, mode 0)
@@ -361,6 +393,7 @@ __global__ void __launch_bounds__(kDctThreads) k_dct_lines(int m, int n, int bat
                                                            const double* __restrict__ cd, DctIo in, DctIo out,
                                                            DctGamma gam) {
   extern __shared__ double dsm[];
+  const int nt = blockDim.x;
   const int L = cols ? m : n;
   const long long n_lines = (long long)batch * (cols ? n : m);
   const long long l0 = (long long)blockIdx.x * kDctLines;
@@ -370,34 +403,43 @@ __global__ void __launch_bounds__(kDctThreads) k_dct_lines(int m, int n, int bat
   float* fs = reinterpret_cast<float*>(dsm + L * S);  // DF: 4 hc S floats after xs
   const float* ch = cf;
   const float* cl = cf + (size_t)L * L;
-  // Field and first element of a line, and the step between its elements.
-  const int per = cols ? n : m;  // lines per field
-  const int step = cols ? n : 1;
-  // Load: coalesced along the line for rows, across lines for columns.
-  for (int idx = threadIdx.x; idx < kDctLines * L; idx += kDctThreads) {
-    int e, l;
-    if (cols) { e = idx / kDctLines; l = idx % kDctLines; }
-    else { l = idx / L; e = idx % L; }
-    const long long line = l0 + l;
-    double x = 0.0;
-    if (line < n_lines) {
-      const long long f = line / per;
-      const int q = (int)(line % per), at = (cols ? q : q * n) + e * step;
-      x = in.field(f)[at];
-      if (INV && gam.lam2) x = rcp_fast(1.0 + gam.s[f >> 1] * gam.lam2[at]) * x;
-    }
-    xs[e * S + l] = x;
+  // The lines' places, found once per line: first elements of input and
+  // output, of the line in lambda^2, and s of its pair.
+  __shared__ const double* src_s[kDctLines];
+  __shared__ double* dst_s[kDctLines];
+  __shared__ int at_s[kDctLines];
+  __shared__ double s_s[kDctLines];
+  const int step = cols ? n : 1;  // between the elements of a line
+  if (threadIdx.x < kDctLines) {
+    const long long line = l0 + threadIdx.x, per = cols ? n : m;
+    const long long f = line < n_lines ? line / per : 0;
+    const int q = line < n_lines ? (int)(line - f * per) : 0, at = cols ? q : q * n;
+    src_s[threadIdx.x] = line < n_lines ? in.field(f) + at : nullptr;
+    dst_s[threadIdx.x] = line < n_lines ? out.field(f) + at : nullptr;
+    at_s[threadIdx.x] = at;
+    s_s[threadIdx.x] = INV && gam.lam2 ? gam.of(f >> 1) : 0.0;
   }
   __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = kDctThreads / 32;
-  const int split_n = gridDim.y, share = blockIdx.y;
-  const long long my_line = l0 + lane;
-  const bool mine = my_line < n_lines;
-  double* dst = nullptr;  // this lane's output line
-  if (mine) {
-    const int q = (int)(my_line % per);
-    dst = out.field(my_line / per) + (cols ? q : (long long)q * n);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = nt / 32;
+  auto fetch = [&](int l, int e) {
+    const double* p = src_s[l];
+    double x = p ? p[(long long)e * step] : 0.0;
+    if (INV && gam.lam2) x = rcp_fast(1.0 + s_s[l] * gam.lam2[at_s[l] + e * step]) * x;
+    xs[e * S + l] = x;
+  };
+  // Coalesced along the line for rows, across lines for columns.
+  if (cols) {
+#pragma unroll 8
+    for (int e = warp; e < L; e += nw) fetch(lane, e);
+  } else {
+#pragma unroll 4
+    for (unsigned idx = threadIdx.x; idx < (unsigned)(kDctLines * L); idx += nt)
+      fetch((int)(idx / (unsigned)L), (int)(idx % (unsigned)L));
   }
+  __syncthreads();
+  const int split_n = gridDim.y, share = blockIdx.y;
+  double* dst = dst_s[lane];  // this lane's output line
+  const bool mine = dst != nullptr;
   auto split = [](double x, float& hi, float& lo) {
     hi = (float)x;
     lo = (float)(x - (double)hi);
@@ -447,29 +489,28 @@ __global__ void __launch_bounds__(kDctThreads) k_dct_lines(int m, int n, int bat
       }
     } else {
       // Two outputs of one parity per turn share the loaded sums.
-      for (int g = share * nw + warp; 4 * g < L; g += nw * split_n)
-        for (int par = 0; par < 2; ++par) {
-          const int k0 = 4 * g + par, k1 = k0 + 2;
-          if (k0 >= L) continue;
-          const double* c0 = cd + (long long)k0 * L;
-          const double* c1 = cd + (long long)min(k1, L - 1) * L;
-          double a0 = (L & 1) ? c0[h] * mid : 0.0, a1 = (L & 1) ? c1[h] * mid : 0.0;
-          const double* x = par ? xs + (L - 1) * S + lane : xs + lane;
-          const int xstep = par ? -S : S;
-#pragma unroll 4
-          for (int i = 0; i < h; ++i, x += xstep) {
-            a0 = fma(c0[i], *x, a0);
-            a1 = fma(c1[i], *x, a1);
-          }
-          if (mine) dst[(long long)k0 * step] = a0;
-          if (mine && k1 < L) dst[(long long)k1 * step] = a1;
+      for (int g = share * nw + warp; 2 * g < L + 2; g += nw * split_n) {
+        const int par = g & 1, k0 = 4 * (g >> 1) + par, k1 = k0 + 2;
+        if (k0 >= L) continue;
+        const double* c0 = cd + (long long)k0 * L;
+        const double* c1 = cd + (long long)min(k1, L - 1) * L;
+        double a0 = (L & 1) ? c0[h] * mid : 0.0, a1 = (L & 1) ? c1[h] * mid : 0.0;
+        const double* x = par ? xs + (L - 1) * S + lane : xs + lane;
+        const int xstep = par ? -S : S;
+#pragma unroll 8
+        for (int i = 0; i < h; ++i, x += xstep) {
+          a0 = fma(__ldg(c0 + i), *x, a0);
+          a1 = fma(__ldg(c1 + i), *x, a1);
         }
+        if (mine) dst[(long long)k0 * step] = a0;
+        if (mine && k1 < L) dst[(long long)k1 * step] = a1;
+      }
     }
   } else if (DF) {
     // The inputs as hi/lo floats.
     float* xh = fs;
     float* xl = fs + L * S;
-    for (int idx = threadIdx.x; idx < L * kDctLines; idx += kDctThreads) {
+    for (int idx = threadIdx.x; idx < L * kDctLines; idx += nt) {
       const int q = (idx / kDctLines) * S + idx % kDctLines;
       split(xs[q], xh[q], xl[q]);
     }
@@ -489,17 +530,20 @@ __global__ void __launch_bounds__(kDctThreads) k_dct_lines(int m, int n, int bat
     for (int g = share * nw + warp; 2 * g < hc; g += nw * split_n) {
       const int i0 = 2 * g, i1 = min(i0 + 1, hc - 1);
       double e0 = 0.0, e1 = 0.0, o0 = 0.0, o1 = 0.0;
-#pragma unroll 2
-      for (int k = 0; k < L; k += 2) {
-        const double x = xs[k * S + lane];
+#pragma unroll 4
+      for (int k = 0; k + 1 < L; k += 2) {
+        const double x = xs[k * S + lane], y = xs[(k + 1) * S + lane];
         const double* c = cd + (long long)k * L;
-        e0 = fma(c[i0], x, e0);
-        e1 = fma(c[i1], x, e1);
-        if (k + 1 < L) {
-          const double y = xs[(k + 1) * S + lane];
-          o0 = fma(c[L + i0], y, o0);
-          o1 = fma(c[L + i1], y, o1);
-        }
+        e0 = fma(__ldg(c + i0), x, e0);
+        e1 = fma(__ldg(c + i1), x, e1);
+        o0 = fma(__ldg(c + L + i0), y, o0);
+        o1 = fma(__ldg(c + L + i1), y, o1);
+      }
+      if (L & 1) {
+        const double x = xs[(L - 1) * S + lane];
+        const double* c = cd + (long long)(L - 1) * L;
+        e0 = fma(__ldg(c + i0), x, e0);
+        e1 = fma(__ldg(c + i1), x, e1);
       }
       if (!mine) continue;
       dst[(long long)i0 * step] = e0 + o0;
@@ -511,14 +555,15 @@ __global__ void __launch_bounds__(kDctThreads) k_dct_lines(int m, int n, int bat
   }
   if (!DF || split_n > 1) return;
   __syncthreads();
-  for (int idx = threadIdx.x; idx < kDctLines * L; idx += kDctThreads) {
-    int e, l;
-    if (cols) { e = idx / kDctLines; l = idx % kDctLines; }
-    else { l = idx / L; e = idx % L; }
-    const long long line = l0 + l;
-    if (line >= n_lines) continue;
-    const int q = (int)(line % per);
-    out.field(line / per)[(cols ? q : q * n) + e * step] = xs[e * S + l];
+  if (cols) {
+    for (int e = warp; e < L; e += nw)
+      if (mine) dst[(long long)e * step] = xs[e * S + lane];
+  } else {
+#pragma unroll 4
+    for (unsigned idx = threadIdx.x; idx < (unsigned)(kDctLines * L); idx += nt) {
+      const int l = (int)(idx / (unsigned)L), e = (int)(idx % (unsigned)L);
+      if (dst_s[l]) dst_s[l][e] = xs[e * S + l];
+    }
   }
 }
 
@@ -528,16 +573,18 @@ __global__ void k_apply_gamma(long long mn, int n_pairs, DctGamma gam, double* _
   if (t >= 2 * mn) return;
   const long long e = t % mn;
   double* f = fd + (long long)pair * 2 * mn + t;
-  *f = rcp_fast(1.0 + gam.s[pair] * gam.lam2[e]) * *f;
+  *f = rcp_fast(1.0 + gam.of(pair) * gam.lam2[e]) * *f;
 }
 
 // One DCT pass over `batch` fields: forward (DCT-II) or inverse (DCT-III)
 // along rows (cols = 0, tables of size n) or columns (cols = 1, size m). Lines
 // of up to kDctMaxLen positions take the double-float products, longer ones
 // the float64 products (the double-float error grows with the length), both
-// staged with the symmetric split. Measured: 63 x 63, one pair, 18 -> 11 us
-// per pass by the shares; 253 x 253, one pair, 70 us per pass by plain float64
-// dot products, 55 us so (31 us of it at the float64 rate).
+// staged with the symmetric split. Measured, the four passes of one pair: 31 x
+// 31 30 us, 253 x 253 200 us (plain float64 dot products 283 us), 170 x 137
+// 106 us (87 us, plus 5 us for gamma and 6 us for the copies, which are part
+// of these passes); 16 pairs of 253 x 253 2.13 ms (3.36 ms), of which 1.65 ms
+// at the float64 rate.
 template <bool INV>
 static int dct_pass(int m, int n, int batch, int cols, const SmoothTables& t, DctIo in, DctIo out, DctGamma gam,
                     cudaStream_t stream) {
@@ -559,21 +606,21 @@ static int dct_pass(int m, int n, int batch, int cols, const SmoothTables& t, Dc
   const double* cd = cols ? t.cm : t.cn;
   const long long blocks = (n_lines + kDctLines - 1) / kDctLines;
   // Shares of the outputs: as many as the SMs take, each warp of a share
-  // with at least one output.
-  const int turns = df ? (INV ? (L + 1) / 2 : L) : (L + 3) / 4;
-  int shares = (turns + kDctThreads / 32 - 1) / (kDctThreads / 32);
+  // with at least one turn (fewer warps per CTA stage the lines too slowly).
+  const int turns = df ? (INV ? (L + 1) / 2 : L) : (INV ? (L + 3) / 4 : (L + 1) / 2);
   const long long room = blocks < sm_count() ? sm_count() / blocks : 1;
-  if (shares > room) shares = (int)room;
+  const int shares = (int)std::min<long long>((turns + kDctThreads / 32 - 1) / (kDctThreads / 32), room);
+  const int threads = kDctThreads;
   const dim3 grid((unsigned)blocks, (unsigned)shares);
   if (df) {
     const size_t smem = (size_t)(L + 2 * ((L + 1) / 2)) * (kDctLines + 1) * sizeof(double);
-    k_dct_lines<INV, true><<<grid, kDctThreads, smem, stream>>>(m, n, batch, cols, cf, cd, in, out, gam);
+    k_dct_lines<INV, true><<<grid, threads, smem, stream>>>(m, n, batch, cols, cf, cd, in, out, gam);
   } else {
     const size_t smem = (size_t)L * (kDctLines + 1) * sizeof(double);
     cudaError_t e = cudaFuncSetAttribute(k_dct_lines<INV, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          kDctLongLen * (kDctLines + 1) * (int)sizeof(double));
     if (e != cudaSuccess) return set_cuda_error(e, "cudaFuncSetAttribute(k_dct_lines)");
-    k_dct_lines<INV, false><<<grid, kDctThreads, smem, stream>>>(m, n, batch, cols, cf, cd, in, out, gam);
+    k_dct_lines<INV, false><<<grid, threads, smem, stream>>>(m, n, batch, cols, cf, cd, in, out, gam);
   }
   return check("k_dct_lines");
 }
@@ -769,12 +816,9 @@ k_gcv(int m, int n, int c, const double* __restrict__ fd, double* __restrict__ f
   }
 }
 
-// A given parameter: s = 10^p of every pair (and p itself).
-__global__ void k_fill_s(int count, double p, double* s, double* p_out) {
+__global__ void k_fill(int count, double value, double* out) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= count) return;
-  s[t] = pow(10.0, p);
-  if (p_out) p_out[t] = p;
+  if (t < count) out[t] = value;
 }
 
 // Bounds of p = log10(s) for order 2 (gpu_smoothn.py:320-338), on the host.
@@ -1173,6 +1217,7 @@ static int smoothn_weighted(int m, int n, int n_pairs, const double* u_in, const
     t = kept_tables(tables, m, n);
   } else {
     t.cm2 = cm2; t.cn2 = cn2; t.cnt2 = cnt2; t.lam2 = lam2;
+    share_square(m, n, t);
     const int rc = build_tables(m, n, t, stream);
     if (rc) return rc;
   }
@@ -1208,7 +1253,8 @@ int smoothn(int m, int n, int n_pairs, const double* u_in, const double* v_in, d
   }
   const DctIo in{const_cast<double*>(u_in), const_cast<double*>(v_in), mn}, result{u_out, v_out, mn};
   const DctIo fd{sc.fd, sc.fd + mn, 2 * mn}, tmp{sc.tmp, sc.tmp + mn, 2 * mn};
-  const DctGamma none{nullptr, nullptr}, gam{sc.t.lam2, sc.s};
+  const DctGamma none{nullptr, nullptr, 0.0};
+  DctGamma gam{sc.t.lam2, sc.s, 0.0};
   // Forward DCT-II: rows, then columns.
   PIV_RC(dct_pass<false>(m, n, 2 * n_pairs, 0, sc.t, in, tmp, none, stream));
   PIV_RC(dct_pass<false>(m, n, 2 * n_pairs, 1, sc.t, tmp, fd, none, stream));
@@ -1219,8 +1265,10 @@ int smoothn(int m, int n, int n_pairs, const double* u_in, const double* v_in, d
     PIV_RC(launch_cluster(k_gcv, n_pairs, c, kVT / c, stream, "k_gcv", m, n, c, sc.fd, sc.f2, sc.f2f, sc.t.lam2,
                           sc.t.lam2f, pmin, pmax, p_out, sc.s, flags));
   } else {
-    k_fill_s<<<(n_pairs + 127) / 128, 128, 0, stream>>>(n_pairs, log10(s), sc.s, p_out);
-    PIV_RC(check("k_fill_s"));
+    gam.s = nullptr;
+    gam.given = pow(10.0, log10(s));
+    if (p_out) k_fill<<<(n_pairs + 127) / 128, 128, 0, stream>>>(n_pairs, log10(s), p_out);
+    PIV_RC(check("k_fill"));
   }
   // Inverse DCT (DCT-III): rows, their inputs scaled by 1 / (1 + s lambda^2),
   // then columns.
