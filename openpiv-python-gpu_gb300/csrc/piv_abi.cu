@@ -155,6 +155,8 @@ struct piv_plan {
   int* status = nullptr;      // device status word of bounded device-side waits
   int* tie_counts = nullptr;  // [n_iters] near-tie windows of the last run per iteration
   int* tie_list = nullptr;    // refined tensor form: near-tie windows of a pass (max_pairs * max windows) + count
+  int* f64_lists = nullptr;   // float64: windows that a pass's search leaves open (set_f64_lists)
+  size_t f64_windows = 0;
   float* win_means = nullptr; // refined tensor form: window means of a pass (max_pairs * max windows * 2)
   uint8_t* outliers = nullptr;
   double* u_final = nullptr;
@@ -457,6 +459,10 @@ int piv_plan_create(const piv_config* cfg, piv_plan** out) {
     rc = plan_alloc_t(p, &p->tie_list, max_mn * P + 1);
     if (rc == PIV_OK) rc = plan_alloc_t(p, &p->win_means, 2 * max_mn * P);
   }
+  if (rc == PIV_OK && cfg->dtype == PIV_DTYPE_F64) {
+    p->f64_windows = max_mn * P;
+    rc = plan_alloc_t(p, &p->f64_lists, f64_list_ints(p->f64_windows));
+  }
   if (rc == PIV_OK) {
     const size_t cnt = p->st.back().mn * P;
     rc = plan_alloc_t(p, &p->outliers, cnt);
@@ -674,6 +680,7 @@ static int run_pre(piv_plan* p, int k, RunCtx& x, cudaStream_t s, CorrArgs& c) {
     c.tie_list_count = p->tie_list;
     c.win_means = p->win_means;
   }
+  if (p->f64_lists) set_f64_lists(c, p->f64_lists, p->f64_windows);
   st.corr = c;
   st.corr_valid = true;
   return PIV_OK;
@@ -882,12 +889,27 @@ int piv_correlate(const piv_geometry* g, int n_pairs, const void* frames_a, cons
     if (rc == PIV_OK && st != 0) rc = set_error(st, "tensor correlation: a bounded wait gave up");
     return rc;
   }
-  if (need) {
-    PIV_TRY(cuda_ok(cudaMallocAsync(&c.scratch, need, s), "cudaMallocAsync"));
-    c.scratch_bytes = need;
+  // Scratch: the transforms' buffers, then (float64) the lists of windows that
+  // the search leaves open, and the peaks where the caller wants none.
+  const size_t cnt = (size_t)n_pairs * g->m * g->n;
+  const size_t lists = f64_list_ints(cnt), ints = dtype == PIV_DTYPE_F64 && !s2n ? lists + 2 * cnt : 0;
+  void* scratch = nullptr;
+  if (need || ints) {
+    const size_t head = (need + 255) / 256 * 256;
+    PIV_TRY(cuda_ok(cudaMallocAsync(&scratch, head + ints * sizeof(int), s), "cudaMallocAsync"));
+    if (need) {
+      c.scratch = scratch;
+      c.scratch_bytes = need;
+    }
+    if (ints) {
+      int* list = (int*)((char*)scratch + head);
+      set_f64_lists(c, list, cnt);
+      if (!c.peak_i) c.peak_i = list + lists;
+      if (!c.peak_j) c.peak_j = list + lists + cnt;
+    }
   }
   int rc = correlate_fft(c, 0, s);
-  if (c.scratch) cudaFreeAsync(c.scratch, s);
+  if (scratch) cudaFreeAsync(scratch, s);
   return rc;
 }
 

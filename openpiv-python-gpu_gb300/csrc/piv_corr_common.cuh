@@ -9,23 +9,23 @@
 namespace piv {
 
 // Subpixel peak (gpu_process.py:1256-1294) from the five map values.
-PIV_D void subpixel_fit(int subpixel, int pi_, int pj, float c, float cd, float cu, float cl, float cr, float& isp,
-                        float& jsp) {
-  const float eps = 1e-7f;
-  isp = (float)pi_;
-  jsp = (float)pj;
+template <typename T>
+PIV_D void subpixel_fit(int subpixel, int pi_, int pj, T c, T cd, T cu, T cl, T cr, T& isp, T& jsp) {
+  const T eps = (T)1e-7, half = (T)0.5, two = (T)2;
+  isp = (T)pi_;
+  jsp = (T)pj;
   if (subpixel == PIV_SUBPIXEL_GAUSSIAN) {
     if (c > 0 && cd > 0 && cu > 0 && cl > 0 && cr > 0) {
-      c = logf(c); cd = logf(cd); cu = logf(cu); cl = logf(cl); cr = logf(cr);
-      isp = add_rn((float)pi_, div_rn(mul_rn(0.5f, sub_rn(cd, cu)), add_rn(add_rn(sub_rn(cd, mul_rn(2.f, c)), cu), eps)));
-      jsp = add_rn((float)pj, div_rn(mul_rn(0.5f, sub_rn(cl, cr)), add_rn(add_rn(sub_rn(cl, mul_rn(2.f, c)), cr), eps)));
+      c = log(c); cd = log(cd); cu = log(cu); cl = log(cl); cr = log(cr);
+      isp = add_rn((T)pi_, div_rn(mul_rn(half, sub_rn(cd, cu)), add_rn(add_rn(sub_rn(cd, mul_rn(two, c)), cu), eps)));
+      jsp = add_rn((T)pj, div_rn(mul_rn(half, sub_rn(cl, cr)), add_rn(add_rn(sub_rn(cl, mul_rn(two, c)), cr), eps)));
     }
   } else if (subpixel == PIV_SUBPIXEL_PARABOLIC) {
-    isp = add_rn((float)pi_, div_rn(mul_rn(0.5f, sub_rn(cd, cu)), add_rn(add_rn(sub_rn(cd, mul_rn(2.f, c)), cu), eps)));
-    jsp = add_rn((float)pj, div_rn(mul_rn(0.5f, sub_rn(cl, cr)), add_rn(add_rn(sub_rn(cl, mul_rn(2.f, c)), cr), eps)));
+    isp = add_rn((T)pi_, div_rn(mul_rn(half, sub_rn(cd, cu)), add_rn(add_rn(sub_rn(cd, mul_rn(two, c)), cu), eps)));
+    jsp = add_rn((T)pj, div_rn(mul_rn(half, sub_rn(cl, cr)), add_rn(add_rn(sub_rn(cl, mul_rn(two, c)), cr), eps)));
   } else {
-    isp = add_rn((float)pi_, div_rn(sub_rn(cu, cd), add_rn(add_rn(add_rn(cd, c), cu), eps)));
-    jsp = add_rn((float)pj, div_rn(sub_rn(cr, cl), add_rn(add_rn(add_rn(cl, c), cr), eps)));
+    isp = add_rn((T)pi_, div_rn(sub_rn(cu, cd), add_rn(add_rn(add_rn(cd, c), cu), eps)));
+    jsp = add_rn((T)pj, div_rn(sub_rn(cr, cl), add_rn(add_rn(add_rn(cl, c), cr), eps)));
   }
 }
 

@@ -153,6 +153,68 @@ struct Top2 {
   }
 };
 
+// Search mode (float64 passes, correlate_f64): the float32 map only finds the
+// integer peak. The window means are removed in a way that leaves rounding of
+// the differences alone: whole-number pixels less the nearest whole number of
+// the mean and then its fraction, other pixels in float64. A window is settled
+// when its two largest values are further apart than kSearchTol |a| |b| (the
+// 2-norms of the mean-removed windows); the others go to the list. The float32
+// transform's error in a map value is below 6.7 u log2(N^2) |a| |b| per
+// transform (Higham, Accuracy and Stability of Numerical Algorithms, section
+// 24.1; u = 2^-24), three transforms of N = 128: 1.7e-5 |a| |b|, so a gap of
+// 6.1e-5 |a| |b| is beyond the errors of both values.
+constexpr float kSearchTol = 1.0f / 16384.0f;
+// Gap that settles a window; infinite where the scale's intermediate values
+// leave the float32 range (nothing is settled then).
+PIV_D float search_gap(float norm_a, float norm_b) {
+  const float scale = sqrtf(norm_a) * sqrtf(norm_b);
+  return scale > 1e-25f && scale < 1e25f ? kSearchTol * scale : INFINITY;
+}
+// The open window g: a record of its candidates (values within `gap` of the
+// largest; count may exceed kCandMax), or its place in the window list.
+PIV_D void search_open(const CorrArgs& a, long long g, int count, const int* at) {
+  if (count >= 2 && count <= kCandMax) {
+    const int q = atomicAdd(a.cand_count, 1);
+    if (q < a.cand_cap) {
+      int* rec = a.cand + (long long)q * kCandInts;
+      rec[0] = (int)g;
+      rec[1] = count;
+      for (int k = 0; k < count; ++k) rec[2 + k] = at[k];
+      return;
+    }
+  }
+  a.tie_list[atomicAdd(a.tie_list_count, 1)] = (int)g;
+}
+
+// Loads CNT pixels of each frame (element k at offset of(k) from the window's
+// corner) as X: float for the plain form (any pixel type) and for whole-number
+// pixels, double for the search of float pixels.
+template <typename X, bool SEARCH, int CNT, class Of>
+PIV_D void load_window(const CorrArgs& a, long long base, bool ok, Of of, X (&xa)[CNT], X (&xb)[CNT]) {
+  auto load = [&](auto tag) {
+    using P = decltype(tag);
+    const P* fa = reinterpret_cast<const P*>(a.frame_a) + base;
+    const P* fb = reinterpret_cast<const P*>(a.frame_b) + base;
+#pragma unroll
+    for (int k = 0; k < CNT; ++k) {
+      const long long at = of(k);
+      xa[k] = ok ? (X)__ldg(fa + at) : (X)0;
+      xb[k] = ok ? (X)__ldg(fb + at) : (X)0;
+    }
+  };
+  constexpr bool whole = !SEARCH || sizeof(X) == 4, other = !SEARCH || sizeof(X) == 8;
+  if (whole && a.pixel_type == PIV_PIXEL_U8) load(uint8_t{});
+  else if (whole && a.pixel_type == PIV_PIXEL_U16) load(uint16_t{});
+  else if (other && a.pixel_type == PIV_PIXEL_F32) load(float{});
+  else if (other) load(double{});
+}
+
+// x less the window mean.
+template <bool SEARCH>
+PIV_D float less_mean(float x, float mean, float frac) {
+  return SEARCH ? (x - mean) - frac : x - mean;
+}
+
 // ---------------------------------------------------------------------------
 // N = 64 and 128: one window per CTA, lines split as N = 8 R2.
 // ---------------------------------------------------------------------------
@@ -162,7 +224,7 @@ struct HalfCfg {
   using Fft = FftCfg<N, float, 8, N / 8, 1, NT>;  // layout and search of the general kernel
 };
 
-template <class H>
+template <class H, bool SEARCH = false, typename X = float>
 __global__ void __launch_bounds__(H::NT, H::MIN_CTAS) k_corr_fft_half(CorrArgs a) {
   using C = typename H::Fft;
   using L = FftLayout<C>;
@@ -177,6 +239,9 @@ __global__ void __launch_bounds__(H::NT, H::MIN_CTAS) k_corr_fft_half(CorrArgs a
   Cplx<float>* buf = reinterpret_cast<Cplx<float>*>(smem_raw + L::SMEM_SMALL);
   __shared__ float sum_part[2][NW0];
   __shared__ Top2 top_part[NW];
+  __shared__ double dsum_part[2][SEARCH ? NW : 1], dmean[2];  // search
+  __shared__ float norm_part[2][SEARCH ? NW : 1], cand_from;
+  __shared__ int cand_n, cand_at[kCandMax];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   for (int k = tid; k < 256; k += NT) {
     const float2 w = c_tw256_f[k];
@@ -190,58 +255,107 @@ __global__ void __launch_bounds__(H::NT, H::MIN_CTAS) k_corr_fft_half(CorrArgs a
     long long base;
     const bool ok = window_corner(a, g, base);
     // The window's pixels, PER per virtual thread, and the means.
-    float xa[NV][PER], xb[NV][PER];
-    auto load = [&](auto tag) {
-      using P = decltype(tag);
-      const P* fa = reinterpret_cast<const P*>(a.frame_a) + base;
-      const P* fb = reinterpret_cast<const P*>(a.frame_b) + base;
+    X xa[NV * PER], xb[NV * PER];
+    auto elem = [&](int k) { return tid + (k / PER) * NT + (k % PER) * NT0; };
+    load_window<X, SEARCH>(a, base, ok,
+                           [&](int k) { return (long long)(elem(k) / SS) * a.width + elem(k) % SS; }, xa, xb);
+    if constexpr (!SEARCH) {
 #pragma unroll
-      for (int v = 0; v < NV; ++v)
+      for (int v = 0; v < NV; ++v) {
+        float sa = 0.f, sb = 0.f;
 #pragma unroll
         for (int q = 0; q < PER; ++q) {
-          const int e = tid + v * NT + q * NT0, r = e / SS, c = e % SS;
-          const long long at = (long long)r * a.width + c;
-          xa[v][q] = ok ? (float)__ldg(fa + at) : 0.f;
-          xb[v][q] = ok ? (float)__ldg(fb + at) : 0.f;
+          sa += xa[v * PER + q];
+          sb += xb[v * PER + q];
         }
-    };
-    switch (a.pixel_type) {
-      case PIV_PIXEL_U8: load(uint8_t{}); break;
-      case PIV_PIXEL_U16: load(uint16_t{}); break;
-      case PIV_PIXEL_F32: load(float{}); break;
-      default: load(double{}); break;
-    }
+        sa = warp_sum(sa);
+        sb = warp_sum(sb);
+        if (lane == 0) {
+          sum_part[0][warp + v * NW] = sa;
+          sum_part[1][warp + v * NW] = sb;
+        }
+      }
+    } else if constexpr (sizeof(X) == 4) {
+      int sa = 0, sb = 0;  // whole numbers: at most 4096 x 65535
 #pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      float sa = 0.f, sb = 0.f;
+      for (int k = 0; k < NV * PER; ++k) {
+        sa += (int)xa[k];
+        sb += (int)xb[k];
+      }
+      sa = __reduce_add_sync(~0u, sa);
+      sb = __reduce_add_sync(~0u, sb);
+      if (lane == 0) {
+        dsum_part[0][warp] = (double)sa;
+        dsum_part[1][warp] = (double)sb;
+      }
+    } else {
+      double sa = 0.0, sb = 0.0;
 #pragma unroll
-      for (int q = 0; q < PER; ++q) {
-        sa += xa[v][q];
-        sb += xb[v][q];
+      for (int k = 0; k < NV * PER; ++k) {
+        sa += xa[k];
+        sb += xb[k];
       }
       sa = warp_sum(sa);
       sb = warp_sum(sb);
       if (lane == 0) {
-        sum_part[0][warp + v * NW] = sa;
-        sum_part[1][warp + v * NW] = sb;
+        dsum_part[0][warp] = sa;
+        dsum_part[1][warp] = sb;
       }
     }
     __syncthreads();
     if (lane == 0 && warp < 2) {
-      float t = 0.f;
-      for (int q = 0; q < NW0; ++q) t += sum_part[warp][q];
-      S.means[warp] = t / (float)(SS * SS);
+      if constexpr (!SEARCH) {
+        float t = 0.f;
+        for (int q = 0; q < NW0; ++q) t += sum_part[warp][q];
+        S.means[warp] = t / (float)(SS * SS);
+      } else {
+        double t = 0.0;
+        for (int q = 0; q < NW; ++q) t += dsum_part[warp][q];
+        dmean[warp] = t / (double)(SS * SS);
+      }
     }
     __syncthreads();
+    float na = 0.f, nb = 0.f;  // search: sums of squares
     {
-      const float ma = S.means[0], mb = S.means[1];
+      float ma = 0.f, mb = 0.f, fa = 0.f, fb = 0.f;
+      double da = 0.0, db = 0.0;
+      if constexpr (!SEARCH) {
+        ma = S.means[0];
+        mb = S.means[1];
+      } else {
+        da = dmean[0];
+        db = dmean[1];
+        ma = (float)rint(da);
+        mb = (float)rint(db);
+        fa = (float)(da - rint(da));
+        fb = (float)(db - rint(db));
+      }
 #pragma unroll
-      for (int v = 0; v < NV; ++v)
-#pragma unroll
-        for (int q = 0; q < PER; ++q) {
-          const int e = tid + v * NT + q * NT0, r = e / SS, c = e % SS;
-          buf[(PAD + r) * LD + PAD + c] = ok ? cmake<float>(xa[v][q] - ma, xb[v][q] - mb) : cmake<float>(0.f, 0.f);
+      for (int k = 0; k < NV * PER; ++k) {
+        const int e = elem(k), r = e / SS, c = e % SS;
+        float va, vb;
+        if constexpr (sizeof(X) == 8) {
+          va = (float)(xa[k] - da);
+          vb = (float)(xb[k] - db);
+        } else {
+          va = less_mean<SEARCH>(xa[k], ma, fa);
+          vb = less_mean<SEARCH>(xb[k], mb, fb);
         }
+        if (!ok) va = vb = 0.f;
+        if (SEARCH) {
+          na = fmaf(va, va, na);
+          nb = fmaf(vb, vb, nb);
+        }
+        buf[(PAD + r) * LD + PAD + c] = cmake<float>(va, vb);
+      }
+    }
+    if (SEARCH) {
+      na = warp_sum(na);
+      nb = warp_sum(nb);
+      if (lane == 0) {
+        norm_part[0][warp] = na;
+        norm_part[1][warp] = nb;
+      }
     }
     __syncthreads();
 
@@ -452,6 +566,35 @@ __global__ void __launch_bounds__(H::NT, H::MIN_CTAS) k_corr_fft_half(CorrArgs a
       S.pi[0] = t.at / N;
       S.pj[0] = t.at % N;
     }
+    if constexpr (SEARCH) {
+      if (tid == 0) {
+        float ta = 0.f, tb = 0.f;
+        for (int w = 0; w < NW; ++w) {
+          ta += norm_part[0][w];
+          tb += norm_part[1][w];
+        }
+        const float gap = search_gap(ta, tb), best = S.pval[0];
+        a.peak_i[g] = S.pi[0];
+        a.peak_j[g] = S.pj[0];
+        if (a.near_tie) a.near_tie[g] = 0;
+        // The values that the window's candidates reach (open windows only).
+        cand_from = !ok || (!bad && best - S.means[0] > gap) ? INFINITY : (bad ? -INFINITY : best - gap);
+        cand_n = 0;
+      }
+      __syncthreads();
+      const float from = cand_from;
+      if (from == INFINITY) continue;
+      if (from > -INFINITY) {
+        for (int f = tid; f < N * N; f += NT)
+          if (corr_at<N, float>(buf, f / N, f % N, SS) >= from) {
+            const int q = atomicAdd(&cand_n, 1);
+            if (q < kCandMax) cand_at[q] = f;
+          }
+      }
+      __syncthreads();
+      if (tid == 0) search_open(a, g, cand_n, cand_at);
+      continue;
+    }
     if (tid == 0) S.valid[0] = ok ? 1 : 0;
     if (a.maps || a.s2n) __syncthreads();
     if (a.maps) {
@@ -471,6 +614,7 @@ __global__ void __launch_bounds__(H::NT, H::MIN_CTAS) k_corr_fft_half(CorrArgs a
 // ---------------------------------------------------------------------------
 static constexpr int kWarpFftWarps = 4, kWarpFftCtas = 4;
 
+template <bool SEARCH = false, typename X = float>
 __global__ void __launch_bounds__(32 * kWarpFftWarps, kWarpFftCtas) k_corr_fft_warp32(CorrArgs a) {
   constexpr int N = 32, SS = 16, PAD = 8, LD = N + 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -486,37 +630,65 @@ __global__ void __launch_bounds__(32 * kWarpFftWarps, kWarpFftCtas) k_corr_fft_w
     const bool ok = window_corner(a, g, base);
     // Pixels e = lane + 32 v + 128 q: the sums of the general kernel's 128
     // threads (pairs e, e + 128), then its four warps in order.
-    float xa[8], xb[8];
-    auto load = [&](auto tag) {
-      using P = decltype(tag);
-      const P* fa = reinterpret_cast<const P*>(a.frame_a) + base;
-      const P* fb = reinterpret_cast<const P*>(a.frame_b) + base;
+    X xa[8], xb[8];
+    load_window<X, SEARCH>(
+        a, base, ok, [&](int k) { return (long long)((lane + 32 * k) / SS) * a.width + (lane + 32 * k) % SS; }, xa, xb);
+    float ma = 0.f, mb = 0.f, fa = 0.f, fb = 0.f;
+    double da = 0.0, db = 0.0;
+    if constexpr (!SEARCH) {
+      float ta = 0.f, tb = 0.f;
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int e = lane + 32 * q, r = e / SS, c = e % SS;
-        const long long at = (long long)r * a.width + c;
-        xa[q] = ok ? (float)__ldg(fa + at) : 0.f;
-        xb[q] = ok ? (float)__ldg(fb + at) : 0.f;
+      for (int v = 0; v < 4; ++v) {
+        ta += warp_sum(xa[v] + xa[v + 4]);
+        tb += warp_sum(xb[v] + xb[v + 4]);
       }
-    };
-    switch (a.pixel_type) {
-      case PIV_PIXEL_U8: load(uint8_t{}); break;
-      case PIV_PIXEL_U16: load(uint16_t{}); break;
-      case PIV_PIXEL_F32: load(float{}); break;
-      default: load(double{}); break;
-    }
-    float ta = 0.f, tb = 0.f;
+      ma = ta / (float)(SS * SS);
+      mb = tb / (float)(SS * SS);
+    } else {
+      if constexpr (sizeof(X) == 4) {
+        int sa = 0, sb = 0;
 #pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      ta += warp_sum(xa[v] + xa[v + 4]);
-      tb += warp_sum(xb[v] + xb[v + 4]);
+        for (int k = 0; k < 8; ++k) {
+          sa += (int)xa[k];
+          sb += (int)xb[k];
+        }
+        da = (double)__reduce_add_sync(~0u, sa);
+        db = (double)__reduce_add_sync(~0u, sb);
+      } else {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          da += xa[k];
+          db += xb[k];
+        }
+        da = warp_sum(da);
+        db = warp_sum(db);
+      }
+      da /= (double)(SS * SS);
+      db /= (double)(SS * SS);
+      ma = (float)rint(da);
+      mb = (float)rint(db);
+      fa = (float)(da - rint(da));
+      fb = (float)(db - rint(db));
     }
-    const float ma = ta / (float)(SS * SS), mb = tb / (float)(SS * SS);
+    float na = 0.f, nb = 0.f;  // search: sums of squares
     __syncwarp();  // the previous window's map has been read
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int e = lane + 32 * q, r = e / SS, c = e % SS;
-      buf[(PAD + r) * LD + PAD + c] = ok ? cmake<float>(xa[q] - ma, xb[q] - mb) : cmake<float>(0.f, 0.f);
+    for (int k = 0; k < 8; ++k) {
+      const int e = lane + 32 * k, r = e / SS, c = e % SS;
+      float va, vb;
+      if constexpr (sizeof(X) == 8) {
+        va = (float)(xa[k] - da);
+        vb = (float)(xb[k] - db);
+      } else {
+        va = less_mean<SEARCH>(xa[k], ma, fa);
+        vb = less_mean<SEARCH>(xb[k], mb, fb);
+      }
+      if (!ok) va = vb = 0.f;
+      if (SEARCH) {
+        na = fmaf(va, va, na);
+        nb = fmaf(vb, vb, nb);
+      }
+      buf[(PAD + r) * LD + PAD + c] = cmake<float>(va, vb);
     }
     __syncwarp();
     Cplx<float> x[N];
@@ -589,11 +761,37 @@ __global__ void __launch_bounds__(32 * kWarpFftWarps, kWarpFftCtas) k_corr_fft_w
         top.merge(t);
       }
     }
+    if constexpr (SEARCH) {
+      const float gap = search_gap(warp_sum(na), warp_sum(nb));
+      if (lane == 0) {
+        a.peak_i[g] = top.at / N;
+        a.peak_j[g] = top.at % N;
+        if (a.near_tie) a.near_tie[g] = 0;
+      }
+      if (ok && (bad || !(top.best - top.second > gap))) {
+        const float from = bad ? INFINITY : top.best - gap;
+        int count = 0, at[kCandMax];
+        // Candidates in map order, counted by every lane.
+        for (int f0 = 0; f0 < N * N && from > -INFINITY; f0 += 32) {
+          const int f = f0 + lane;
+          unsigned hit = __ballot_sync(~0u, corr_at<N, float>(buf, f / N, f % N, SS) >= from);
+          while (hit) {
+            const int k = __ffs(hit) - 1;
+            hit &= hit - 1;
+#pragma unroll
+            for (int q = 0; q < kCandMax; ++q)
+              if (q == count) at[q] = f0 + k;
+            ++count;
+          }
+        }
+        if (lane == 0) search_open(a, g, count, at);
+      }
+      continue;
+    }
     if (a.maps) {
       float* mo = reinterpret_cast<float*>(a.maps) + g * N * N;
       for (int f = lane; f < N * N; f += 32) mo[f] = corr_at<N, float>(buf, f / N, f % N, SS);
     }
-    // Lanes 0 .. 4 fetch the fit's values; lane 0 fits and writes.
     const int pi = top.at / N, pj = top.at % N;
     const bool inner = pi > 0 && pi < N - 1 && pj > 0 && pj < N - 1;
     if (lane == 0) {
@@ -616,7 +814,7 @@ __global__ void __launch_bounds__(32 * kWarpFftWarps, kWarpFftCtas) k_corr_fft_w
   }
 }
 
-template <class H>
+template <class H, bool SEARCH = false, typename X = float>
 static int launch_corr_fft_half(const CorrArgs& a, cudaStream_t stream) {
   using L = FftLayout<typename H::Fft>;
   const long long total = (long long)a.n_pairs * a.m * a.n;
@@ -626,21 +824,22 @@ static int launch_corr_fft_half(const CorrArgs& a, cudaStream_t stream) {
   int dev = 0;
   cudaGetDevice(&dev);
   if (configured_dev != dev) {
-    cudaError_t e = cudaFuncSetAttribute(k_corr_fft_half<H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::SMEM);
+    cudaError_t e = cudaFuncSetAttribute(k_corr_fft_half<H, SEARCH, X>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::SMEM);
     if (e != cudaSuccess) return set_cuda_error(e, "cudaFuncSetAttribute(k_corr_fft_half)");
     per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_corr_fft_half<H>, H::NT, L::SMEM);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_corr_fft_half<H, SEARCH, X>, H::NT, L::SMEM);
     if (per_sm < 1) per_sm = 1;
     configured_dev = dev;
   }
   const long long room = (long long)sm_count() * per_sm;
   CorrArgs b = a;
   b.tie_tol = kTieTolF32;
-  k_corr_fft_half<H><<<(unsigned)std::min(total, room), H::NT, L::SMEM, stream>>>(b);
+  k_corr_fft_half<H, SEARCH, X><<<(unsigned)std::min(total, room), H::NT, L::SMEM, stream>>>(b);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? PIV_OK : set_cuda_error(e, "k_corr_fft_half launch");
 }
 
+template <bool SEARCH = false, typename X = float>
 static int launch_corr_fft_warp32(const CorrArgs& a, cudaStream_t stream) {
   const long long total = (long long)a.n_pairs * a.m * a.n;
   if (total == 0) return PIV_OK;
@@ -650,24 +849,26 @@ static int launch_corr_fft_warp32(const CorrArgs& a, cudaStream_t stream) {
   const long long room = (long long)sm_count() * kWarpFftCtas;
   CorrArgs b = a;
   b.tie_tol = kTieTolF32;
-  k_corr_fft_warp32<<<(unsigned)std::min(blocks, room), 32 * kWarpFftWarps, smem, stream>>>(b);
+  k_corr_fft_warp32<SEARCH, X><<<(unsigned)std::min(blocks, room), 32 * kWarpFftWarps, smem, stream>>>(b);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? PIV_OK : set_cuda_error(e, "k_corr_fft_warp32 launch");
 }
 
-// Passes that the kernels above take.
-static bool corr_fft_half_supported(const CorrArgs& a) {
-  return a.dtype == PIV_DTYPE_F32 && (a.fft_size == 32 || a.fft_size == 64 || a.fft_size == 128) &&
-         a.fft_size == 2 * a.ss && a.ws == a.ss && !(a.fft_size == 32 && a.s2n);
+// Passes that the kernels above take (float32 passes; the search of float64
+// passes on the same windows).
+static bool corr_fft_half_windows(const CorrArgs& a) {
+  return (a.fft_size == 32 || a.fft_size == 64 || a.fft_size == 128) &&
+         a.fft_size == 2 * a.ss && a.ws == a.ss;
 }
 
 // Threads per CTA: N = 64 six CTAs of 128 per SM (four or five: 72, 70 us); N
 // = 128, whose map takes most of an SM's shared memory, 512 (256 threads 95
 // us, 1024 with 64 registers each 133 us).
+template <bool SEARCH, typename X>
 static int correlate_fft_half(const CorrArgs& a, cudaStream_t stream) {
-  if (a.fft_size == 32) return launch_corr_fft_warp32(a, stream);
-  if (a.fft_size == 64) return launch_corr_fft_half<HalfCfg<64, 128, 6>>(a, stream);
-  return launch_corr_fft_half<HalfCfg<128, 512, 1>>(a, stream);
+  if (a.fft_size == 32) return launch_corr_fft_warp32<SEARCH, X>(a, stream);
+  if (a.fft_size == 64) return launch_corr_fft_half<HalfCfg<64, 128, sizeof(X) == 8 ? 4 : 6>, SEARCH, X>(a, stream);
+  return launch_corr_fft_half<HalfCfg<128, 512, 1>, SEARCH, X>(a, stream);
 }
 
 }  // namespace piv

@@ -26,6 +26,7 @@ static const FftVariant kFft128f[] = {PIV_FFT_VAR(128, float, 8, 16, 1, 1024), P
 static const FftVariant kFft256f[] = {PIV_FFT_VAR(256, float, 16, 16, 1, 1024)};
 
 const FftVariant* fft_variants_f64(int fft_size, int* count);  // piv_correlate_f64.cu
+int correlate_f64(const CorrArgs& a, const FftVariant& t, cudaStream_t stream);
 
 static const FftVariant* fft_variants(int fft_size, int dtype, int* count) {
   *count = 0;
@@ -71,7 +72,9 @@ int correlate_fft(const CorrArgs& a, int variant, cudaStream_t stream) {
   const FftVariant* t = fft_variants(a.fft_size, a.dtype, &n);
   if (!t) return set_error(PIV_E_UNSUPPORTED, "fft_size %d is not supported (8..256)", a.fft_size);
   if (variant < 0 || variant >= n) variant = 0;
-  if (variant == 0 && corr_fft_half_supported(a)) return correlate_fft_half(a, stream);
+  if (a.dtype == PIV_DTYPE_F64) return correlate_f64(a, t[variant], stream);
+  if (variant == 0 && corr_fft_half_windows(a) && !(a.fft_size == 32 && a.s2n))
+    return correlate_fft_half<false, float>(a, stream);
   return t[variant].launch(a, stream);
 }
 

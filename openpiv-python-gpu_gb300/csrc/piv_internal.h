@@ -70,12 +70,20 @@ struct CorrArgs {
   // (window indices pair-major, as the outputs are indexed) are correlated.
   const int* win_list;
   const int* win_count;
+  // Float64 passes: scratch for the indices of the windows that the float32
+  // search leaves open (n_pairs m n ints) and their count.
   // Refined tensor form: scratch for the near-tie windows' indices (n_pairs m
   // n ints) and their count; when set, those windows are correlated again by
   // the float32 FFT engine, which resolves their integer peaks (NULL: they
   // keep the fp16 maps' peaks and are counted as near ties).
   int* tie_list;
   int* tie_list_count;
+  // Float64 passes: records of the windows that the search leaves with up to
+  // kCandMax candidates (window, their number, their flat map positions),
+  // room for cand_cap of them, and their number.
+  int* cand;
+  int* cand_count;
+  int cand_cap;
   // Refined tensor form: the fp16 engine writes each window's mean of frame a
   // and of frame b here ([n_pairs m n][2]), and the refinement reads them.
   float* win_means;
@@ -87,6 +95,22 @@ struct CorrArgs {
   long long seg_windows;
   CorrSeg segs[kMaxCorrSegs];
 };
+
+constexpr int kCandMax = 8, kCandInts = 2 + kCandMax;
+// Ints of a float64 pass's lists over `windows` windows (set_f64_lists): two
+// counts, the window list, and records for up to a quarter of the windows.
+inline int f64_cand_cap(size_t windows) {
+  const size_t c = windows / 4 + 64;
+  return (int)(c < (size_t)1 << 20 ? c : (size_t)1 << 20);
+}
+inline size_t f64_list_ints(size_t windows) { return 2 + windows + (size_t)f64_cand_cap(windows) * kCandInts; }
+inline void set_f64_lists(CorrArgs& a, int* base, size_t windows) {
+  a.tie_list_count = base;
+  a.cand_count = base + 1;
+  a.tie_list = base + 2;
+  a.cand = base + 2 + windows;
+  a.cand_cap = f64_cand_cap(windows);
+}
 
 // Relative tie tolerances of the engines (map error relative to the map
 // maximum, with margin): float32 FFT and hi/lo split tensor products ~1e-6,
