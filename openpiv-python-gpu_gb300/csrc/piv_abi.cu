@@ -59,6 +59,54 @@ int sm_count() {
   return counts[dev];
 }
 
+// Scratch of the stage entry points, stream-ordered from a pool of this
+// library's own per device. The device's default pool gives its memory back at
+// every synchronisation, so each call after one mapped its scratch anew (250
+// us of a 360 us correlation). This pool keeps up to kPoolKeep bytes; it is
+// trimmed when a plan is destroyed and when a plan's allocation fails.
+// Allocations made while `s` is captured become the graph's own, as before.
+static constexpr unsigned long long kPoolKeep = 64ull << 20;
+static std::mutex g_pool_mu;
+static cudaMemPool_t g_pools[64] = {nullptr};
+
+static cudaMemPool_t scratch_pool() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  if (!g_pools[dev]) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t pool = nullptr;
+    unsigned long long keep = kPoolKeep;
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    g_pools[dev] = pool;
+  }
+  return g_pools[dev];
+}
+
+static void scratch_pool_trim() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  if (g_pools[dev] && cudaMemPoolTrimTo(g_pools[dev], 0) != cudaSuccess) cudaGetLastError();
+}
+
+static cudaError_t scratch_alloc(void** ptr, size_t bytes, cudaStream_t s) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
+    cudaMemPool_t pool = scratch_pool();
+    if (pool && cudaMallocFromPoolAsync(ptr, bytes, pool, s) == cudaSuccess) return cudaSuccess;
+  }
+  cudaGetLastError();
+  return cudaMallocAsync(ptr, bytes, s);
+}
+
 static size_t pixel_bytes(int pixel_type) {
   switch (pixel_type) {
     case PIV_PIXEL_U8: return 1;
@@ -201,6 +249,11 @@ static int plan_alloc(piv_plan* p, void** ptr, size_t bytes) {
   *ptr = nullptr;
   if (bytes == 0) return PIV_OK;
   cudaError_t e = cudaMalloc(ptr, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    scratch_pool_trim();
+    e = cudaMalloc(ptr, bytes);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     return set_error(PIV_E_OOM, "cudaMalloc(%zu bytes) failed: %s", bytes, cudaGetErrorString(e));
@@ -309,6 +362,7 @@ void piv_plan_destroy(piv_plan* p) {
   for (auto e : p->event_pool) cudaEventDestroy(e);
   for (void* a : p->allocs) cudaFree(a);
   delete p;
+  scratch_pool_trim();
 }
 
 int piv_plan_set_timing(piv_plan* p, int enable) {
@@ -870,13 +924,13 @@ int piv_correlate(const piv_geometry* g, int n_pairs, const void* frames_a, cons
   cudaStream_t s = (cudaStream_t)stream;
   const size_t need = correlate_fft_scratch_bytes(fft_size, dtype);
   if (correlate_tensor_supported(c, dft_mode)) {
-    PIV_TRY(cuda_ok(cudaMallocAsync((void**)&c.status, sizeof(int), s), "cudaMallocAsync"));
+    PIV_TRY(cuda_ok(scratch_alloc((void**)&c.status, sizeof(int), s), "scratch allocation"));
     cudaMemsetAsync(c.status, 0, sizeof(int), s);
     int* peaks = nullptr;  // the refined form reads the peaks back: device peaks when the caller wants none
     const size_t cnt = (size_t)n_pairs * g->m * g->n;
     if ((dft_mode == PIV_DFT_TENSOR_REFINED || (dft_mode == PIV_DFT_TENSOR_SPLIT && c.ss == 64)) &&
         (!c.peak_i || !c.peak_j)) {
-      PIV_TRY(cuda_ok(cudaMallocAsync((void**)&peaks, 2 * cnt * sizeof(int), s), "cudaMallocAsync"));
+      PIV_TRY(cuda_ok(scratch_alloc((void**)&peaks, 2 * cnt * sizeof(int), s), "scratch allocation"));
       if (!c.peak_i) c.peak_i = peaks;
       if (!c.peak_j) c.peak_j = peaks + cnt;
     }
@@ -896,7 +950,7 @@ int piv_correlate(const piv_geometry* g, int n_pairs, const void* frames_a, cons
   void* scratch = nullptr;
   if (need || ints) {
     const size_t head = (need + 255) / 256 * 256;
-    PIV_TRY(cuda_ok(cudaMallocAsync(&scratch, head + ints * sizeof(int), s), "cudaMallocAsync"));
+    PIV_TRY(cuda_ok(scratch_alloc(&scratch, head + ints * sizeof(int), s), "scratch allocation"));
     if (need) {
       c.scratch = scratch;
       c.scratch_bytes = need;
@@ -924,7 +978,7 @@ int piv_correlate_maps(const piv_geometry* g, int n_pairs, const void* frames_a,
   const size_t cnt = (size_t)n_pairs * g->m * g->n;
   const size_t tsz = dtype == PIV_DTYPE_F64 ? 8 : 4;
   void* u = nullptr;
-  PIV_TRY(cuda_ok(cudaMallocAsync(&u, 2 * cnt * tsz, s), "cudaMallocAsync"));
+  PIV_TRY(cuda_ok(scratch_alloc(&u, 2 * cnt * tsz, s), "scratch allocation"));
   CorrArgs c{};
   c.frame_a = frames_a;
   c.frame_b = frames_b;
@@ -949,7 +1003,7 @@ int piv_correlate_maps(const piv_geometry* g, int n_pairs, const void* frames_a,
   c.maps = maps;
   int rc;
   if (correlate_tensor_supported(c, dft_mode)) {
-    PIV_TRY(cuda_ok(cudaMallocAsync((void**)&c.status, sizeof(int), s), "cudaMallocAsync"));
+    PIV_TRY(cuda_ok(scratch_alloc((void**)&c.status, sizeof(int), s), "scratch allocation"));
     cudaMemsetAsync(c.status, 0, sizeof(int), s);
     rc = correlate_tensor(c, dft_mode, 0, s);
     cudaFreeAsync(c.status, s);
@@ -958,7 +1012,7 @@ int piv_correlate_maps(const piv_geometry* g, int n_pairs, const void* frames_a,
   }
   const size_t need = correlate_fft_scratch_bytes(fft_size, dtype);
   if (need) {
-    PIV_TRY(cuda_ok(cudaMallocAsync(&c.scratch, need, s), "cudaMallocAsync"));
+    PIV_TRY(cuda_ok(scratch_alloc(&c.scratch, need, s), "scratch allocation"));
     c.scratch_bytes = need;
   }
   rc = correlate_fft(c, 0, s);
@@ -1011,7 +1065,7 @@ int piv_validate(int m, int n, int n_pairs, const double* u, const double* v, co
             field_mask, exclude, fp32};
   cudaStream_t s = (cudaStream_t)stream;
   double* stats = nullptr;
-  if (!isnan(rms_tol)) PIV_TRY(cuda_ok(cudaMallocAsync((void**)&stats, 4 * 8 * (size_t)n_pairs, s), "cudaMallocAsync"));
+  if (!isnan(rms_tol)) PIV_TRY(cuda_ok(scratch_alloc((void**)&stats, 4 * 8 * (size_t)n_pairs, s), "scratch allocation"));
   int rc = validate(a, val, stats, s);
   if (stats) cudaFreeAsync(stats, s);
   return rc;
@@ -1036,7 +1090,7 @@ int piv_replace(int m, int n, int n_pairs, double* u, double* v, uint8_t* val, c
   a.dtype = dtype;
   a.status = nullptr;
   const size_t need = replace_scratch_bytes(m, n, n_pairs);
-  PIV_TRY(cuda_ok(cudaMallocAsync(&a.scratch, need, s), "cudaMallocAsync"));
+  PIV_TRY(cuda_ok(scratch_alloc(&a.scratch, need, s), "scratch allocation"));
   int rc = replace(a, s);
   cudaFreeAsync(a.scratch, s);
   return rc;
@@ -1052,7 +1106,7 @@ int piv_smoothn_flags(int m, int n, int n_pairs, double* u, double* v, const uin
   if (!u || !v) return set_error(PIV_E_ARG, "NULL argument");
   cudaStream_t s = (cudaStream_t)stream;
   void* scratch = nullptr;
-  PIV_TRY(cuda_ok(cudaMallocAsync(&scratch, smoothn_scratch_bytes(m, n, n_pairs), s), "cudaMallocAsync"));
+  PIV_TRY(cuda_ok(scratch_alloc(&scratch, smoothn_scratch_bytes(m, n, n_pairs), s), "scratch allocation"));
   int rc = smoothn(m, n, n_pairs, u, v, u, v, field_mask, sp, p_out, scratch, s, flags_out);
   cudaFreeAsync(scratch, s);
   return rc;
@@ -1100,7 +1154,7 @@ int piv_plan_autotune(piv_plan* p, int n_pairs, const void* frames_a, const void
   // passes) are those of these frames.
   const size_t cnt = p->st.back().mn * (size_t)n_pairs;
   double* uv = nullptr;
-  PIV_TRY(cuda_ok(cudaMallocAsync((void**)&uv, 2 * cnt * sizeof(double), s), "cudaMallocAsync"));
+  PIV_TRY(cuda_ok(scratch_alloc((void**)&uv, 2 * cnt * sizeof(double), s), "scratch allocation"));
   int rc = piv_plan_run(p, n_pairs, frames_a, frames_b, frames_on_host, uv, uv + cnt, nullptr, nullptr, 0, stream_ptr);
   cudaFreeAsync(uv, s);
   if (rc != PIV_OK) return rc;
@@ -1210,7 +1264,7 @@ int piv_selftest_bounded_wait(unsigned int max_polls, int* status, void* stream_
   if (!status) return set_error(PIV_E_ARG, "NULL argument");
   cudaStream_t s = (cudaStream_t)stream_ptr;
   int* dev = nullptr;
-  PIV_TRY(cuda_ok(cudaMallocAsync((void**)&dev, sizeof(int), s), "cudaMallocAsync"));
+  PIV_TRY(cuda_ok(scratch_alloc((void**)&dev, sizeof(int), s), "scratch allocation"));
   cudaMemsetAsync(dev, 0, sizeof(int), s);
   int rc = bounded_wait_probe(max_polls, dev, s);
   if (rc == PIV_OK) rc = cuda_ok(cudaMemcpyAsync(status, dev, sizeof(int), cudaMemcpyDeviceToHost, s), "status copy");
