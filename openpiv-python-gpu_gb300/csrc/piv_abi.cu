@@ -765,8 +765,7 @@ static int run_post(piv_plan* p, int k, RunCtx& x, cudaStream_t s) {
   va.field_mask = st.field_mask;
   va.exclude = nullptr;
   va.fp32 = st.fp32;
-  PIV_TRY(validate(va, st.val0, p->rms_stats, s));
-  PIV_TRY(cuda_ok(cudaMemcpyAsync(st.val, st.val0, cnt, cudaMemcpyDeviceToDevice, s), "val copy"));
+  PIV_TRY(validate(va, st.val0, p->rms_stats, s, st.val));
   mark(p, x, k * PIV_STAGES + 3, s);
   RepArgs ra;
   ra.val = va;
@@ -795,6 +794,19 @@ static int run_post(piv_plan* p, int k, RunCtx& x, cudaStream_t s) {
   return PIV_OK;
 }
 
+// Device results of a run in one launch (four copies on the stream took 4 us
+// each, whatever their size).
+__global__ void k_results(int count, const double* __restrict__ u, const double* __restrict__ v,
+                          const uint8_t* __restrict__ val, const uint8_t* __restrict__ out, double* uo, double* vo,
+                          uint8_t* valo, uint8_t* outo) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= count) return;
+  uo[t] = u[t];
+  vo[t] = v[t];
+  if (valo) valo[t] = val[t];
+  if (outo) outo[t] = out[t];
+}
+
 static int run_end(piv_plan* p, RunCtx& x, double* u, double* v, uint8_t* val_locations, uint8_t* outliers,
                    int outputs_on_host, cudaStream_t s) {
   const piv_config& cfg = p->cfg;
@@ -807,11 +819,17 @@ static int run_end(piv_plan* p, RunCtx& x, double* u, double* v, uint8_t* val_lo
     ru = p->u_final;
     rv = p->v_final;
   }
-  const cudaMemcpyKind ok = outputs_on_host ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
-  PIV_TRY(cuda_ok(cudaMemcpyAsync(u, ru, cnt * 8, ok, s), "result copy"));
-  PIV_TRY(cuda_ok(cudaMemcpyAsync(v, rv, cnt * 8, ok, s), "result copy"));
-  if (val_locations) PIV_TRY(cuda_ok(cudaMemcpyAsync(val_locations, last.val0, cnt, ok, s), "result copy"));
-  if (outliers) PIV_TRY(cuda_ok(cudaMemcpyAsync(outliers, p->outliers, cnt, ok, s), "result copy"));
+  if (!outputs_on_host && (((uintptr_t)u | (uintptr_t)v) & 7) == 0) {
+    k_results<<<(unsigned)((cnt + 255) / 256), 256, 0, s>>>(cnt, ru, rv, last.val0, p->outliers, u, v, val_locations,
+                                                           outliers);
+    PIV_TRY(cuda_ok(cudaGetLastError(), "k_results"));
+  } else {
+    const cudaMemcpyKind ok = outputs_on_host ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
+    PIV_TRY(cuda_ok(cudaMemcpyAsync(u, ru, cnt * 8, ok, s), "result copy"));
+    PIV_TRY(cuda_ok(cudaMemcpyAsync(v, rv, cnt * 8, ok, s), "result copy"));
+    if (val_locations) PIV_TRY(cuda_ok(cudaMemcpyAsync(val_locations, last.val0, cnt, ok, s), "result copy"));
+    if (outliers) PIV_TRY(cuda_ok(cudaMemcpyAsync(outliers, p->outliers, cnt, ok, s), "result copy"));
+  }
   mark(p, x, (int)p->st.size() * PIV_STAGES + 1, s);
   return PIV_OK;
 }

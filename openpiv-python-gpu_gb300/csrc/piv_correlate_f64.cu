@@ -245,14 +245,14 @@ static int launch_fit64(const CorrArgs& a, cudaStream_t stream) {
 // a list buffer and peak arrays and reads neither maps nor S2N.
 static bool correlate_f64_searched(const CorrArgs& a) {
   return a.dtype == PIV_DTYPE_F64 && corr_fft_half_windows(a) && !a.maps && !a.s2n && !a.win_list && a.tie_list &&
-         a.tie_list_count && a.peak_i && a.peak_j && a.cand && a.cand_count && a.cand_cap > 0;
+         a.tie_list_count && a.peak_i && a.peak_j && a.cand && a.cand_count == a.tie_list_count + 1 &&
+         a.cand_cap > 0;
 }
 
 int correlate_f64(const CorrArgs& a, const FftVariant& t, cudaStream_t stream) {
   const long long total = (long long)a.n_pairs * a.m * a.n;
   if (!correlate_f64_searched(a) || total == 0 || total > 2147483647LL) return t.launch(a, stream);
-  cudaError_t e = cudaMemsetAsync(a.tie_list_count, 0, sizeof(int), stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(a.cand_count, 0, sizeof(int), stream);
+  cudaError_t e = cudaMemsetAsync(a.tie_list_count, 0, 2 * sizeof(int), stream);  // and cand_count (set_f64_lists)
   if (e != cudaSuccess) return set_cuda_error(e, "window list counts");
   const bool whole = a.pixel_type == PIV_PIXEL_U8 || a.pixel_type == PIV_PIXEL_U16;
   int rc = whole ? correlate_fft_half<true, float>(a, stream) : correlate_fft_half<true, double>(a, stream);

@@ -190,7 +190,8 @@ struct ValArgs {
   const uint8_t* exclude;     // [pairs][m][n] or NULL
   int fp32;
 };
-int validate(const ValArgs& a, uint8_t* val, double* rms_stats, cudaStream_t stream);
+// val2 (may be NULL) receives a second copy of the mask.
+int validate(const ValArgs& a, uint8_t* val, double* rms_stats, cudaStream_t stream, uint8_t* val2 = nullptr);
 
 struct RepArgs {
   ValArgs val;                // revalidation settings (u/v/exclude ignored)

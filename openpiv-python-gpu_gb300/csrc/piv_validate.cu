@@ -265,8 +265,10 @@ __global__ void k_field_stats(int m, int n, const double* __restrict__ u, const 
   }
 }
 
+// val2 (may be NULL) receives a copy of val.
 template <typename T>
-__global__ void k_validate(ValArgs a, uint8_t* __restrict__ val, const double* __restrict__ rms) {
+__global__ void k_validate(ValArgs a, uint8_t* __restrict__ val, uint8_t* __restrict__ val2,
+                           const double* __restrict__ rms) {
   const long long npts = (long long)a.m * a.n;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= npts * a.n_pairs) return;
@@ -274,15 +276,18 @@ __global__ void k_validate(ValArgs a, uint8_t* __restrict__ val, const double* _
   const int p = (int)(t % npts);
   if ((a.field_mask && a.field_mask[p]) || (a.exclude && a.exclude[t])) {
     val[t] = 0;
+    if (val2) val2[t] = 0;
     return;
   }
   const long long off = (long long)pair * npts;
   FieldView fu{a.u + off, a.m, a.n, nullptr, 0.0}, fv{a.v + off, a.m, a.n, nullptr, 0.0};
   ValSettings s{a.size, a.s2n_tol, a.median_tol, a.mad_tol, a.mean_tol, a.rms_tol, a.fp32, a.s2n, a.s2n_dtype};
-  val[t] = point_invalid<T>(s, fu, fv, t, p / a.n, p % a.n, rms ? rms + pair * 4 : nullptr) ? 1 : 0;
+  const uint8_t bad = point_invalid<T>(s, fu, fv, t, p / a.n, p % a.n, rms ? rms + pair * 4 : nullptr) ? 1 : 0;
+  val[t] = bad;
+  if (val2) val2[t] = bad;
 }
 
-int validate(const ValArgs& a, uint8_t* val, double* rms_stats, cudaStream_t stream) {
+int validate(const ValArgs& a, uint8_t* val, double* rms_stats, cudaStream_t stream, uint8_t* val2) {
   if (a.size > 3 || a.size < 1) return set_error(PIV_E_UNSUPPORTED, "validation_size %d (supported: 1..3)", a.size);
   const long long total = (long long)a.m * a.n * a.n_pairs;
   if (total == 0) return PIV_OK;
@@ -295,8 +300,8 @@ int validate(const ValArgs& a, uint8_t* val, double* rms_stats, cudaStream_t str
   }
   const int bs = 128;
   const unsigned grid = (unsigned)((total + bs - 1) / bs);
-  if (a.fp32) k_validate<float><<<grid, bs, 0, stream>>>(a, val, rms);
-  else k_validate<double><<<grid, bs, 0, stream>>>(a, val, rms);
+  if (a.fp32) k_validate<float><<<grid, bs, 0, stream>>>(a, val, val2, rms);
+  else k_validate<double><<<grid, bs, 0, stream>>>(a, val, val2, rms);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? PIV_OK : set_cuda_error(e, "k_validate launch");
 }

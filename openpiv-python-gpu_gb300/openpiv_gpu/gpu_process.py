@@ -249,8 +249,8 @@ class piv_gpu:
             all(np.issubdtype(frame.dtype, np.number) for frame in frames) and \
             all(not np.iscomplex(frame).any() for frame in frames), \
             "Both frames must be an ndarray of {} values with shape {}.".format("real", self.frame_shape)
-        u, v = self.gpu_process(frame_a, frame_b)
-        return u.cpu().numpy(), v.cpu().numpy()
+        uv = self.gpu_process._pair(frame_a, frame_b).cpu().numpy()  # both fields in one copy
+        return uv[0, 0], uv[1, 0]
 
     @property
     def field_shape(self):
@@ -509,7 +509,35 @@ class PIVGPU:
         results are copied into pinned host memory before the call returns and
         come back as NumPy arrays.
         """
+        if not host_out:
+            uv = self._run_device(frames_a, frames_b)
+            return uv[0], uv[1]
         torch = _torch()
+        plan, B, fa, fb, pa, pb, host_a = self._batch(frames_a, frames_b)
+        m, n = self.piv_fields[-1].field_shape
+        key = (B, m, n)
+        if getattr(self, "_host_out", (None,))[0] != key:
+            self._host_out = (key,) + tuple(torch.empty((B, m, n), dtype=dt, pin_memory=True)
+                                            for dt in (torch.float64, torch.float64, torch.uint8, torch.uint8))
+        u, v, val, out = self._host_out[1:]
+        stream = torch.cuda.current_stream().cuda_stream
+        self._maybe_tune(plan, B, pa, pb, host_a, stream)
+        _lib.check(_lib.lib().piv_plan_run(plan, B, pa, pb, host_a, u.data_ptr(), v.data_ptr(), val.data_ptr(),
+                                           out.data_ptr(), 1, stream))
+        self._last = (plan, B, fa, fb)
+        self.init_val_locations = val.bool()
+        self.val_locations = out.bool()
+        self._log_smoothing(plan, B)
+        u, v = u.numpy(), v.numpy()
+        self.init_val_locations = self.init_val_locations.numpy()
+        self.val_locations = self.val_locations.numpy()
+        if self.max_iters == 1 and self.dtype_f == np.float32:
+            u, v = u.astype(np.float32), v.astype(np.float32)
+        return u, v
+
+    def _batch(self, frames_a, frames_b):
+        """The plan of a batch and its frames: (plan, pairs, frames a, frames b,
+        their addresses, whether they are on the host)."""
         fa, pt_a, host_a = self._frames(frames_a)
         fb, pt_b, host_b = self._frames(frames_b)
         if pt_a != pt_b or host_a != host_b:
@@ -519,39 +547,28 @@ class PIVGPU:
         B = fa.shape[0]
         assert tuple(fa.shape[1:]) == self.frame_shape and tuple(fb.shape) == tuple(fa.shape)
         plan = self._plan(pt_a, B)
-        m, n = self.piv_fields[-1].field_shape
-        if host_out:
-            key = (B, m, n)
-            if getattr(self, "_host_out", (None,))[0] != key:
-                self._host_out = (key,) + tuple(torch.empty((B, m, n), dtype=dt, pin_memory=True)
-                                                for dt in (torch.float64, torch.float64, torch.uint8, torch.uint8))
-            u, v, val, out = self._host_out[1:]
-        else:
-            dev = torch.device("cuda", torch.cuda.current_device())
-            u = torch.empty((B, m, n), dtype=torch.float64, device=dev)
-            v = torch.empty_like(u)
-            val = torch.empty((B, m, n), dtype=torch.uint8, device=dev)
-            out = torch.empty_like(val)
         pa = fa.ctypes.data if host_a else fa.data_ptr()
         pb = fb.ctypes.data if host_b else fb.data_ptr()
+        return plan, B, fa, fb, pa, pb, host_a
+
+    def _run_device(self, frames_a, frames_b):
+        """One plan run with device results: the fields as one tensor [2, B, m, n]."""
+        torch = _torch()
+        plan, B, fa, fb, pa, pb, host_a = self._batch(frames_a, frames_b)
+        m, n = self.piv_fields[-1].field_shape
+        dev = torch.device("cuda", torch.cuda.current_device())
+        uv = torch.empty((2, B, m, n), dtype=torch.float64, device=dev)
+        masks = torch.empty((2, B, m, n), dtype=torch.uint8, device=dev)
+        step = B * m * n
         stream = torch.cuda.current_stream().cuda_stream
         self._maybe_tune(plan, B, pa, pb, host_a, stream)
-        _lib.check(_lib.lib().piv_plan_run(plan, B, pa, pb, host_a, u.data_ptr(), v.data_ptr(), val.data_ptr(),
-                                           out.data_ptr(), int(bool(host_out)), stream))
+        _lib.check(_lib.lib().piv_plan_run(plan, B, pa, pb, host_a, uv.data_ptr(), uv.data_ptr() + 8 * step,
+                                           masks.data_ptr(), masks.data_ptr() + step, 0, stream))
         self._last = (plan, B, fa, fb)
-        self.init_val_locations = val.bool()
-        self.val_locations = out.bool()
+        masks = masks.view(torch.bool)  # zeros and ones
+        self.init_val_locations, self.val_locations = masks[0], masks[1]
         self._log_smoothing(plan, B)
-        if host_out:
-            u, v = u.numpy(), v.numpy()
-            self.init_val_locations = self.init_val_locations.numpy()
-            self.val_locations = self.val_locations.numpy()
-            if self.max_iters == 1 and self.dtype_f == np.float32:
-                u, v = u.astype(np.float32), v.astype(np.float32)
-            return u, v
-        if self.max_iters == 1 and self.dtype_f == np.float32:
-            u, v = u.float(), v.float()
-        return u, v
+        return uv.float() if self.max_iters == 1 and self.dtype_f == np.float32 else uv
 
     def run_batches(self, batches):
         """Pipelined run over an iterable of (frames_a, frames_b) batches of
@@ -696,14 +713,19 @@ class PIVGPU:
 
         Returns (u, v) as torch CUDA tensors.
         """
+        uv = self._pair(frame_a, frame_b)
+        return uv[0, 0], uv[1, 0]
+
+    def _pair(self, frame_a, frame_b):
+        """The fields of one pair as one tensor [2, 1, m, n]."""
         if isinstance(frame_a, np.ndarray):
             fa, fb = frame_a[None], frame_b[None]
         else:
             fa, fb = frame_a.unsqueeze(0), frame_b.unsqueeze(0)
-        u, v = self.run_batch(fa, fb)
+        uv = self._run_device(fa, fb)
         self.init_val_locations = self.init_val_locations[0]
         self.val_locations = self.val_locations[0]
-        return u[0], v[0]
+        return uv
 
     def iteration_outputs(self, pair=0):
         """Per-iteration intermediates of the last run, as host NumPy arrays."""
