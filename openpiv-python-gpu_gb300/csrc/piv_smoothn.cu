@@ -287,8 +287,17 @@ PIV_D double warp_sums(const T (&x)[K]) {
   return v[0];
 }
 
-// warp_sums of four values: two levels that halve the values, then the tree;
-// the sum of x[k] is in the lanes whose bits 4 and 3 are k's bits 1 and 0.
+// warp_sums of two values: one level that halves them, then the tree; the sum
+// of x0 is in lanes 0 .. 15, that of x1 in lanes 16 .. 31.
+PIV_D double warp_sums2(double x0, double x1) {
+  const bool up = threadIdx.x & 16;
+  double v = (up ? x1 : x0) + __shfl_xor_sync(~0u, up ? x0 : x1, 16);
+  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(~0u, v, o);
+  return v;
+}
+
+// warp_sums of four values: the sum of x[k] is in the lanes whose bits 4 and 3
+// are k's bits 1 and 0.
 PIV_D double warp_sums4(double x0, double x1, double x2, double x3) {
   const int lane = threadIdx.x & 31;
   const bool u16 = lane & 16, u8 = lane & 8;
@@ -297,6 +306,16 @@ PIV_D double warp_sums4(double x0, double x1, double x2, double x3) {
   double v = (u8 ? b : a) + __shfl_xor_sync(~0u, u8 ? a : b, 8);
   for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(~0u, v, o);
   return v;
+}
+
+// x / c for a constant c with rc = 1 / c rounded: the correctly rounded
+// quotient (Markstein 1990: the product's remainder is exact in one FMA, and
+// one correction rounds as the division), a third of the division's chain of
+// float64 instructions. Outside the range where that holds, the division.
+PIV_D double div_const(double x, double c, double rc) {
+  if (!(fabs(x) > 1e-280 && fabs(x) < 1e300)) return x / c;
+  const double q = x * rc;
+  return fma(fma(-q, c, x), rc, q);
 }
 
 // Fields of a DCT pass: component c of pair k at (c ? v : u) + k * stride.
@@ -648,12 +667,16 @@ PIV_D int smooth_flags(bool is_auto, double p, double pmin, double pmax, bool la
 // cancellation, each term within a few float32 ulps, the score within ~1e-9)
 // only ranks the scan points, all ten in one pass over the field; the
 // L-BFGS-B evaluations, whose difference quotients divide score differences
-// by 1e-8, use the float64 score, the point and its neighbour together.
+// by 1e-8, use the float64 score, the point and its neighbour together. SETS
+// = 2 (clusters of eight, whose CTAs hold two virtual warps): a second set of
+// the virtual threads sums the scores of the odd points, so that all four
+// float64 units of an SM work.
 // Bound by the float64 pipe and by the latency of the search's steps. One
 // score at a time on one CTA, with the scan in ten passes, took 396 us for
 // the 31 x 31 and 63 x 63 fields of one 1024 x 1024 pair; this takes 157 us.
+template <int SETS>
 __global__ void __launch_bounds__(kVT)
-k_gcv(int m, int n, int c, const double* __restrict__ fd, double* __restrict__ f2, float* __restrict__ f2f,
+k_gcv(int m, int n, int c, double rmn, const double* __restrict__ fd, double* __restrict__ f2, float* __restrict__ f2f,
       const double* __restrict__ lam2, const float* __restrict__ lam2f, double pmin, double pmax,
       double* __restrict__ p_out, double* __restrict__ s_out, int* __restrict__ flags) {
   __shared__ double part[2][kVW][20];  // by parity of the evaluation: the virtual warps' partial sums
@@ -662,53 +685,57 @@ k_gcv(int m, int n, int c, const double* __restrict__ fd, double* __restrict__ f
   const int pair = blockIdx.x / c;
   const int rank = c > 1 ? (int)cluster_rank() : 0;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int vt = rank * blockDim.x + threadIdx.x, vw = vt >> 5;
+  const int vtn = kVT / c, set = SETS == 2 && (int)threadIdx.x >= vtn;
+  const int vt = rank * vtn + (threadIdx.x - set * vtn), vw = vt >> 5;
   const bool w0 = warp == 0;
   const long long mn = (long long)m * n;
   const double* fu = fd + 2 * pair * mn;
   double* f2p = f2 + pair * mn;
   float* f2fp = f2f + pair * mn;
   const double n_finite = (double)mn;
-  // fd_u^2 + fd_v^2; each virtual thread reads only what it wrote.
-  for (long long e = vt; e < mn; e += kVT) {
+  // fd_u^2 + fd_v^2, by the first set.
+  for (long long e = vt; !set && e < mn; e += kVT) {
     const double a = fu[e], b = fu[mn + e];
     const double q = a * a + b * b;
     f2p[e] = q;
     f2fp[e] = (float)q;
   }
   int par = 0;
-  auto publish = [&](int count, int slot, bool holds, double v) {
-    if (holds && slot < count)
-      for (int r = 0; r < c; ++r) {
-        if (c == 1) part[par][vw][slot] = v;
-        else st_cluster(&part[par][vw][slot], (unsigned)r, v);
-      }
-    cluster_barrier(c);
+  // Leaves v as the virtual warp's partial sum `slot` in CTA r of the cluster.
+  auto put = [&](int slot, double v, int r) {
+    if (c == 1) part[par][vw][slot] = v;
+    else st_cluster(&part[par][vw][slot], (unsigned)r, v);
   };
   // 10-point scan (gpu_smoothn.py:182-188), ranked with the fast score; when
   // other points score within 1e-6 of the best, those points are scored
   // again in float64 and the first minimum among them is kept (np.argmin).
-  auto scan_point = [&](int k) { return ((double)k * (1.0 / 9.0)) * (pmax - pmin) + pmin; };
+  auto scan_point = [&](int k) { return fma((double)k * (1.0 / 9.0), pmax - pmin, pmin); };
   if (threadIdx.x < 10) sh_s[threadIdx.x] = pow(10.0, scan_point(threadIdx.x));
   __syncthreads();
   {
-    float acc[20], s[10];
+    // Points SETS k + set: sums of the residuals in acc[k], of 1 - gamma in
+    // acc[PER + k].
+    constexpr int PER = 10 / SETS;
+    float acc[2 * PER], s[PER];
 #pragma unroll
-    for (int k = 0; k < 10; ++k) {
-      s[k] = (float)sh_s[k];
-      acc[k] = acc[10 + k] = 0.f;
+    for (int k = 0; k < PER; ++k) {
+      s[k] = (float)sh_s[SETS * k + set];
+      acc[k] = acc[PER + k] = 0.f;
     }
     for (long long e = vt; e < mn; e += kVT) {
       const float l = lam2f[e], f = f2fp[e];
 #pragma unroll
-      for (int k = 0; k < 10; ++k) {
+      for (int k = 0; k < PER; ++k) {
         const float sl = s[k] * l;
         const float d = sl * __frcp_rn(1.0f + sl);  // 1 - gamma
         acc[k] = fmaf(f * d, d, acc[k]);
-        acc[10 + k] += d;
+        acc[PER + k] += d;
       }
     }
-    publish(20, lane, true, warp_sums(acc));
+    const double v = warp_sums(acc);
+    if (lane < 2 * PER)
+      for (int r = 0; r < c; ++r) put((lane < PER ? 0 : 10) + SETS * (lane % PER) + set, v, r);
+    cluster_barrier(c);
   }
   double p0 = pmin;
   unsigned rescore = 0;  // scan points within 1e-6 of the best fast score, when there are several
@@ -719,8 +746,8 @@ k_gcv(int m, int n, int c, const double* __restrict__ fd, double* __restrict__ f
       trss += part[par][k][q];
       ttr += part[par][k][10 + q];
     }
-    const double w = ttr / (double)mn;
-    const double f = trss / n_finite / (w * w) / 2;
+    const double w = div_const(ttr, n_finite, rmn);
+    const double f = div_const(trss, n_finite, rmn) / (w * w) / 2;
     double best_f = INFINITY;
     double fast[10];
 #pragma unroll
@@ -748,24 +775,41 @@ k_gcv(int m, int n, int c, const double* __restrict__ fd, double* __restrict__ f
   };
   // Float64 scores at the two announced points (valid in warp 0).
   auto score2 = [&](double& fa, double& fb) {
-    const double sa = sh_s[0], sb = sh_s[1];
-    double ra = 0.0, ta = 0.0, rb = 0.0, tb = 0.0;
-    for (long long e = vt; e < mn; e += kVT) {
-      const double l = lam2[e], f = f2p[e];
-      const double ga = rcp_fast(1.0 + sa * l), gb = rcp_fast(1.0 + sb * l);
-      const double da = ga - 1.0, db = gb - 1.0;
-      ra += f * da * da;
-      ta += ga;
-      rb += f * db * db;
-      tb += gb;
+    if constexpr (SETS == 2) {
+      const double s = sh_s[set];
+      double rss = 0.0, tr = 0.0;
+      for (long long e = vt; e < mn; e += kVT) {
+        const double gm = rcp_fast(1.0 + s * lam2[e]);
+        const double d = gm - 1.0;
+        rss += f2p[e] * d * d;
+        tr += gm;
+      }
+      // Lane l holds sum l / 16, for CTA l % 16.
+      const double v = warp_sums2(rss, tr);
+      if ((lane & 15) < c) put(2 * set + (lane >> 4), v, lane & 15);
+    } else {
+      const double sa = sh_s[0], sb = sh_s[1];
+      double ra = 0.0, ta = 0.0, rb = 0.0, tb = 0.0;
+      for (long long e = vt; e < mn; e += kVT) {
+        const double l = lam2[e], f = f2p[e];
+        const double ga = rcp_fast(1.0 + sa * l), gb = rcp_fast(1.0 + sb * l);
+        const double da = ga - 1.0, db = gb - 1.0;
+        ra += f * da * da;
+        ta += ga;
+        rb += f * db * db;
+        tb += gb;
+      }
+      // Lane l holds sum l / 8, for CTA l % 8.
+      const double v = warp_sums4(ra, ta, rb, tb);
+      if ((lane & 7) < c) put(lane >> 3, v, lane & 7);
     }
-    publish(4, lane >> 3, (lane & 7) == 0, warp_sums4(ra, ta, rb, tb));
+    cluster_barrier(c);
     if (w0) {
       double t = 0.0;
       for (int k = 0; k < kVW; ++k) t += part[par][k][lane & 3];
       const double trss = __shfl_sync(~0u, t, (lane & 1) * 2), ttr = __shfl_sync(~0u, t, (lane & 1) * 2 + 1);
-      const double q = 1.0 - ttr / (double)mn;
-      const double f = trss / n_finite / (q * q) / 2;
+      const double q = 1.0 - div_const(ttr, n_finite, rmn);
+      const double f = div_const(trss, n_finite, rmn) / (q * q) / 2;
       fa = __shfl_sync(~0u, f, 0);
       fb = __shfl_sync(~0u, f, 1);
     }
@@ -851,17 +895,19 @@ static void gcv_bounds(int m, int n, double* pmin, double* pmax) {
 // global memory (L2) with one cluster barrier in between; the forward column
 // pass leaves the rows that the inverse row pass of the same CTA starts from.
 // The sums run over virtual threads as in k_gcv, so the result does not
-// depend on c. Bound by the DCTs' dot products and the barriers between
-// passes: one pair of 63 x 63 around a masked disc takes 0.90 ms with 8 CTAs.
+// depend on c. Sums of two products have their roundings written out (the
+// search stops where its curve is flat: a last bit of a score moves p by
+// 1e-4). Bound by the DCTs' dot products and the barriers between
+// passes: one pair of 63 x 63 around a masked disc takes 0.84 ms with 8 CTAs.
 // On one CTA, with strided matrix reads and 10^p formed by every thread, it
 // took 6.4 ms.
 // ---------------------------------------------------------------------------
 static constexpr int kSwThreads = 512;
 
 struct SwShared {
-  double red[2][4][kVW];
-  double sums[4];
-  double s[2];
+  double red[2][20][kVW];  // by parity of the sums: the virtual warps' partial sums
+  double sums[20];
+  double s[10];
   int go;
 };
 
@@ -925,23 +971,18 @@ PIV_D void sw_col_pass(const SwCtx& x, bool inv, const float2* in, Store store) 
   }
 }
 
-// Sums over the pair's virtual threads of up to four values, into sh->sums
+// Leaves v as partial sum `slot` of virtual warp vw in CTA r of the cluster.
+PIV_D void sw_put(SwCtx& x, int slot, int vw, double v, int r) {
+  if (x.c == 1) x.sh->red[x.par][slot][vw] = v;
+  else st_cluster(&x.sh->red[x.par][slot][vw], (unsigned)r, v);
+}
+
+// After every virtual warp's sw_put: the sums of `count` values into sh->sums
 // (every thread of the cluster calls it; it ends with a barrier).
-PIV_D void sw_sums(SwCtx& x, double a, double b, double c, double d) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int vtn = kVT / x.c;
-  if ((int)threadIdx.x < vtn) {
-    const double v = warp_sums4(a, b, c, d);
-    const int vw = (x.rank * vtn + threadIdx.x) >> 5;
-    if ((lane & 7) == 0)
-      for (int r = 0; r < x.c; ++r) {
-        if (x.c == 1) x.sh->red[x.par][lane >> 3][vw] = v;
-        else st_cluster(&x.sh->red[x.par][lane >> 3][vw], (unsigned)r, v);
-      }
-  }
+PIV_D void sw_take(SwCtx& x, int count) {
+  const int lane = threadIdx.x & 31, q = (threadIdx.x >> 5) * 2 + (lane >> 4);
   cluster_barrier(x.c);
-  if (warp < 2) {
-    const int q = warp * 2 + (lane >> 4);
+  if (q < ((count + 1) & ~1)) {  // whole warps: two values each
     double t = x.sh->red[x.par][q][lane & 15];
     for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(~0u, t, o);
     if ((lane & 15) == 0) x.sh->sums[q] = t;
@@ -950,59 +991,97 @@ PIV_D void sw_sums(SwCtx& x, double a, double b, double c, double d) {
   x.par ^= 1;
 }
 
-// GCV scores at the two announced points (gpu_smoothn.py:353-372; s in
-// sh->s); valid in warp 0. fd: DCT of both fields.
-PIV_D void sw_score2(SwCtx& x, double& fa, double& fb) {
-  const int mn = x.mn, vtn = kVT / x.c;
-  const int vt = (int)threadIdx.x < vtn ? x.rank * vtn + (int)threadIdx.x : 0x7fffffff;
-  const double s[2] = {x.sh->s[0], x.sh->s[1]};
-  double rss[2] = {0.0, 0.0}, tr[2] = {0.0, 0.0};
+// Sums over the pair's virtual threads of two values, into sh->sums[0 .. 1].
+PIV_D void sw_sums(SwCtx& x, double a, double b) {
+  const int lane = threadIdx.x & 31, vtn = kVT / x.c;
+  if ((int)threadIdx.x < vtn) {
+    const double v = warp_sums2(a, b);
+    if ((lane & 15) < x.c) sw_put(x, lane >> 4, (x.rank * vtn + threadIdx.x) >> 5, v, lane & 15);
+  }
+  sw_take(x, 2);
+}
+
+// GCV scores of the first `count` (2 or 10) announced points (gpu_smoothn.py:
+// 353-372; s in sh->s), score k in lane k of warp 0. fd: DCT of both fields.
+// The points are shared between two sets of the virtual threads (the even ones
+// and the odd ones) where the CTA has room for both.
+template <int COUNT>
+PIV_D double sw_scores(SwCtx& x) {
+  constexpr int PER = COUNT / 2;
+  const int mn = x.mn, vtn = kVT / x.c, lane = threadIdx.x & 31;
+  const int sets = 2 * vtn <= kSwThreads ? 2 : 1, set = (int)threadIdx.x / vtn;
+  const int vt = set < sets ? x.rank * vtn + (int)threadIdx.x % vtn : 0x7fffffff;
+  const int vw = vt >> 5;
   if (x.w_mean > 0.9) {
-    for (int e = vt; e < mn; e += kVT) {
-      const double l = x.lam2[e], fu = x.fd[e], fv = x.fd[mn + e];
+    for (int g = set; g < 2 && set < sets; g += sets) {  // points 2 k + g
+      double s[PER], acc[2 * PER];
 #pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        const double gm = rcp_fast(1.0 + s[k] * l);
-        const double d = gm - 1.0;
-        rss[k] += (fu * fu + fv * fv) * d * d;
-        tr[k] += gm;
+      for (int k = 0; k < PER; ++k) {
+        s[k] = x.sh->s[2 * k + g];
+        acc[k] = acc[PER + k] = 0.0;
+      }
+      for (int e = vt; e < mn; e += kVT) {
+        const double l = x.lam2[e], fu = x.fd[e], fv = x.fd[mn + e];
+        const double f2 = fma(fu, fu, __dmul_rn(fv, fv));
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+          const double gm = rcp_fast(1.0 + s[k] * l);
+          const double d = gm - 1.0;
+          acc[k] = fma(f2 * d, d, acc[k]);
+          acc[PER + k] += gm;
+        }
+      }
+      if constexpr (PER == 1) {
+        const double v = warp_sums2(acc[0], acc[1]);
+        if ((lane & 15) < x.c) sw_put(x, 2 * (lane >> 4) + g, vw, v, lane & 15);
+      } else {
+        const double v = warp_sums(acc);
+        if (lane < 2 * PER)
+          for (int r = 0; r < x.c; ++r) sw_put(x, (lane < PER ? 0 : COUNT) + 2 * (lane % PER) + g, vw, v, r);
       }
     }
   } else {
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      for (int e = vt; e < mn; e += kVT) tr[k] += rcp_fast(1.0 + s[k] * x.lam2[e]);
+    const int vt1 = (int)threadIdx.x < vtn ? vt : 0x7fffffff;  // one set: the refit takes every thread
+    for (int k = 0; k < COUNT; ++k) {
+      const double s = x.sh->s[k];
+      double rss = 0.0, tr = 0.0;
+      for (int e = vt1; e < mn; e += kVT) tr += rcp_fast(1.0 + s * x.lam2[e]);
       // f_hat = IDCT2(gamma fd), into the spare z buffer.
-      sw_row_pass(x, true, [&](int e) { return x.fd[e] * rcp_fast(1.0 + s[k] * x.lam2[e >= mn ? e - mn : e]); },
+      sw_row_pass(x, true, [&](int e) { return __dmul_rn(x.fd[e], rcp_fast(1.0 + s * x.lam2[e >= mn ? e - mn : e])); },
                   reinterpret_cast<float2*>(x.zo), reinterpret_cast<float2*>(x.tmp));
       cluster_barrier(x.c);
       sw_col_pass(x, true, reinterpret_cast<const float2*>(x.tmp), [&](int e, double v) { x.zo[e] = v; });
       cluster_barrier(x.c);
       for (int fi = 0; fi < 2; ++fi)
-        for (int e = vt; e < mn; e += kVT) {
+        for (int e = vt1; e < mn; e += kVT) {
           const double fv = x.f[fi * mn + e];
           if (isfinite(fv) || x.w[e] > 0) {
             const double d = fv - x.zo[fi * mn + e];
-            rss[k] += x.w[e] * d * d;
+            rss += x.w[e] * d * d;
           }
         }
+      if ((int)threadIdx.x < vtn) {
+        const double v = warp_sums2(rss, tr);
+        if ((lane & 15) < x.c) sw_put(x, COUNT * (lane >> 4) + k, vw, v, lane & 15);
+      }
       cluster_barrier(x.c);  // the next refit rewrites the buffers
     }
   }
-  sw_sums(x, rss[0], tr[0], rss[1], tr[1]);
+  sw_take(x, 2 * COUNT);
+  double f = 0.0;
   if (threadIdx.x < 32) {
-    const int k = threadIdx.x & 1;
-    const double q = 1.0 - x.sh->sums[2 * k + 1] / (double)mn;
-    const double f = x.sh->sums[2 * k] / x.n_finite / (q * q) / 2.0;
-    fa = __shfl_sync(~0u, f, 0);
-    fb = __shfl_sync(~0u, f, 1);
+    const int k = lane < COUNT ? lane : 0;
+    const double q = 1.0 - x.sh->sums[COUNT + k] / (double)mn;
+    f = x.sh->sums[k] / x.n_finite / (q * q) / 2.0;
   }
+  return f;
 }
 
-// Announces 10^pa and 10^pb (warp 0) and whether the search goes on.
-PIV_D void sw_announce(SwCtx& x, double pa, double pb, bool go) {
+// Announces 10^p of a point per lane (count lanes of warp 0) and whether the
+// search goes on.
+PIV_D void sw_announce(SwCtx& x, int count, double p, bool go) {
   __syncthreads();  // every read of the previous announcement is done
-  if (threadIdx.x < 2) x.sh->s[threadIdx.x] = pow(10.0, threadIdx.x ? pb : pa);
+  if ((int)threadIdx.x < count) x.sh->s[threadIdx.x] = pow(10.0, p);
   if (threadIdx.x == 0) x.sh->go = go;
   __syncthreads();
 }
@@ -1012,16 +1091,18 @@ PIV_D void sw_announce(SwCtx& x, double pa, double pb, bool go) {
 // (gpu_smoothn.py:179-193), its scalar steps in warp 0 of every CTA.
 PIV_D double sw_search(SwCtx& x, double p, bool have_p, double pmin, double pmax) {
   const bool w0 = threadIdx.x < 32;
-  auto scan_point = [&](int k) { return ((double)k * (1.0 / 9.0)) * (pmax - pmin) + pmin; };
+  const int lane = threadIdx.x & 31;
+  auto scan_point = [&](int k) { return fma((double)k * (1.0 / 9.0), pmax - pmin, pmin); };
   if (!have_p) {
-    double best_f = INFINITY;
-    for (int k = 0; k < 10; k += 2) {
-      const double pa = scan_point(k), pb = scan_point(k + 1);
-      sw_announce(x, pa, pb, true);
-      double fa = 0.0, fb = 0.0;
-      sw_score2(x, fa, fb);
-      if (k == 0 || fa < best_f) { best_f = fa; p = pa; }
-      if (fb < best_f) { best_f = fb; p = pb; }
+    sw_announce(x, 10, scan_point(lane), true);
+    const double f = sw_scores<10>(x);
+    if (w0) {
+      double best_f = INFINITY;
+#pragma unroll
+      for (int k = 0; k < 10; ++k) {
+        const double fk = __shfl_sync(~0u, f, k);
+        if (k == 0 || fk < best_f) { best_f = fk; p = scan_point(k); }
+      }
     }
   }
   Lb1 lb;
@@ -1033,11 +1114,13 @@ PIV_D double sw_search(SwCtx& x, double p, bool have_p, double pmin, double pmax
       xt = lb.xt;
       xs = lb_fd_point(xt, pmin, pmax);
     }
-    sw_announce(x, xt, xs, !lb.done);
+    sw_announce(x, 2, lane == 0 ? xt : xs, !lb.done);
     if (!x.sh->go) break;
-    double f = 0.0, fh = 0.0;
-    sw_score2(x, f, fh);
-    if (w0) lb_feed(lb, f, (fh - f) / (xs - xt));
+    const double f2 = sw_scores<2>(x);
+    if (w0) {
+      const double f = __shfl_sync(~0u, f2, 0), fh = __shfl_sync(~0u, f2, 1);
+      lb_feed(lb, f, (fh - f) / (xs - xt));
+    }
   }
   return w0 ? lb.x : p;
 }
@@ -1075,7 +1158,7 @@ k_smoothn_weighted(int m, int n, int c, const double* u_in, const double* v_in, 
     nf += fin ? 1.0 : 0.0;
     ws += wv;
   }
-  sw_sums(x, nf, ws, 0.0, 0.0);
+  sw_sums(x, nf, ws);
   nf = sh.sums[0];
   ws = sh.sums[1];
   x.n_finite = nf;
@@ -1142,7 +1225,7 @@ k_smoothn_weighted(int m, int n, int c, const double* u_in, const double* v_in, 
   const double rf = weighted ? 1.75 : 1.0;
   double p = fixed_p;
   bool have_p = !is_auto;
-  if (have_p) sw_announce(x, p, p, true);
+  if (have_p) sw_announce(x, 1, p, true);
   int k_last = 0;  // index of the last iteration run
   for (int k = 0; k < 100; ++k) {
     k_last = k;
@@ -1158,17 +1241,17 @@ k_smoothn_weighted(int m, int n, int c, const double* u_in, const double* v_in, 
       cluster_barrier(c);  // the scores read every row of fd
       p = sw_search(x, p, have_p, pmin, pmax);
       have_p = true;
-      sw_announce(x, p, p, true);
+      sw_announce(x, 1, p, true);
       cluster_barrier(c);  // fd is rewritten below
     }
     const double s = sh.s[0];
     // The inverse row pass takes the rows of fd that this CTA just wrote and
     // leaves its (hi, lo) results in their place.
-    sw_row_pass(x, true, [&](int e) { return x.fd[e] * rcp_fast(1.0 + s * lam2[e >= mn ? e - mn : e]); },
+    sw_row_pass(x, true, [&](int e) { return __dmul_rn(x.fd[e], rcp_fast(1.0 + s * lam2[e >= mn ? e - mn : e])); },
                 reinterpret_cast<float2*>(x.zo), reinterpret_cast<float2*>(x.fd));
     cluster_barrier(c);
     sw_col_pass(x, true, reinterpret_cast<const float2*>(x.fd),
-                [&](int e, double v) { x.zo[e] = rf * v + (1.0 - rf) * x.z[e]; });
+                [&](int e, double v) { x.zo[e] = fma(1.0 - rf, x.z[e], __dmul_rn(rf, v)); });
     cluster_barrier(c);
     double num = 0.0, den = 0.0;
     for (int fi = 0; fi < 2; ++fi)
@@ -1177,7 +1260,7 @@ k_smoothn_weighted(int m, int n, int c, const double* u_in, const double* v_in, 
         num += (z0 - z1) * (z0 - z1);
         den += z1 * z1;
       }
-    sw_sums(x, num, den, 0.0, 0.0);
+    sw_sums(x, num, den);
     double* t = x.z;
     x.z = x.zo;
     x.zo = t;
@@ -1262,8 +1345,10 @@ int smoothn(int m, int n, int n_pairs, const double* u_in, const double* v_in, d
     double pmin = 0, pmax = 0;
     gcv_bounds(m, n, &pmin, &pmax);
     const int c = cluster_size(n_pairs);
-    PIV_RC(launch_cluster(k_gcv, n_pairs, c, kVT / c, stream, "k_gcv", m, n, c, sc.fd, sc.f2, sc.f2f, sc.t.lam2,
-                          sc.t.lam2f, pmin, pmax, p_out, sc.s, flags));
+    auto search = c == 8 ? k_gcv<2> : k_gcv<1>;
+    PIV_RC(launch_cluster(search, n_pairs, c, c == 8 ? 2 * kVT / c : kVT / c, stream, "k_gcv", m, n, c,
+                          1.0 / (double)mn, sc.fd, sc.f2, sc.f2f, sc.t.lam2, sc.t.lam2f, pmin, pmax, p_out, sc.s,
+                          flags));
   } else {
     gam.s = nullptr;
     gam.given = pow(10.0, log10(s));
