@@ -60,11 +60,18 @@ struct LagSums {
   PIV_D static int pivot(int sum, int ss) { return (sum + ss * ss / 2) / (ss * ss); }
   PIV_D double value(int k, int ss, int di, int dj) const {
     if constexpr (whole) {
-      const double fa = (double)(sum_a - pivot(sum_a, ss) * ss * ss) / (ss * ss);
-      const double fb = (double)(sum_b - pivot(sum_b, ss) * ss * ss) / (ss * ss);
-      const int hy = ss - abs(di), hx = ss - abs(dj);
-      const double cnt = hy > 0 && hx > 0 ? (double)(hy * hx) : 0.0;
-      return (double)s[k] - (fa * (double)tb[k] + fb * (double)ta[k]) + cnt * fa * fb;
+      // With n = ss^2 pixels, A n = sum_a - ra: the value times n^2 is a whole
+      // number. 8-bit frames: below 2^53, so the value is exact.
+      const int n = ss * ss, ra = sum_a - pivot(sum_a, ss) * n, rb = sum_b - pivot(sum_b, ss) * n;
+      const int hy = ss - abs(di), hx = ss - abs(dj), cnt = hy > 0 && hx > 0 ? hy * hx : 0;
+      if constexpr (sizeof(P) == 1) {
+        const long long v = ((long long)n * s[k] - ((long long)ra * tb[k] + (long long)rb * ta[k])) * n +
+                            (long long)cnt * ra * rb;
+        return (double)v / ((double)n * n);  // a power of two
+      } else {
+        const double fa = (double)ra / n, fb = (double)rb / n;
+        return (double)s[k] - (fa * (double)tb[k] + fb * (double)ta[k]) + (double)cnt * fa * fb;
+      }
     } else {
       return s[k];
     }
@@ -242,9 +249,12 @@ static int launch_fit64(const CorrArgs& a, cudaStream_t stream) {
 }
 
 // Windows of a float64 pass with n_fft 2 and no shrink, when the caller gives
-// a list buffer and peak arrays and reads neither maps nor S2N.
+// a list buffer and peak arrays and reads neither maps nor S2N. Masked passes
+// keep the transforms: their fields enter the weighted smoothing, whose search
+// for the parameter stops where its curve is flat, and a last bit of a
+// displacement moves the smoothed field there by up to 2e-3 px.
 static bool correlate_f64_searched(const CorrArgs& a) {
-  return a.dtype == PIV_DTYPE_F64 && corr_fft_half_windows(a) && !a.maps && !a.s2n && !a.win_list && a.tie_list &&
+  return a.dtype == PIV_DTYPE_F64 && corr_fft_half_windows(a) && !a.win_mask && !a.maps && !a.s2n && !a.win_list && a.tie_list &&
          a.tie_list_count && a.peak_i && a.peak_j && a.cand && a.cand_count == a.tie_list_count + 1 &&
          a.cand_cap > 0;
 }

@@ -43,7 +43,8 @@ def _frames(seed, h, w, dtype, kind):
                                         ("float64", "plain"), ("float64", "ties"), ("float64", "offset"),
                                         ("float64", "tiny"), ("float64", "nan")])
 @pytest.mark.parametrize("shape", [(64, 64), (101, 147)])
-def test_peaks_and_fits_are_the_float64_maps(ss, dtype, kind, shape):
+@pytest.mark.parametrize("masked", [False, True])  # masked passes take the float64 transforms
+def test_peaks_and_fits_are_the_float64_maps(ss, dtype, kind, shape, masked):
     import torch
 
     from openpiv_gpu import _build, _lib
@@ -60,23 +61,24 @@ def test_peaks_and_fits_are_the_float64_maps(ss, dtype, kind, shape):
     da, db = (torch.as_tensor(np.ascontiguousarray(f).view(np.uint8)).cuda() for f in (a, b))
     pt = _lib.PIXEL[{"uint8": "u8", "uint16": "u16", "float32": "f32", "float64": "f64"}[dtype]]
     mask = np.zeros((m, n), dtype=np.uint8)
-    mask[0, 0] = 1
+    mask[0, 0] = masked
     dm = torch.as_tensor(mask).cuda()
+    mask_ptr = dm.data_ptr() if masked else None
     f64 = _lib.DTYPE["float64"]
     stream = torch.cuda.current_stream().cuda_stream
     maps = torch.empty((m, n, N, N), dtype=torch.float64, device="cuda")
     _lib.check(lib.piv_correlate_maps(ctypes.byref(geom), 1, da.data_ptr(), db.data_ptr(), pt, f64, N, 1,
-                                      dm.data_ptr(), maps.data_ptr(), _lib.DFT["fft"], stream))
+                                      mask_ptr, maps.data_ptr(), _lib.DFT["fft"], stream))
     u = torch.empty((m, n), dtype=torch.float64, device="cuda")
     v = torch.empty_like(u)
     pi = torch.empty((m, n), dtype=torch.int32, device="cuda")
     pj = torch.empty_like(pi)
     _lib.check(lib.piv_correlate(ctypes.byref(geom), 1, da.data_ptr(), db.data_ptr(), pt, f64, N, 1,
-                                 _lib.SUBPIXEL["gaussian"], dm.data_ptr(), u.data_ptr(), v.data_ptr(), pi.data_ptr(),
+                                 _lib.SUBPIXEL["gaussian"], mask_ptr, u.data_ptr(), v.data_ptr(), pi.data_ptr(),
                                  pj.data_ptr(), 0, 2, None, _lib.DFT["fft"], stream))
     u2, v2 = torch.empty_like(u), torch.empty_like(u)  # without peak arrays: the same fields
     _lib.check(lib.piv_correlate(ctypes.byref(geom), 1, da.data_ptr(), db.data_ptr(), pt, f64, N, 1,
-                                 _lib.SUBPIXEL["gaussian"], dm.data_ptr(), u2.data_ptr(), v2.data_ptr(), None, None, 0,
+                                 _lib.SUBPIXEL["gaussian"], mask_ptr, u2.data_ptr(), v2.data_ptr(), None, None, 0,
                                  2, None, _lib.DFT["fft"], stream))
     maps, u, v, u2, v2, pi, pj = (t.cpu().numpy() for t in (maps, u, v, u2, v2, pi, pj))
     np.testing.assert_array_equal(u, u2)
@@ -84,7 +86,7 @@ def test_peaks_and_fits_are_the_float64_maps(ss, dtype, kind, shape):
     flat = maps.reshape(m, n, -1)
     at = np.argmax(np.where(np.isnan(flat), np.inf, flat), axis=2)  # a map of NaN: its first NaN, as argmax has it
     np.testing.assert_array_equal(pi * N + pj, at)
-    assert np.isnan(u[0, 0]) and np.isnan(v[0, 0])
+    assert not masked or (np.isnan(u[0, 0]) and np.isnan(v[0, 0]))
     for r in range(m):
         for k in range(n):
             if mask[r, k]:
