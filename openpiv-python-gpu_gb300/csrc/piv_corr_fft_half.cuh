@@ -15,7 +15,7 @@
 //   * the twiddles inside the register DFTs are constants.
 // Shared-memory traffic and instruction issue bound the kernel. Measured (one
 // 1024 x 1024 pair at 50% overlap, 8-bit frames; the general kernel, then
-// this): N = 32 136 -> 64 us, N = 64 139 -> 68 us, N = 128 174 -> 92 us.
+// this): N = 32 136 -> 57 us, N = 64 139 -> 68 us, N = 128 174 -> 90 us.
 #pragma once
 
 #include "piv_corr_common.cuh"
@@ -56,6 +56,18 @@ PIV_D Cplx<float> cmul_k(Cplx<float> a, float wx, float wy) {
 }
 PIV_D Cplx<float> cmul_k(Cplx<float> a, Cplx<float> w) { return cmul_k(a, w.x, w.y); }
 
+// a + b and a - b of both parts in one packed float32 pair instruction each
+// (rounded as the scalar ones; half the issue slots): N = 32 64.2 -> 56.5 us,
+// N = 64 68.4 -> 67.6 us, N = 128 92.2 -> 90.4 us on the pair above. A rotated
+// operand (W = -+i) takes scalar sums instead: packing its swapped parts would
+// cost the moves that the pair saves.
+PIV_D void butterfly(Cplx<float> a, Cplx<float> b, Cplx<float>& sum, Cplx<float>& dif) {
+  asm("{\n.reg .b64 a, b, s, d;\nmov.b64 a, {%4, %5};\nmov.b64 b, {%6, %7};\nadd.rn.f32x2 s, a, b;\nsub.rn.f32x2 d, a, b;\n"
+      "mov.b64 {%0, %1}, s;\nmov.b64 {%2, %3}, d;\n}\n"
+      : "=f"(sum.x), "=f"(sum.y), "=f"(dif.x), "=f"(dif.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+}
+
 // Radix-2 stages from span LEN up of the R-point register DFT (dft_stage with
 // constant twiddles).
 template <int R, int LEN, bool INV>
@@ -66,16 +78,18 @@ PIV_D void dft_stage_k(Cplx<float> (&y)[R]) {
     for (int j = 0; j < LEN / 2; ++j) {
       const Cplx<float> a = y[i + j];
       Cplx<float> b = y[i + j + LEN / 2];
-      if (j != 0) {
-        if (LEN >= 4 && j == LEN / 4) {
-          b = INV ? cmake<float>(-b.y, b.x) : cmake<float>(b.y, -b.x);
-        } else {
-          const TwPair w = tw32(j * (32 / LEN));  // constant once unrolled
-          b = cmul_k(b, w.x, INV ? -w.y : w.y);
-        }
+      if (LEN >= 4 && j == LEN / 4) {
+        // W = -i (forward) or +i (inverse): a +- (b.y, -b.x) or its negative.
+        const Cplx<float> lo = cmake<float>(a.x + b.y, a.y - b.x), hi = cmake<float>(a.x - b.y, a.y + b.x);
+        y[i + j] = INV ? hi : lo;
+        y[i + j + LEN / 2] = INV ? lo : hi;
+        continue;
       }
-      y[i + j] = cadd(a, b);
-      y[i + j + LEN / 2] = csub(a, b);
+      if (j != 0) {
+        const TwPair w = tw32(j * (32 / LEN));  // constant once unrolled
+        b = cmul_k(b, w.x, INV ? -w.y : w.y);
+      }
+      butterfly(a, b, y[i + j], y[i + j + LEN / 2]);
     }
   }
   if constexpr (LEN < R) dft_stage_k<R, 2 * LEN, INV>(y);
