@@ -232,11 +232,6 @@ PIV_D void st8(unsigned char* base, uint32_t off, const float* v) {
   *reinterpret_cast<uint4*>(base + off) = q;
 }
 
-PIV_D void sth(unsigned char* base, uint32_t off, float v) {
-  if (!in_dyn_smem(base + off, 2)) return;
-  *reinterpret_cast<__half*>(base + off) = __float2half_rn(v);
-}
-
 template <bool SPLIT>
 PIV_D void st8s(unsigned char* base, int lo, uint32_t off, const float* v) {
   st8(base, off, v);
@@ -248,12 +243,24 @@ PIV_D void st8s(unsigned char* base, int lo, uint32_t off, const float* v) {
   }
 }
 
-template <bool SPLIT>
-PIV_D void sths(unsigned char* base, int lo, uint32_t off, float v) {
-  if (!in_dyn_smem(base + off, 2) || (SPLIT && !in_dyn_smem(base + lo + off, 2))) return;
-  const __half h = __float2half_rn(v);
-  *reinterpret_cast<__half*>(base + off) = h;
-  if (SPLIT) *reinterpret_cast<__half*>(base + lo + off) = __float2half_rn(v - __half2float(h));
+// Constant operand of ROWS rows and K columns (no-swizzle K-major, off_k) with
+// element (r, k) = value(r, k): eight columns of one row per thread and step,
+// which is the tile's chunk c at byte 16 c, so that neighbouring threads store
+// neighbouring chunks without bank conflicts. Every CTA builds its constants
+// before its first tile, so a small launch is bound by it: one 2-byte store,
+// index chain and rounding per element took 8 us more (1037 x 1393 frames,
+// ss = 32 at 50% overlap: launch 55.5 -> 47.5 us; a mixed submission's three
+// ss = 32 launches 380 -> 288 us, its ss = 64 ones 258 -> 243 us).
+template <bool SPLIT, int ROWS, int K, int NT, class Value>
+PIV_D void fill_operand(unsigned char* base, int lo, int tid, Value value) {
+  static_assert(ROWS % 8 == 0 && K % 8 == 0, "whole chunks");
+  for (int c = tid; c < ROWS * K / 8; c += NT) {
+    const int r = c / K * 8 + (c & 7), k0 = (c >> 3) % (K / 8) * 8;
+    float v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = value(r, k0 + i);
+    st8s<SPLIT>(base, lo, (uint32_t)(16 * c), v);
+  }
 }
 
 // D (+)= A B over `ks_n` k-steps, issued by one elected lane of the calling
@@ -426,31 +433,26 @@ __global__ void __launch_bounds__(TcLayout<SS, SPLIT>::NT, TcLayout<SS, SPLIT>::
   __syncthreads();
   const float inv_n = 1.0f / (float)N;
   const int p0 = SS / 2;
-  for (int e = tid; e < N * SS; e += NT) {  // F[k][x]
-    const int k = e / SS, x = e % SS, f = k >> 1, q = (f * (x + p0)) % N;
-    float v;
-    if (k == 0) v = 1.0f;
-    else if (k == 1) v = ((x + p0) & 1) ? -1.0f : 1.0f;
-    else v = (k & 1) ? tw_im[q] : tw_re[q];
-    sths<SPLIT>(sm + L::B1, L::NB1, off_k(k, x, SS), v);
-  }
+  fill_operand<SPLIT, N, SS, NT>(sm + L::B1, L::NB1, tid, [&](int k, int x) {  // F[k][x]
+    const int q = ((k >> 1) * (x + p0)) % N;
+    if (k == 0) return 1.0f;
+    if (k == 1) return ((x + p0) & 1) ? -1.0f : 1.0f;
+    return (k & 1) ? tw_im[q] : tw_re[q];
+  });
   // The split form keeps the inverse DFTs' 1/N out of B3 and B4 (their lo
   // parts would fall below the fp16 normal range) and scales Q and U instead.
   const float bscale = SPLIT ? 1.0f : inv_n;
-  for (int e = tid; e < 3 * N * HN; e += NT) {  // B3 blocks C, -S, S: [r][g]
-    const int blk = e / (N * HN), r = (e / HN) % N, g = e % HN;
-    const int q = (g * r) % N;
-    const float v = stage3_weight(blk, r, g, tw_re[q] * bscale, -tw_im[q] * bscale, bscale);
-    sths<SPLIT>(sm + L::B3 + blk * L::P * L::NB3, L::NB3, off_k(r, g, HN), v);
-  }
-  for (int e = tid; e < N * N; e += NT) {  // B4[s][kappa], kappa = (part, c)
-    const int s_ = e / N, kap = e % N, part = kap / HN, c = kap % HN;
-    const int q = (c * s_) % N;
-    float v;
-    if (c == 0) v = part == 0 ? bscale : ((s_ & 1) ? -bscale : bscale);
-    else v = part == 0 ? 2.0f * tw_re[q] * bscale : 2.0f * tw_im[q] * bscale;
-    sths<SPLIT>(sm + L::B4, L::NB4, off_k(s_, kap, N), v);
-  }
+#pragma unroll 1
+  for (int blk = 0; blk < 3; ++blk)  // B3 blocks C, -S, S: [r][g]
+    fill_operand<SPLIT, N, HN, NT>(sm + L::B3 + blk * L::P * L::NB3, L::NB3, tid, [&](int r, int g) {
+      const int q = (g * r) % N;
+      return stage3_weight(blk, r, g, tw_re[q] * bscale, -tw_im[q] * bscale, bscale);
+    });
+  fill_operand<SPLIT, N, N, NT>(sm + L::B4, L::NB4, tid, [&](int s_, int kap) {  // B4[s][kappa], kappa = (part, c)
+    const int part = kap / HN, c = kap % HN, q = (c * s_) % N;
+    if (c == 0) return part == 0 ? bscale : ((s_ & 1) ? -bscale : bscale);
+    return part == 0 ? 2.0f * tw_re[q] * bscale : 2.0f * tw_im[q] * bscale;
+  });
   const float oscale = SPLIT ? inv_n : 1.0f;  // applied to Q and U in the split form
   if (warp == 0) tc::tmem_alloc(&tmem_base_s, L::TCOLS);
   tc::fence_async_smem();
@@ -1105,28 +1107,23 @@ __global__ void __maxnreg__(96) k_corr_tc64(CorrArgs a, int* status) {
   __syncthreads();
   const float inv_n = 1.0f / (float)N;
   const int p0 = SS / 2;
-  for (int e = tid; e < N * SS; e += L::NT) {  // F[k][x]
-    const int k = e / SS, x = e % SS, f = k >> 1, qq = (f * (x + p0)) % N;
-    float v;
-    if (k == 0) v = 1.0f;
-    else if (k == 1) v = ((x + p0) & 1) ? -1.0f : 1.0f;
-    else v = (k & 1) ? tw_im[qq] : tw_re[qq];
-    sth(sm + L::B1, off_k(k, x, SS), v);
-  }
-  for (int e = tid; e < 3 * N * HN; e += L::NT) {  // B3 blocks C, -S, S: [r][g]
-    const int blk = e / (N * HN), r = (e / HN) % N, g = e % HN;
-    const int qq = (g * r) % N;
-    sth(sm + L::B3 + blk * L::NB3, off_k(r, g, HN),
-        stage3_weight(blk, r, g, tw_re[qq] * inv_n, -tw_im[qq] * inv_n, inv_n));
-  }
-  for (int e = tid; e < N * N; e += L::NT) {  // B4[s][kappa = (part, c)]
-    const int s_ = e / N, kap = e % N, part = kap / HN, c = kap % HN;
-    const int qq = (c * s_) % N;
-    float v;
-    if (c == 0) v = part == 0 ? inv_n : ((s_ & 1) ? -inv_n : inv_n);
-    else v = part == 0 ? 2.0f * tw_re[qq] * inv_n : 2.0f * tw_im[qq] * inv_n;
-    sth(sm + L::B4, off_k(s_, kap, N), v);
-  }
+  fill_operand<false, N, SS, L::NT>(sm + L::B1, 0, tid, [&](int k, int x) {  // F[k][x]
+    const int qq = ((k >> 1) * (x + p0)) % N;
+    if (k == 0) return 1.0f;
+    if (k == 1) return ((x + p0) & 1) ? -1.0f : 1.0f;
+    return (k & 1) ? tw_im[qq] : tw_re[qq];
+  });
+#pragma unroll 1
+  for (int blk = 0; blk < 3; ++blk)  // B3 blocks C, -S, S: [r][g]
+    fill_operand<false, N, HN, L::NT>(sm + L::B3 + blk * L::NB3, 0, tid, [&](int r, int g) {
+      const int qq = (g * r) % N;
+      return stage3_weight(blk, r, g, tw_re[qq] * inv_n, -tw_im[qq] * inv_n, inv_n);
+    });
+  fill_operand<false, N, N, L::NT>(sm + L::B4, 0, tid, [&](int s_, int kap) {  // B4[s][kappa = (part, c)]
+    const int part = kap / HN, c = kap % HN, qq = (c * s_) % N;
+    if (c == 0) return part == 0 ? inv_n : ((s_ & 1) ? -inv_n : inv_n);
+    return part == 0 ? 2.0f * tw_re[qq] * inv_n : 2.0f * tw_im[qq] * inv_n;
+  });
   if (warp == 0) tc::tmem_alloc(&tmem_base_s, L::TCOLS);
   tc::fence_async_smem();
   tc::fence_before_sync();
