@@ -440,20 +440,29 @@ __global__ void __launch_bounds__(kDctThreads) k_dct_lines(int m, int n, int bat
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = nt / 32;
-  auto fetch = [&](int l, int e) {
-    const double* p = src_s[l];
-    double x = p ? p[(long long)e * step] : 0.0;
-    if (INV && gam.lam2) x = rcp_fast(1.0 + s_s[l] * gam.lam2[at_s[l] + e * step]) * x;
-    xs[e * S + l] = x;
-  };
-  // Coalesced along the line for rows, across lines for columns.
-  if (cols) {
-#pragma unroll 8
-    for (int e = warp; e < L; e += nw) fetch(lane, e);
-  } else {
-#pragma unroll 4
-    for (unsigned idx = threadIdx.x; idx < (unsigned)(kDctLines * L); idx += nt)
-      fetch((int)(idx / (unsigned)L), (int)(idx % (unsigned)L));
+  // Staging, coalesced along the line for rows and across lines for columns:
+  // kBatch loads of a thread are in flight together (64 pairs of 63 x 63, four
+  // passes: 139 us with four at a time, 126 us with eight).
+  constexpr int kBatch = DF ? 8 : 16;
+  const unsigned n_el = (unsigned)(kDctLines * L);
+  for (unsigned b0 = threadIdx.x; b0 < n_el; b0 += kBatch * nt) {
+    double v[kBatch];
+    int l[kBatch], e[kBatch];
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k) {
+      const unsigned id = b0 + k * nt;
+      const bool ok = id < n_el;
+      l[k] = !ok ? 0 : (int)(cols ? id % kDctLines : id / (unsigned)L);
+      e[k] = !ok ? 0 : (int)(cols ? id / kDctLines : id % (unsigned)L);
+      const double* p = ok ? src_s[l[k]] : nullptr;
+      v[k] = p ? p[(long long)e[k] * step] : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k) {
+      if (b0 + k * nt >= n_el) break;
+      if (INV && gam.lam2) v[k] = rcp_fast(1.0 + s_s[l[k]] * gam.lam2[at_s[l[k]] + e[k] * step]) * v[k];
+      xs[e[k] * S + l[k]] = v[k];
+    }
   }
   __syncthreads();
   const int split_n = gridDim.y, share = blockIdx.y;
@@ -501,6 +510,7 @@ __global__ void __launch_bounds__(kDctThreads) k_dct_lines(int m, int n, int bat
         const float* ckl = cl + (long long)k * L;
         DfAcc acc;
         if (L & 1) acc.add(ckh[h], ckl[h], mid_h, mid_l);
+#pragma unroll 8
         for (int i = 0; i < h; ++i) acc.add(ckh[i], ckl[i], sh[i * S + lane], sl[i * S + lane]);
         float rh, rl;
         acc.result(rh, rl);
@@ -536,7 +546,9 @@ __global__ void __launch_bounds__(kDctThreads) k_dct_lines(int m, int n, int bat
     __syncthreads();
     for (int i = share * nw + warp; i < hc; i += nw * split_n) {
       DfAcc ev, od;
+#pragma unroll 8
       for (int k = 0; k < L; k += 2) ev.add(ch[(long long)k * L + i], cl[(long long)k * L + i], xh[k * S + lane], xl[k * S + lane]);
+#pragma unroll 8
       for (int k = 1; k < L; k += 2) od.add(ch[(long long)k * L + i], cl[(long long)k * L + i], xh[k * S + lane], xl[k * S + lane]);
       float eh, el, oh, ol;
       ev.result(eh, el);
@@ -586,13 +598,15 @@ __global__ void __launch_bounds__(kDctThreads) k_dct_lines(int m, int n, int bat
   }
 }
 
-__global__ void k_apply_gamma(long long mn, int n_pairs, DctGamma gam, double* __restrict__ fd) {
-  const int pair = blockIdx.y;
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 2 * mn) return;
-  const long long e = t % mn;
-  double* f = fd + (long long)pair * 2 * mn + t;
-  *f = rcp_fast(1.0 + gam.of(pair) * gam.lam2[e]) * *f;
+// Both fields of every pair times 1 / (1 + s lambda^2).
+__global__ void k_apply_gamma(long long mn, DctGamma gam, DctIo io) {
+  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x, pair = blockIdx.y;
+  if (e >= mn) return;
+  const double g = rcp_fast(1.0 + gam.of(pair) * gam.lam2[e]);
+  double* u = io.field(2 * pair) + e;
+  double* v = io.field(2 * pair + 1) + e;
+  *u = g * *u;
+  *v = g * *v;
 }
 
 // One DCT pass over `batch` fields: forward (DCT-II) or inverse (DCT-III)
@@ -600,35 +614,40 @@ __global__ void k_apply_gamma(long long mn, int n_pairs, DctGamma gam, double* _
 // of up to kDctMaxLen positions take the double-float products, longer ones
 // the float64 products (the double-float error grows with the length), both
 // staged with the symmetric split. Measured, the four passes of one pair: 31 x
-// 31 30 us, 253 x 253 200 us (plain float64 dot products 283 us), 170 x 137
-// 106 us (87 us, plus 5 us for gamma and 6 us for the copies, which are part
+// 31 30 us, 253 x 253 174 us (plain float64 dot products 283 us), 170 x 137
+// 89 us (87 us, plus 5 us for gamma and 6 us for the copies, which are part
 // of these passes); 16 pairs of 253 x 253 2.13 ms (3.36 ms), of which 1.65 ms
-// at the float64 rate.
+// at the float64 rate. The staging's loads in flight matter as much as the
+// products for a few lines: four of a thread at a time 200 / 106 us.
 template <bool INV>
 static int dct_pass(int m, int n, int batch, int cols, const SmoothTables& t, DctIo in, DctIo out, DctGamma gam,
                     cudaStream_t stream) {
   const int L = cols ? m : n;
   const long long n_lines = (long long)batch * (cols ? n : m);
-  if (L > kDctLongLen) {
-    if (gam.lam2) {
-      const long long mn = (long long)m * n;
-      k_apply_gamma<<<dim3((unsigned)((2 * mn + 255) / 256), (unsigned)(batch / 2)), 256, 0, stream>>>(mn, batch / 2,
-                                                                                                     gam, in.u);
-    }
-    const long long tot = (long long)m * n * batch;
-    const int mode = cols ? (INV ? 3 : 2) : (INV ? 1 : 0);
-    k_dct_apply<<<(unsigned)((tot + 255) / 256), 256, 0, stream>>>(m, n, batch, mode, cols ? t.cm : t.cn, in, out);
-    return check("k_dct_apply");
-  }
   const bool df = L <= kDctMaxLen;
-  const float* cf = cols ? t.cmf : t.cnf;
-  const double* cd = cols ? t.cm : t.cn;
   const long long blocks = (n_lines + kDctLines - 1) / kDctLines;
   // Shares of the outputs: as many as the SMs take, each warp of a share
   // with at least one turn (fewer warps per CTA stage the lines too slowly).
   const int turns = df ? (INV ? (L + 1) / 2 : L) : (INV ? (L + 3) / 4 : (L + 1) / 2);
   const long long room = blocks < sm_count() ? sm_count() / blocks : 1;
   const int shares = (int)std::min<long long>((turns + kDctThreads / 32 - 1) / (kDctThreads / 32), room);
+  // Every share of the staged kernels scales all of its lines' inputs, nine
+  // float64 instructions each: from three shares on, one launch that scales
+  // them once costs less (253 x 253, nine shares: the inverse row
+  // pass 56 -> 41 us for a launch of 3 us).
+  if (gam.lam2 && (L > kDctLongLen || (!df && shares >= 3))) {
+    const long long mn = (long long)m * n;
+    k_apply_gamma<<<dim3((unsigned)((mn + 127) / 128), (unsigned)(batch / 2)), 128, 0, stream>>>(mn, gam, in);
+    gam = DctGamma{nullptr, nullptr, 0.0};
+  }
+  if (L > kDctLongLen) {
+    const long long tot = (long long)m * n * batch;
+    const int mode = cols ? (INV ? 3 : 2) : (INV ? 1 : 0);
+    k_dct_apply<<<(unsigned)((tot + 255) / 256), 256, 0, stream>>>(m, n, batch, mode, cols ? t.cm : t.cn, in, out);
+    return check("k_dct_apply");
+  }
+  const float* cf = cols ? t.cmf : t.cnf;
+  const double* cd = cols ? t.cm : t.cn;
   const int threads = kDctThreads;
   const dim3 grid((unsigned)blocks, (unsigned)shares);
   if (df) {

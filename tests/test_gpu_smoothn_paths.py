@@ -80,3 +80,18 @@ def test_line_lengths_around_the_kernels_limits(shape, pairs):
         for f, g in ((u, got[0]), (v, got[1])):
             ref = idctn(dctn(f[k], norm="ortho") / (1 + s * lam * lam), norm="ortho")
             np.testing.assert_allclose(g[k], ref, rtol=0, atol=tol)
+
+
+# A pair alone has three shares of outputs or more, and its inputs are scaled
+# by a launch of their own; with 40 pairs the only share scales them itself.
+@pytest.mark.parametrize("shape", [(92, 91), (91, 92)])
+@pytest.mark.parametrize("s", [0.7, float("nan")])
+def test_scaling_before_the_inverse_does_not_depend_on_the_shares(shape, s):
+    env = _env()
+    u, v = _fields(6, 40, *shape)
+    ub, vb, pb = _smooth(env, u, v, s)
+    for k in (0, 21, 39):
+        ua, va, pa = _smooth(env, u[k:k + 1], v[k:k + 1], s)
+        np.testing.assert_array_equal(ua[0], ub[k])
+        np.testing.assert_array_equal(va[0], vb[k])
+        assert pa[0] == pb[k]
