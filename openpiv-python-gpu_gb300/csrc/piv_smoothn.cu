@@ -633,8 +633,8 @@ static int dct_pass(int m, int n, int batch, int cols, const SmoothTables& t, Dc
   const int shares = (int)std::min<long long>((turns + kDctThreads / 32 - 1) / (kDctThreads / 32), room);
   // Every share of the staged kernels scales all of its lines' inputs, nine
   // float64 instructions each: from three shares on, one launch that scales
-  // them once costs less (253 x 253, nine shares: the inverse row
-  // pass 56 -> 41 us for a launch of 3 us).
+  // them once costs less (253 x 253, nine shares: both inverse passes 105 us,
+  // now 82 us and a launch of 3 us).
   if (gam.lam2 && (L > kDctLongLen || (!df && shares >= 3))) {
     const long long mn = (long long)m * n;
     k_apply_gamma<<<dim3((unsigned)((mn + 127) / 128), (unsigned)(batch / 2)), 128, 0, stream>>>(mn, gam, in);

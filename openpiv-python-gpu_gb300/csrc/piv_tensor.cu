@@ -66,8 +66,9 @@ struct TcLayout {
   // [128][2N] K-major; A4 2 x [128][N] MN-major.
   static constexpr int OP = B4 + P * NB4;
   static constexpr int STG = OP + P * NOP;              // next tile's float rows [frame][128][SS], 16-byte chunks swizzled
-  static constexpr int NBR = STG + 2 * 128 * SS * 4;    // [W][3][N] floats: map rows pi-1, pi, pi+1 (natural columns)
-  static constexpr int END = NBR + W * 3 * N * 4;
+  static constexpr int NBR = STG + 2 * 128 * SS * 4;    // [W][3][NBP] floats: map rows pi-1, pi, pi+1 (natural columns)
+  static constexpr int NBP = N + 4;                     // pitch: the three lanes of a window store to different banks
+  static constexpr int END = NBR + W * 3 * NBP * 4;
   static constexpr int A1_BYTES = 128 * SS * 2;
   static constexpr int A2_BYTES = 128 * SS * 2;
   static constexpr int A4_BYTES = 128 * N * 2;
@@ -812,7 +813,7 @@ __global__ void __launch_bounds__(TcLayout<SS, SPLIT>::NT, TcLayout<SS, SPLIT>::
     // ---- Epilogue. Row rt*128 + tid of the tile is map row r of window w
     // (scaled by 2^(e_a + e_b)); shifted row index i = r ^ N/2, shifted
     // column j = s ^ N/2. Lags without window overlap (i = 0 or j = 0) are 0.
-    float* nbrow = reinterpret_cast<float*>(sm + L::NBR);  // [W][3][N]: rows pi-1, pi, pi+1 (natural columns)
+    float* nbrow = reinterpret_cast<float*>(sm + L::NBR);  // [W][3][NBP]: rows pi-1, pi, pi+1 (natural columns)
     // Subpixel fit and outputs of window ww with flat peak index pidx (its
     // neighbour rows in nbrow).
     auto finish = [&](int ww, int pidx) {
@@ -824,7 +825,7 @@ __global__ void __launch_bounds__(TcLayout<SS, SPLIT>::NT, TcLayout<SS, SPLIT>::
         // x 2^ue as two exact power-of-two products (|ue| <= 240; each factor is a normal float).
         const float s1 = pow2i(ue >> 1), s2 = pow2i(ue - (ue >> 1));
         auto at = [&](int i, int j) -> float {
-          return (i == 0 || j == 0) ? 0.f : nbrow[(ww * 3 + (i - pi_ + 1)) * N + (j ^ HN)] * s1 * s2;
+          return (i == 0 || j == 0) ? 0.f : nbrow[(ww * 3 + (i - pi_ + 1)) * L::NBP + (j ^ HN)] * s1 * s2;
         };
         subpixel_fit(a.subpixel, pi_, pj, at(pi_, pj), at(pi_ - 1, pj), at(pi_ + 1, pj), at(pi_, pj - 1),
                      at(pi_, pj + 1), isp, jsp);
@@ -844,7 +845,7 @@ __global__ void __launch_bounds__(TcLayout<SS, SPLIT>::NT, TcLayout<SS, SPLIT>::
       if (sq.peak_i) sq.peak_i[gl] = pi_;
       if (sq.peak_j) sq.peak_j[gl] = pj;
     };
-    auto peak_row = [&](int ww) { return nbrow + (ww * 3 + 1) * N; };
+    auto peak_row = [&](int ww) { return nbrow + (ww * 3 + 1) * L::NBP; };
     bool stop = false;
     if constexpr (N == 32 && TPL == 1) {
       // One window per warp and row tile (N = 32 rows): the warp finds its
@@ -881,7 +882,7 @@ __global__ void __launch_bounds__(TcLayout<SS, SPLIT>::NT, TcLayout<SS, SPLIT>::
           if (lane == 0) sec_key[w] = k;
         }
         if ((ties && i == pi_) || (pi_ > 0 && pi_ < N - 1 && pj > 0 && pj < N - 1 && i >= pi_ - 1 && i <= pi_ + 1)) {
-          float4* dst = reinterpret_cast<float4*>(nbrow + (w * 3 + (i - pi_ + 1)) * N);
+          float4* dst = reinterpret_cast<float4*>(nbrow + (w * 3 + (i - pi_ + 1)) * L::NBP);
           if (in_dyn_smem(dst, N * 4))
 #pragma unroll
             for (int c4 = 0; c4 < N / 4; ++c4)
@@ -966,7 +967,7 @@ __global__ void __launch_bounds__(TcLayout<SS, SPLIT>::NT, TcLayout<SS, SPLIT>::
           tc::tmem_ld_wait();
           tc::reg_fence(v);
           if (mine) {
-            float4* dst = reinterpret_cast<float4*>(nbrow + (w * 3 + (i - pi_ + 1)) * N);
+            float4* dst = reinterpret_cast<float4*>(nbrow + (w * 3 + (i - pi_ + 1)) * L::NBP);
             if (in_dyn_smem(dst, N * 4))
 #pragma unroll
               for (int c4 = 0; c4 < N / 4; ++c4)
