@@ -548,31 +548,88 @@ __global__ void __launch_bounds__(TcLayout<SS, SPLIT>::NT, TcLayout<SS, SPLIT>::
     cp_async_commit();
   }
   const bool ties = any_tie_output(seg_s, n_seg);
-  // Near-tie flag of window `lane` of the current tile (lanes < W of the
+  float* nbrow = reinterpret_cast<float*>(sm + L::NBR);  // [W][3][NBP]: rows pi-1, pi, pi+1 (natural columns)
+  // First maximum of window w over its NPART warp partials (each thread that
+  // needs it combines them itself: no further barrier).
+  auto window_peak = [&](int w) -> int {
+    float v = NPART > 1 ? pk_val[w][0] : 0.f;
+    int idx = pk_idx[w][0];
+#pragma unroll
+    for (int p = 1; p < NPART; ++p)
+      if (pk_val[w][p] > v || (pk_val[w][p] == v && pk_idx[w][p] < idx)) {
+        v = pk_val[w][p];
+        idx = pk_idx[w][p];
+      }
+    return idx;
+  };
+  // Near-tie flag of window `lane` of the tile in slot psl (lanes < W of the
   // calling warp; tile_near_ties's result) to the window's outputs.
-  int cur_sl = 0;
-  long long cur_g0 = 0;
-  auto write_near_ties = [&](bool tie) {
-    if (lane >= W || cur_g0 + lane >= total) return;
-    const CorrSeg& sq = seg_s[win_seg[cur_sl][lane]];
-    const long long gl = win_loc[cur_sl][lane];
-    tie = tie && win_valid[cur_sl][lane];
+  auto write_near_ties = [&](int psl, long long pg0, bool tie) {
+    if (lane >= W || pg0 + lane >= total) return;
+    const CorrSeg& sq = seg_s[win_seg[psl][lane]];
+    const long long gl = win_loc[psl][lane];
+    tie = tie && win_valid[psl][lane];
     if (!in_bounds(gl >= 0 && gl < (long long)sq.n_pairs * sq.m * sq.n)) return;
     if (sq.near_tie) sq.near_tie[gl] = tie ? 1 : 0;
     if (tie && sq.tie_count) atomicAdd(sq.tie_count, 1);
   };
+  // Subpixel fit and outputs of window ww of the tile in slot psl with flat
+  // peak index pidx (its neighbour rows in nbrow).
+  auto finish = [&](int psl, int ww, int pidx) {
+    const int pi_ = pidx / N, pj = pidx % N;
+    float isp = (float)pi_, jsp = (float)pj;
+    if (pi_ > 0 && pi_ < N - 1 && pj > 0 && pj < N - 1) {
+      const int ue = -sc_e[psl][0][ww] - sc_e[psl][1][ww];
+      // Shifted (i, j) -> stored row slot i - pi + 1, natural column j ^ N/2.
+      // x 2^ue as two exact power-of-two products (|ue| <= 240; each factor is a normal float).
+      const float s1 = pow2i(ue >> 1), s2 = pow2i(ue - (ue >> 1));
+      auto at = [&](int i, int j) -> float {
+        return (i == 0 || j == 0) ? 0.f : nbrow[(ww * 3 + (i - pi_ + 1)) * L::NBP + (j ^ HN)] * s1 * s2;
+      };
+      subpixel_fit(a.subpixel, pi_, pj, at(pi_, pj), at(pi_ - 1, pj), at(pi_ + 1, pj), at(pi_, pj - 1),
+                   at(pi_, pj + 1), isp, jsp);
+    }
+    const CorrSeg& sq = seg_s[win_seg[psl][ww]];
+    const long long gl = win_loc[psl][ww];
+    float* uo = reinterpret_cast<float*>(sq.u);
+    float* vo = reinterpret_cast<float*>(sq.v);
+    if (!in_bounds(gl >= 0 && gl < (long long)sq.n_pairs * sq.m * sq.n)) return;
+    if (win_valid[psl][ww]) {
+      uo[gl] = sub_rn(jsp, (float)HN);
+      vo[gl] = sub_rn(isp, (float)HN);
+    } else {
+      uo[gl] = NAN;
+      vo[gl] = NAN;
+    }
+    if (sq.peak_i) sq.peak_i[gl] = pi_;
+    if (sq.peak_j) sq.peak_j[gl] = pj;
+  };
+  // The near-tie test and the fits of the tile in slot psl, in warps 1 and 3,
+  // once every warp has left its peaks and neighbour rows (a barrier before):
+  // they run while stage 1 of the next tile is on the tensor core, off the
+  // path from one tile's map to the next tile's staging, and need no barrier
+  // of their own. Measured against fits right after the map (64 pairs of 1024
+  // x 1024): ss 16 1449 -> 1398 us, ss 32 1568 -> 1572 us.
+  auto finish_tile = [&](int psl, long long pg0) {
+    if (warp == 1) {
+      if (ties)
+        write_near_ties(psl, pg0, tile_near_ties<N, W>(lane, sec_key, a.tie_tol, window_peak,
+                                                       [&](int ww) { return nbrow + (ww * 3 + 1) * L::NBP; }));
+      __syncwarp();
+      if (lane < W) sec_key[lane] = kKeyNegInf;  // for the tile that follows
+    }
+    if (warp == 3 && lane < W && pg0 + lane < total) finish(psl, lane, window_peak(lane));
+  };
 
-  int sl = 0;
-  for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, sl = sl == 2 ? 0 : sl + 1) {
+  int sl = 0, tile = blockIdx.x;
+  bool stopped = false;
+  for (; tile < n_tiles; tile += gridDim.x, sl = sl == 2 ? 0 : sl + 1) {
     const int sl1 = sl == 2 ? 0 : sl + 1, sl2 = sl1 == 2 ? 0 : sl1 + 1;
     const long long g0 = (long long)tile * W;
-    // No barrier here: warps 0 and 1 may still be finishing the previous
-    // tile's near-tie test and fits while the others stage this tile (its
-    // rows are the ones each thread copied itself). The stage-1 barrier
-    // below waits for all of them.
+    // No barrier here: each thread stages the rows that it copied itself, and
+    // the stage-1 barrier below orders this tile's product after every warp's
+    // reads of the previous tile's map.
     if (ASYNC) cp_async_wait_all();
-    cur_sl = sl;
-    cur_g0 = g0;
 
     // ---- Staging: thread (half, t = (w, y)) takes row y of window w of its
     // frames (both with one thread per TMEM lane: their reduction chains run
@@ -645,7 +702,10 @@ __global__ void __launch_bounds__(TcLayout<SS, SPLIT>::NT, TcLayout<SS, SPLIT>::
           st8s<SPLIT>(sm + L::OP + f * L::A1_BYTES, L::NOP, off_k(t, x, SS), r[fi] + x);
       }
     }
-    if (!sync_for_mma()) break;
+    if (!sync_for_mma()) {
+      stopped = true;
+      break;
+    }
 
     // ---- Stage 1: T = a F^T per frame -> TMEM cols [f N, f N + N).
     if (warp == 0) {  // MMA issue: a converged warp, one elected lane issues
@@ -656,8 +716,14 @@ __global__ void __launch_bounds__(TcLayout<SS, SPLIT>::NT, TcLayout<SS, SPLIT>::
                          L::NB1, 256, 128, SS * 16, SS / 16, id, false);
       tc::mma_commit<true>(&bar);
     }
-    // The near-tie keys of this tile (the previous tile's test is done).
-    if (tid < W) sec_key[tid] = kKeyNegInf;
+    // While the product runs: the previous tile's test and fits (slot sl2), and
+    // the corners of the next tile but for the first (its integer divisions in
+    // warp 2); slot sl1 was last read by the fits of the tile before that.
+    if (tile != (int)blockIdx.x) {
+      finish_tile(sl2, g0 - (long long)gridDim.x * W);
+      if (warp == 2 && lane < W) window_setup(tile + gridDim.x, sl1, lane);
+      __syncwarp();  // the TMEM loads below want whole warps
+    }
     wait_mma();
 
     // ---- Stage 1 -> 2: row (w, y) of T becomes column y of the MN-major rows
@@ -696,7 +762,10 @@ __global__ void __launch_bounds__(TcLayout<SS, SPLIT>::NT, TcLayout<SS, SPLIT>::
         }
       }
     }
-    if (!sync_for_mma()) break;
+    if (!sync_for_mma()) {
+      stopped = true;
+      break;
+    }
 
     // ---- Stage 2: X = T^T F^T for tiles e, o and frames a, b -> TMEM cols [rt 2N + f N, +N).
     if (warp == 0) {  // MMA issue: a converged warp, one elected lane issues
@@ -711,9 +780,8 @@ __global__ void __launch_bounds__(TcLayout<SS, SPLIT>::NT, TcLayout<SS, SPLIT>::
     }
     // The next tile's rows land while this tile runs (issued after the MMAs,
     // so that the issuing thread's copies do not hold up the product). Not
-    // before this tile's stage-1 barrier: warp 2 writes slot sl1's corners
-    // during the previous tile's fits, and that barrier is what orders them
-    // before these reads.
+    // before this tile's stage-2 barrier: warp 2 writes slot sl1's corners
+    // during stage 1, and that barrier orders them before these reads.
     if (ASYNC) {
       stage_async(sl1);
       cp_async_commit();
@@ -757,7 +825,10 @@ __global__ void __launch_bounds__(TcLayout<SS, SPLIT>::NT, TcLayout<SS, SPLIT>::
         st8s<SPLIT>(dst, L::NOP, off_k(t, 3 * HN + g0, 2 * N), rm);
       }
     }
-    if (!sync_for_mma()) break;
+    if (!sync_for_mma()) {
+      stopped = true;
+      break;
+    }
 
     // ---- Stage 3: Re U = [Re P | Im M] [C; -S] -> TMEM cols [0, N),
     // Im U = [Im P | Re M] [C; S] -> cols [N, 2N).
@@ -797,7 +868,10 @@ __global__ void __launch_bounds__(TcLayout<SS, SPLIT>::NT, TcLayout<SS, SPLIT>::
         }
       }
     }
-    if (!sync_for_mma()) break;
+    if (!sync_for_mma()) {
+      stopped = true;
+      break;
+    }
 
     // ---- Stage 4: c = U E' / N -> TMEM cols [rt N, rt N + N).
     if (warp == 0) {  // MMA issue: a converged warp, one elected lane issues
@@ -813,44 +887,10 @@ __global__ void __launch_bounds__(TcLayout<SS, SPLIT>::NT, TcLayout<SS, SPLIT>::
     // ---- Epilogue. Row rt*128 + tid of the tile is map row r of window w
     // (scaled by 2^(e_a + e_b)); shifted row index i = r ^ N/2, shifted
     // column j = s ^ N/2. Lags without window overlap (i = 0 or j = 0) are 0.
-    float* nbrow = reinterpret_cast<float*>(sm + L::NBR);  // [W][3][NBP]: rows pi-1, pi, pi+1 (natural columns)
-    // Subpixel fit and outputs of window ww with flat peak index pidx (its
-    // neighbour rows in nbrow).
-    auto finish = [&](int ww, int pidx) {
-      const int pi_ = pidx / N, pj = pidx % N;
-      float isp = (float)pi_, jsp = (float)pj;
-      if (pi_ > 0 && pi_ < N - 1 && pj > 0 && pj < N - 1) {
-        const int ue = -sc_e[sl][0][ww] - sc_e[sl][1][ww];
-        // Shifted (i, j) -> stored row slot i - pi + 1, natural column j ^ N/2.
-        // x 2^ue as two exact power-of-two products (|ue| <= 240; each factor is a normal float).
-        const float s1 = pow2i(ue >> 1), s2 = pow2i(ue - (ue >> 1));
-        auto at = [&](int i, int j) -> float {
-          return (i == 0 || j == 0) ? 0.f : nbrow[(ww * 3 + (i - pi_ + 1)) * L::NBP + (j ^ HN)] * s1 * s2;
-        };
-        subpixel_fit(a.subpixel, pi_, pj, at(pi_, pj), at(pi_ - 1, pj), at(pi_ + 1, pj), at(pi_, pj - 1),
-                     at(pi_, pj + 1), isp, jsp);
-      }
-      const CorrSeg& sq = seg_s[win_seg[sl][ww]];
-      const long long gl = win_loc[sl][ww];
-      float* uo = reinterpret_cast<float*>(sq.u);
-      float* vo = reinterpret_cast<float*>(sq.v);
-      if (!in_bounds(gl >= 0 && gl < (long long)sq.n_pairs * sq.m * sq.n)) return;
-      if (win_valid[sl][ww]) {
-        uo[gl] = sub_rn(jsp, (float)HN);
-        vo[gl] = sub_rn(isp, (float)HN);
-      } else {
-        uo[gl] = NAN;
-        vo[gl] = NAN;
-      }
-      if (sq.peak_i) sq.peak_i[gl] = pi_;
-      if (sq.peak_j) sq.peak_j[gl] = pj;
-    };
-    auto peak_row = [&](int ww) { return nbrow + (ww * 3 + 1) * L::NBP; };
-    bool stop = false;
     if constexpr (N == 32 && TPL == 1) {
       // One window per warp and row tile (N = 32 rows): the warp finds its
       // window's peak by shuffles and the lanes of the rows next to it store
-      // them at once (no second TMEM pass); then one barrier, and W lanes fit.
+      // them at once (no second TMEM pass).
 #pragma unroll
       for (int rt = 0; rt < 2; ++rt) {
         const int m = rt * 128 + t, w = m / N, r = m % N, i = r ^ HN;
@@ -890,16 +930,6 @@ __global__ void __launch_bounds__(TcLayout<SS, SPLIT>::NT, TcLayout<SS, SPLIT>::
         }
         if (lane == 0) pk_idx[w][0] = idx;
       }
-      // The peaks and neighbour rows are in shared memory (the map's TMEM
-      // columns are read); the abort decision is the same for every thread.
-      tc::fence_before_sync();
-      stop = __syncthreads_or(abort_s != 0);
-      // The near-tie flags in warp 1 while warp 0 fits.
-      if (ties && warp == 1)
-        write_near_ties(tile_near_ties<N, W>(lane, sec_key, a.tie_tol, [&](int ww) { return pk_idx[ww][0]; },
-                                             peak_row));
-      if (tid < W && g0 + tid < total) finish(tid, pk_idx[tid][0]);
-      if (warp == 2 && lane < W) window_setup(tile + 2 * gridDim.x, sl2, lane);
     } else {
       float rbest[2 / TPL];  // this thread's row maxima
 #pragma unroll
@@ -934,19 +964,6 @@ __global__ void __launch_bounds__(TcLayout<SS, SPLIT>::NT, TcLayout<SS, SPLIT>::
         }
       }
       __syncthreads();
-      // First maximum of window w over its NPART warp partials (each thread
-      // that needs it combines them itself: no further barrier).
-      auto window_peak = [&](int w) -> int {
-        float v = pk_val[w][0];
-        int idx = pk_idx[w][0];
-#pragma unroll
-        for (int p = 1; p < NPART; ++p)
-          if (pk_val[w][p] > v || (pk_val[w][p] == v && pk_idx[w][p] < idx)) {
-            v = pk_val[w][p];
-            idx = pk_idx[w][p];
-          }
-        return idx;
-      };
       // The rows next to the peak go to shared memory for the five-point fit.
 #pragma unroll
       for (int ri = 0; ri < 2 / TPL; ++ri) {
@@ -975,26 +992,16 @@ __global__ void __launch_bounds__(TcLayout<SS, SPLIT>::NT, TcLayout<SS, SPLIT>::
           }
         }
       }
-      // The peaks and neighbour rows are in shared memory (the map's TMEM
-      // columns are read); the abort decision is the same for every thread.
-      tc::fence_before_sync();
-      stop = __syncthreads_or(abort_s != 0);
-      // The near-tie flags in warp 1 while warp 0 fits.
-      if (ties && warp == 1) write_near_ties(tile_near_ties<N, W>(lane, sec_key, a.tie_tol, window_peak, peak_row));
-      if (tid < W && g0 + tid < total) finish(tid, window_peak(tid));
-      if (warp == 2 && lane < W) window_setup(tile + 2 * gridDim.x, sl2, lane);
     }
-    // No barrier: the other warps go on to stage the next tile while warps 0
-    // and 1 finish this one and warp 2 sets up the corners of the tile after
-    // the next (slot sl2, last read by the previous tile) with its integer
-    // divisions off the path of the MMAs; the next tile's stage-1 barrier
-    // waits for all of them.
-    if (stop) break;
+    // No barrier: the next tile's stage-1 barrier waits for every warp's peaks,
+    // neighbour rows and TMEM reads.
   }
   if (ASYNC) cp_async_wait_all();
   tc::fence_before_sync();
-  __syncthreads();
+  stopped = __syncthreads_or(stopped || abort_s != 0);
   if (warp == 0) tc::tmem_free(tmem, L::TCOLS);
+  // The last tile (slot before sl).
+  if (!stopped && tile != (int)blockIdx.x) finish_tile(sl == 0 ? 2 : sl - 1, (long long)(tile - (int)gridDim.x) * W);
 }
 
 // ---------------------------------------------------------------------------
