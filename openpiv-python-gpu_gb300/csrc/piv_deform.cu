@@ -551,9 +551,13 @@ static_assert(kPfR % 8 == 0, "the recursions run in chunks of eight");
 // rows fall on distinct banks for eight consecutive rows (92 = 28 mod 32), and
 // consecutive columns on consecutive banks.
 static constexpr int kPfS = kPfR + 4;
+// Row pitch in bytes of 8-bit regions: 16-byte rows on distinct banks for eight
+// consecutive rows (28 words).
+static constexpr int kPfB = 112;
 static constexpr int kPfL = kPfT / 2 + 2 * kPfK;   // samples of a half line's recursions (56)
 static constexpr int kPfNT = 2 * kPfR + 16;        // threads: two per region row, in whole warps
 static_assert(kPfNT % 32 == 0 && kPfL % 4 == 0, "prefilter launch shape");
+static_assert(kPfR - kPfL + (kPfL + 15) / 16 * 16 <= kPfB, "byte rows hold the last chunk");
 static constexpr float kPole = -0.26794919243112270f;  // sqrt(3) - 2
 
 // Mirror ('d c b | a b c d | c b a') index for any integer q.
@@ -587,14 +591,21 @@ template <typename P>
 __global__ void __launch_bounds__(kPfNT) k_prefilter(int H, int W, const P* __restrict__ in, float* __restrict__ out,
                                                      int pad) {
   __shared__ __align__(16) float reg[kPfR * kPfS];
+  __shared__ int row_s[kPfR];
   const int x0 = blockIdx.x * kPfT, y0 = blockIdx.y * kPfT;
   const long long fbase = (long long)blockIdx.z * H * W;
   const P* src = in + fbase;
   const int t = threadIdx.x;
   const bool interior = x0 >= kPfK && y0 >= kPfK && x0 + kPfT + kPfK <= W && y0 + kPfT + kPfK <= H;
-  if (sizeof(P) == 1 && interior && (W & 3) == 0 && ((uintptr_t)in & 3) == 0) {
+  // 8-bit regions stay bytes until the recursions along x have read them: a
+  // quarter of the shared-memory traffic of those two passes, which bounds the
+  // kernel (64 frames of 1024 x 1024: 107 us as floats, 100 us as bytes; 83%
+  // of the L1 wavefront rate before).
+  constexpr bool kBytes = sizeof(P) == 1;
+  uint8_t* raw = reinterpret_cast<uint8_t*>(reg);
+  if (kBytes && interior && (W & 3) == 0 && ((uintptr_t)in & 3) == 0) {
     // 8-bit frames away from the edges: the region's rows start on 4-byte
-    // boundaries (x0 - 12 is a multiple of 4). Thread t < 176 converts word
+    // boundaries (x0 - 12 is a multiple of 4). Thread t < 176 copies word
     // column t % 22 of region rows t / 22, t / 22 + 8, ...: its addresses
     // advance by a fixed stride, all of its loads in flight together.
     constexpr int kWords = kPfR / 4, kGroups = kPfNT / kWords, kIters = (kPfR + kGroups - 1) / kGroups;
@@ -603,30 +614,43 @@ __global__ void __launch_bounds__(kPfNT) k_prefilter(int H, int W, const P* __re
       const long long wstep = (long long)kGroups * (W / 4);
       const uint32_t* wsrc =
           reinterpret_cast<const uint32_t*>(src + (long long)(y0 - kPfK + r0) * W + (x0 - kPfK)) + wc;
-      float* dst = reg + r0 * kPfS + 4 * wc;
+      uint32_t* dst = reinterpret_cast<uint32_t*>(raw + r0 * kPfB) + wc;
       uint32_t wv[kIters];
 #pragma unroll
       for (int k = 0; k < kIters; ++k) wv[k] = r0 + kGroups * k < kPfR ? __ldg(wsrc + k * wstep) : 0u;
 #pragma unroll
       for (int k = 0; k < kIters; ++k)
-        if (r0 + kGroups * k < kPfR) {
-          const uint32_t w = wv[k];
-          *reinterpret_cast<float4*>(dst + k * kGroups * kPfS) =
-              make_float4(u8_to_float(w, 0), u8_to_float(w, 1), u8_to_float(w, 2), u8_to_float(w, 3));
-        }
+        if (r0 + kGroups * k < kPfR) dst[k * kGroups * (kPfB / 4)] = wv[k];
     }
-  } else if (t < 2 * kPfR) {
-    // Any pixel type, mirrored edges: thread t holds region column t % 88 (its
-    // mirrored frame column found once) and walks half of the region's rows.
-    const int rc = t % kPfR, r0 = (t / kPfR) * (kPfR / 2);
-    int gx = x0 - kPfK + rc;
-    if (gx < 0 || gx >= W) gx = mirror_any(gx, W);
-    const P* col = src + gx;
-#pragma unroll 4
-    for (int r = r0; r < r0 + kPfR / 2; ++r) {
-      int gy = y0 - kPfK + r;
-      if (gy < 0 || gy >= H) gy = mirror_any(gy, H);
-      reg[r * kPfS + rc] = pixel_to_float<P>(__ldg(col + (long long)gy * W));
+  } else {
+    // Any pixel type, mirrored edges: thread t holds region column t % 88 and
+    // walks half of the region's rows, their mirrored frame rows found once
+    // per CTA, in two batches whose loads are all in flight together. Four rows
+    // at a time, each with the mirror rule, 64 frames of 1037 x 1021 took 278
+    // us for 8-bit pixels (now 132 us), of 1024 x 1024 301 us for float32 (now
+    // 151 us), and the edge tiles held up the others (8-bit 140 -> 107 us).
+    if (t < kPfR) {
+      const int gy = y0 - kPfK + t;
+      row_s[t] = gy < 0 || gy >= H ? mirror_any(gy, H) : gy;
+    }
+    __syncthreads();
+    if (t < 2 * kPfR) {
+      constexpr int kBatch = kPfR / 4;
+      const int rc = t % kPfR, r0 = (t / kPfR) * (kPfR / 2);
+      int gx = x0 - kPfK + rc;
+      if (gx < 0 || gx >= W) gx = mirror_any(gx, W);
+      const P* col = src + gx;
+#pragma unroll 1
+      for (int r = r0; r < r0 + kPfR / 2; r += kBatch) {
+        P px[kBatch];
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) px[k] = __ldg(col + (long long)row_s[r + k] * W);
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+          if constexpr (kBytes) raw[(r + k) * kPfB + rc] = px[k];
+          else reg[(r + k) * kPfS + rc] = pixel_to_float<P>(px[k]);
+        }
+      }
     }
   }
   __syncthreads();
@@ -635,11 +659,23 @@ __global__ void __launch_bounds__(kPfNT) k_prefilter(int H, int W, const P* __re
   float v[kPfL];
   const int xr = t % kPfR, xs = (t / kPfR) * (kPfR - kPfL);
   if (t < 2 * kPfR) {
-    const float4* rp = reinterpret_cast<const float4*>(reg + xr * kPfS + xs);
+    if constexpr (kBytes) {
+      const uint4* rp = reinterpret_cast<const uint4*>(raw + xr * kPfB + xs);
 #pragma unroll
-    for (int q = 0; q < kPfL / 4; ++q) {
-      const float4 u = rp[q];
-      v[4 * q] = u.x; v[4 * q + 1] = u.y; v[4 * q + 2] = u.z; v[4 * q + 3] = u.w;
+      for (int q = 0; q < (kPfL + 15) / 16; ++q) {
+        const uint4 u = rp[q];
+        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int k = 0; k < 16; ++k)
+          if (16 * q + k < kPfL) v[16 * q + k] = u8_to_float(w[k / 4], k % 4);
+      }
+    } else {
+      const float4* rp = reinterpret_cast<const float4*>(reg + xr * kPfS + xs);
+#pragma unroll
+      for (int q = 0; q < kPfL / 4; ++q) {
+        const float4 u = rp[q];
+        v[4 * q] = u.x; v[4 * q + 1] = u.y; v[4 * q + 2] = u.z; v[4 * q + 3] = u.w;
+      }
     }
     half_line(v);
   }
@@ -659,13 +695,15 @@ __global__ void __launch_bounds__(kPfNT) k_prefilter(int H, int W, const P* __re
     for (int k = 0; k < kPfL; ++k) v[k] = reg[(ys + k) * kPfS + col];
     half_line(v);
     const int gx = x0 + tc, os = W + 2 * pad;
-    if (gx < W) {
-      float* dst = out + (long long)blockIdx.z * (H + 2 * pad) * os + (long long)pad * os + pad + gx;
+    const int rows = H - (y0 + ys);  // of the half column inside the frame
+    float* dst = out + ((long long)blockIdx.z * (H + 2 * pad) + pad + y0 + ys) * os + pad + gx;
+    if (gx < W && rows >= kPfT / 2) {
 #pragma unroll
-      for (int k = kPfK; k < kPfK + kPfT / 2; ++k) {
-        const int gy = y0 + ys + k - kPfK;
-        if (gy < H) dst[(long long)gy * os] = 36.0f * v[k];
-      }
+      for (int k = 0; k < kPfT / 2; ++k) dst[(long long)k * os] = 36.0f * v[kPfK + k];
+    } else if (gx < W) {
+#pragma unroll
+      for (int k = 0; k < kPfT / 2; ++k)
+        if (k < rows) dst[(long long)k * os] = 36.0f * v[kPfK + k];
     }
   }
 }
