@@ -267,9 +267,15 @@ PIV_D AxisWeight axis_weight(int q, int ss, int off, int sp, int len) {
 
 static constexpr int kDeformThreads = 256;
 static constexpr int kDeformRows = 8;                       // image rows per CTA
-// Field columns / rows one CTA can touch (spacing >= 1).
-static constexpr int kDeformMaxCols = kDeformThreads + 2;
-static constexpr int kDeformMaxGridRows = kDeformRows + 1;
+// Shared memory for the field points that one CTA can touch, u and v: the
+// intervals of its first and last pixel are at most (pixels - 1) / spacing + 1
+// apart, and the last one has a point behind it. Sized by the spacing, not for
+// spacing 1 (18.6 KB a CTA): what is left over caches the taps (64 pairs of
+// 1024 x 1024, two passes of k_deform_cubic: 1081 -> 1054 us).
+static size_t deform_smem(int spacing) {
+  const size_t cols = (kDeformThreads - 1) / spacing + 3, rows = (kDeformRows - 1) / spacing + 3;
+  return 2 * cols * rows * sizeof(float);
+}
 
 // One thread per pixel column of an 8-row x 256-pixel block; each thread
 // handles the block's eight rows. The predictor (float32; the reference
@@ -281,7 +287,7 @@ static constexpr int kDeformMaxGridRows = kDeformRows + 1;
 template <typename T>
 __global__ void __launch_bounds__(kDeformThreads) k_deform(DeformArgs a, AxisMap ax, AxisMap ay, T dta, T dtb,
                                                            int do_a, int do_b) {
-  __shared__ float su[kDeformMaxGridRows][kDeformMaxCols], sv[kDeformMaxGridRows][kDeformMaxCols];
+  extern __shared__ float field_s[];  // u, then v: [nr][nc]
   __shared__ int s_klo, s_khi;
   const piv_geometry& g = a.geom;
   const int H = g.height, W = g.width;
@@ -297,12 +303,14 @@ __global__ void __launch_bounds__(kDeformThreads) k_deform(DeformArgs a, AxisMap
   __syncthreads();
   const int k_lo = s_klo, k_hi = s_khi;
   const int nc = k_hi - k_lo + 1, nr = r_hi - r_lo + 1;
+  float* su = field_s;
+  float* sv = field_s + nr * nc;
   const long long fo = (long long)pair * g.m * g.n;
   for (int e = threadIdx.x; e < nr * nc; e += kDeformThreads) {
     const int r = e / nc, c = e % nc;
     const long long q = fo + (long long)(r_lo + r) * g.n + k_lo + c;
-    su[r][c] = (float)__ldg(a.up + q);
-    sv[r][c] = (float)__ldg(a.vp + q);
+    su[e] = (float)__ldg(a.up + q);
+    sv[e] = (float)__ldg(a.vp + q);
   }
   __syncthreads();
   if (j >= W) return;
@@ -327,11 +335,11 @@ __global__ void __launch_bounds__(kDeformThreads) k_deform(DeformArgs a, AxisMap
       continue;
     }
     const AxisWeight wy = axis_weight(i, ay);
-    const int y0r = wy.i - r_lo, y1r = (g.m < 2 ? wy.i : wy.i + 1) - r_lo;
-    const float u0 = fmaf(wy.t, su[y1r][c0] - su[y0r][c0], su[y0r][c0]);
-    const float u1 = fmaf(wy.t, su[y1r][c1] - su[y0r][c1], su[y0r][c1]);
-    const float v0 = fmaf(wy.t, sv[y1r][c0] - sv[y0r][c0], sv[y0r][c0]);
-    const float v1 = fmaf(wy.t, sv[y1r][c1] - sv[y0r][c1], sv[y0r][c1]);
+    const int y0r = (wy.i - r_lo) * nc, y1r = ((g.m < 2 ? wy.i : wy.i + 1) - r_lo) * nc;
+    const float u0 = fmaf(wy.t, su[y1r + c0] - su[y0r + c0], su[y0r + c0]);
+    const float u1 = fmaf(wy.t, su[y1r + c1] - su[y0r + c1], su[y0r + c1]);
+    const float v0 = fmaf(wy.t, sv[y1r + c0] - sv[y0r + c0], sv[y0r + c0]);
+    const float v1 = fmaf(wy.t, sv[y1r + c1] - sv[y0r + c1], sv[y0r + c1]);
     const T up = (T)fmaf(wx.t, u1 - u0, u0);
     const T vp = (T)fmaf(wx.t, v1 - v0, v0);
     const T y = (T)i;
@@ -422,7 +430,7 @@ PIV_D float sample_cubic32p(const float* __restrict__ coef, int S, int W, int H,
 template <bool PADDED>
 __global__ void __launch_bounds__(kDeformThreads) k_deform_cubic(DeformArgs a, AxisMap ax, AxisMap ay, float dta,
                                                                  float dtb) {
-  __shared__ float su[kDeformMaxGridRows][kDeformMaxCols], sv[kDeformMaxGridRows][kDeformMaxCols];
+  extern __shared__ float field_s[];  // u, then v: [nr][nc]
   __shared__ int s_klo, s_khi;
   __shared__ int s_y0[kDeformRows], s_y1[kDeformRows];
   __shared__ float s_ty[kDeformRows];
@@ -437,21 +445,23 @@ __global__ void __launch_bounds__(kDeformThreads) k_deform_cubic(DeformArgs a, A
   const AxisWeight wx = axis_weight(min(j, W - 1), ax);
   if (threadIdx.x == 0) s_klo = axis_weight(j0, ax).i;
   if (threadIdx.x == kDeformThreads - 1 || j == W - 1) s_khi = min(wx.i + 1, g.n - 1);
-  if (threadIdx.x < kDeformRows) {
-    const AxisWeight wy = axis_weight(min(i0 + (int)threadIdx.x, H - 1), ay);
-    s_y0[threadIdx.x] = wy.i - r_lo;
-    s_y1[threadIdx.x] = (g.m < 2 ? wy.i : wy.i + 1) - r_lo;
-    s_ty[threadIdx.x] = wy.t;
-  }
   __syncthreads();
   const int k_lo = s_klo, k_hi = s_khi;
   const int nc = k_hi - k_lo + 1, nr = r_hi - r_lo + 1;
+  if (threadIdx.x < kDeformRows) {
+    const AxisWeight wy = axis_weight(min(i0 + (int)threadIdx.x, H - 1), ay);
+    s_y0[threadIdx.x] = (wy.i - r_lo) * nc;
+    s_y1[threadIdx.x] = ((g.m < 2 ? wy.i : wy.i + 1) - r_lo) * nc;
+    s_ty[threadIdx.x] = wy.t;
+  }
+  float* su = field_s;
+  float* sv = field_s + nr * nc;
   const long long fo = (long long)pair * g.m * g.n;
   for (int e = threadIdx.x; e < nr * nc; e += kDeformThreads) {
     const int r = e / nc, c = e % nc;
     const long long q = fo + (long long)(r_lo + r) * g.n + k_lo + c;
-    su[r][c] = (float)__ldg(a.up + q);
-    sv[r][c] = (float)__ldg(a.vp + q);
+    su[e] = (float)__ldg(a.up + q);
+    sv[e] = (float)__ldg(a.vp + q);
   }
   __syncthreads();
   if (j >= W) return;
@@ -480,10 +490,10 @@ __global__ void __launch_bounds__(kDeformThreads) k_deform_cubic(DeformArgs a, A
     }
     const int y0r = s_y0[rr], y1r = s_y1[rr];
     const float ty = s_ty[rr];
-    const float u0 = fmaf(ty, su[y1r][c0] - su[y0r][c0], su[y0r][c0]);
-    const float u1 = fmaf(ty, su[y1r][c1] - su[y0r][c1], su[y0r][c1]);
-    const float v0 = fmaf(ty, sv[y1r][c0] - sv[y0r][c0], sv[y0r][c0]);
-    const float v1 = fmaf(ty, sv[y1r][c1] - sv[y0r][c1], sv[y0r][c1]);
+    const float u0 = fmaf(ty, su[y1r + c0] - su[y0r + c0], su[y0r + c0]);
+    const float u1 = fmaf(ty, su[y1r + c1] - su[y0r + c1], su[y0r + c1]);
+    const float v0 = fmaf(ty, sv[y1r + c0] - sv[y0r + c0], sv[y0r + c0]);
+    const float v1 = fmaf(ty, sv[y1r + c1] - sv[y0r + c1], sv[y0r + c1]);
     const float up = fmaf(wx.t, u1 - u0, u0);
     const float vp = fmaf(wx.t, v1 - v0, v0);
     const float y = (float)i;
@@ -516,14 +526,15 @@ int deform(const DeformArgs& a, cudaStream_t stream) {
     return set_error(PIV_E_UNSUPPORTED, "deformation: frames above 2^31 pixels");
   const AxisMap ax = axis_map(a.geom.search_size, a.geom.x_offset, a.geom.spacing, a.geom.n);
   const AxisMap ay = axis_map(a.geom.search_size, a.geom.y_offset, a.geom.spacing, a.geom.m);
+  const size_t smem = deform_smem(a.geom.spacing);
   if (a.dtype == PIV_DTYPE_F64)
-    k_deform<double><<<grid, kDeformThreads, 0, stream>>>(a, ax, ay, dta, dtb, do_a, do_b);
+    k_deform<double><<<grid, kDeformThreads, smem, stream>>>(a, ax, ay, dta, dtb, do_a, do_b);
   else if (a.order == 3 && do_a && do_b && a.coef_pad)
-    k_deform_cubic<true><<<grid, kDeformThreads, 0, stream>>>(a, ax, ay, (float)dta, (float)dtb);
+    k_deform_cubic<true><<<grid, kDeformThreads, smem, stream>>>(a, ax, ay, (float)dta, (float)dtb);
   else if (a.order == 3 && do_a && do_b)
-    k_deform_cubic<false><<<grid, kDeformThreads, 0, stream>>>(a, ax, ay, (float)dta, (float)dtb);
+    k_deform_cubic<false><<<grid, kDeformThreads, smem, stream>>>(a, ax, ay, (float)dta, (float)dtb);
   else
-    k_deform<float><<<grid, kDeformThreads, 0, stream>>>(a, ax, ay, (float)dta, (float)dtb, do_a, do_b);
+    k_deform<float><<<grid, kDeformThreads, smem, stream>>>(a, ax, ay, (float)dta, (float)dtb, do_a, do_b);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? PIV_OK : set_cuda_error(e, "k_deform launch");
 }
