@@ -61,7 +61,9 @@ extern "C" {
 #define PIV_SMOOTH_MAX_ITERS 4   /* the weighted iteration reached its last allowed step (100) */
 
 /* Correlation engines. */
-#define PIV_DFT_FFT32 0          /* in-shared-memory FFT in the correlation float type */
+#define PIV_DFT_FFT32 0          /* in-shared-memory FFT in the correlation float type (float64
+                                    passes with n_fft 2, no mask, maps or S2N: a float32 search
+                                    for the peak and direct float64 sums for the fit) */
 #define PIV_DFT_TENSOR 1         /* tcgen05 tensor-core DFT: FP16 operands, FP32 accumulation
                                     (float32 passes with search 16, 32 or 64 px and n_fft 2;
                                     other passes use the FFT) */

@@ -917,7 +917,7 @@ static void gcv_bounds(int m, int n, double* pmin, double* pmax) {
 // depend on c. Sums of two products have their roundings written out (the
 // search stops where its curve is flat: a last bit of a score moves p by
 // 1e-4). Bound by the DCTs' dot products and the barriers between
-// passes: one pair of 63 x 63 around a masked disc takes 0.84 ms with 8 CTAs.
+// passes: one pair of 63 x 63 around a masked disc takes 0.84 to 0.89 ms with 8 CTAs.
 // On one CTA, with strided matrix reads and 10^p formed by every thread, it
 // took 6.4 ms.
 // ---------------------------------------------------------------------------
