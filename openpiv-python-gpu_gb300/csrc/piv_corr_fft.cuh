@@ -278,9 +278,12 @@ struct CorrShared {
 };
 
 // Subpixel fit, displacement, near-tie flags and S2N of the windows in slots
-// g0 .. g0 + WPC - 1, from their maps in buf and their peaks in S.
+// g0 .. g0 + WPC - 1, from their maps in buf and their peaks in S. second (or
+// NULL): the windows' second peaks, already found (then no barrier here, and the
+// first WPC threads alone have work).
 template <class C, int N = C::N, typename T = typename C::T>
-PIV_D void corr_outputs(const CorrArgs& a, const Cplx<T>* buf, const CorrShared<C>& S, long long g0, long long total) {
+PIV_D void corr_outputs(const CorrArgs& a, const Cplx<T>* buf, const CorrShared<C>& S, long long g0, long long total,
+                        const T* second = nullptr) {
   using L = FftLayout<C>;
   constexpr int WPC = L::WPC;
   const int tid = threadIdx.x, ss = a.ss;
@@ -339,7 +342,18 @@ PIV_D void corr_outputs(const CorrArgs& a, const Cplx<T>* buf, const CorrShared<
   }
 
   // Signal-to-noise ratio.
-  if (a.s2n) {
+  auto ratio = [&](int w, T q2) -> T {
+    const T p1 = S.pval[w];
+    T s = 0;
+    if (S.valid[w]) {
+      if (p1 > 0) s = p1 / q2;
+      if (q2 <= 0 && p1 > 0) s = (T)INFINITY;
+    }
+    return s;
+  };
+  if (a.s2n && second) {
+    if (tid < WPC && g0 + tid < total) reinterpret_cast<T*>(a.s2n)[win_of(g0 + tid)] = ratio(tid, second[tid]);
+  } else if (a.s2n) {
     T* p2 = S.win_v + 3 * WPC;  // [WPC]
     if (a.s2n_method == PIV_S2N_PEAK2PEAK) {
       int* peak2 = S.win_i + 4 * WPC;
@@ -365,13 +379,7 @@ PIV_D void corr_outputs(const CorrArgs& a, const Cplx<T>* buf, const CorrShared<
     __syncthreads();
     if (tid < WPC && g0 + tid < total) {
       const long long g = win_of(g0 + tid);
-      const T p1 = S.pval[tid], q2 = p2[tid];
-      T s = 0;
-      if (S.valid[tid]) {
-        if (p1 > 0) s = p1 / q2;
-        if (q2 <= 0 && p1 > 0) s = (T)INFINITY;
-      }
-      reinterpret_cast<T*>(a.s2n)[g] = s;
+      reinterpret_cast<T*>(a.s2n)[g] = ratio(tid, p2[tid]);
     }
   }
 }

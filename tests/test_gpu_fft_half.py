@@ -65,3 +65,20 @@ def test_same_bits_as_the_general_kernel(ss, dtype, shape, extra):
     for x, y in zip(new[2], old[2]):
         for key in ("u_corr", "v_corr", "i_peak", "j_peak", "near_tie", "val0") + (("s2n",) if extra == "s2n" else ()):
             np.testing.assert_array_equal(x[key], y[key], err_msg=key)
+
+
+# The second peak outside a box of half width `size`: boxes that wrap
+# around, one row and column left, and nothing left.
+@pytest.mark.parametrize("ss", [32, 64])
+@pytest.mark.parametrize("size", [1, 7, 31, 32, 63, 64])
+def test_second_peak_is_the_general_kernels(ss, size):
+    from openpiv_gpu.gpu_process import PIVGPU
+
+    a, b = _frames(ss + size, 3 * ss, 4 * ss, "uint8")
+    proc = PIVGPU(a.shape[1:], ss, overlap_ratio=0.5, dtype_f="float32", dft="fft", s2n_tol=1.1, s2n_size=size,
+                  s2n_method="peak2peak")
+    new = _run(proc, a, b, 0)
+    old = _run(proc, a, b, SAME_RADIX[ss])
+    for x, y in zip(new[2], old[2]):
+        for key in ("i_peak", "j_peak", "s2n", "val0"):
+            np.testing.assert_array_equal(x[key], y[key], err_msg=key)
