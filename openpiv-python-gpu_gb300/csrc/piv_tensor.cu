@@ -399,8 +399,8 @@ __global__ void __launch_bounds__(TcLayout<SS, SPLIT>::NT, TcLayout<SS, SPLIT>::
   __shared__ uint64_t bar;
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_s;
-  // Per tile slot (three: the tile being correlated, the next one, whose rows
-  // are in flight, and the one after, whose corners are being computed).
+  // Per tile slot (three: the tile being correlated, the next one, whose corners
+  // and then rows come in meanwhile, and the one before, whose fits are made).
   __shared__ int sc_e[3][2][W];      // per slot, frame and window: log2 of the operand scale
   __shared__ long long win_base[3][W];
   __shared__ int win_valid[3][W];
