@@ -170,19 +170,33 @@ struct Top2 {
 // Search mode (float64 passes, correlate_f64): the float32 map only finds the
 // integer peak. The window means are removed in a way that leaves rounding of
 // the differences alone: whole-number pixels less the nearest whole number of
-// the mean and then its fraction, other pixels in float64. A window is settled
-// when its two largest values are further apart than kSearchTol |a| |b| (the
-// 2-norms of the mean-removed windows); the others go to the list. The float32
-// transform's error in a map value is below 6.7 u log2(N^2) |a| |b| per
-// transform (Higham, Accuracy and Stability of Numerical Algorithms, section
-// 24.1; u = 2^-24), three transforms of N = 128: 1.7e-5 |a| |b|, so a gap of
-// 6.1e-5 |a| |b| is beyond the errors of both values.
+// the mean and then its fraction, other pixels in float64. Both mean-removed
+// windows are then scaled by powers of two to 2-norms in [1, 2) (search_scale):
+// they share one transform z = a + i b, whose rounding follows |z|, so that the
+// spectrum of the smaller window would carry the larger one's error (frames 1e4
+// apart in contrast: map errors above the gap below, wrong peaks settled).
+// A window is settled when its two largest values are further apart than
+// kSearchTol |a| |b|; the others go to the list. With norms within a factor of
+// two, the forward transforms' errors move a map value by at most 3.4 eta |a|
+// |b|, eta = 6.7 u log2(N^2) the transform's norm-wise bound (Higham, Accuracy
+// and Stability of Numerical Algorithms, section 24.1; u = 2^-24): 1.9e-5 |a|
+// |b| for N = 128, under a third of the gap of 6.1e-5 |a| |b|. The inverse's
+// error is bounded by eta |c|_2 only, and the map's norm |c|_2 exceeds |a| |b|
+// for smooth windows, so there the margin is a measured one: 2.7e-7 |a| |b| in
+// all, the largest error of 12,600 noisy, matched and smooth windows of 16 to
+// 64 px with contrasts up to 1e9 apart.
 constexpr float kSearchTol = 1.0f / 16384.0f;
-// Gap that settles a window; infinite where the scale's intermediate values
-// leave the float32 range (nothing is settled then).
-PIV_D float search_gap(float norm_a, float norm_b) {
-  const float scale = sqrtf(norm_a) * sqrtf(norm_b);
-  return scale > 1e-25f && scale < 1e25f ? kSearchTol * scale : INFINITY;
+// The power of two that brings a window of squared 2-norm `norm` to [1, 2).
+PIV_D float search_scale(float norm) {
+  const int e = (__float_as_int(norm) >> 23) - 127;  // floor of log2
+  return __int_as_float((127 - (e >> 1)) << 23);
+}
+// Gap that settles a window of squared norms norm_a and norm_b, scaled by sa
+// and sb; infinite where the sums of squares leave the float32 range (nothing
+// is settled then).
+PIV_D float search_gap(float norm_a, float norm_b, float sa, float sb) {
+  const bool in_range = norm_a > 1e-30f && norm_a < 1e30f && norm_b > 1e-30f && norm_b < 1e30f;
+  return in_range ? kSearchTol * (sqrtf(norm_a) * sa) * (sqrtf(norm_b) * sb) : INFINITY;
 }
 // The open window g: a record of its candidates (values within `gap` of the
 // largest; count may exceed kCandMax), or its place in the window list.
@@ -373,6 +387,15 @@ __global__ void __launch_bounds__(H::NT, H::MIN_CTAS) k_corr_fft_half(CorrArgs a
       }
     }
     __syncthreads();
+    // Search: the windows' scales, applied as the rows are read, and the gap.
+    float scale_a = 1.f, scale_b = 1.f, gap = 0.f;
+    if constexpr (SEARCH) {
+      na = warp_sum(lane < NW ? norm_part[0][lane] : 0.f);
+      nb = warp_sum(lane < NW ? norm_part[1][lane] : 0.f);
+      scale_a = search_scale(na);
+      scale_b = search_scale(nb);
+      gap = search_gap(na, nb, scale_a, scale_b);
+    }
 
     // Rows of the window: R2-point DFTs, then eight-point ones. Lanes take
     // adjacent rows (bank-conflict free), the in-line index is the warp's.
@@ -382,7 +405,10 @@ __global__ void __launch_bounds__(H::NT, H::MIN_CTAS) k_corr_fft_half(CorrArgs a
       Cplx<float>* p = buf + (PAD + l) * LD + n1;
       Cplx<float> x[R2];
 #pragma unroll
-      for (int k = R2 / 4; k < 3 * R2 / 4; ++k) x[k] = p[k * R1];
+      for (int k = R2 / 4; k < 3 * R2 / 4; ++k) {
+        x[k] = p[k * R1];
+        if (SEARCH) x[k] = cmake<float>(x[k].x * scale_a, x[k].y * scale_b);
+      }
       dft_half<R2>(x);
       if (n1 != 0) {
 #pragma unroll
@@ -583,12 +609,7 @@ __global__ void __launch_bounds__(H::NT, H::MIN_CTAS) k_corr_fft_half(CorrArgs a
     }
     if constexpr (SEARCH) {
       if (tid == 0) {
-        float ta = 0.f, tb = 0.f;
-        for (int w = 0; w < NW; ++w) {
-          ta += norm_part[0][w];
-          tb += norm_part[1][w];
-        }
-        const float gap = search_gap(ta, tb), best = S.pval[0];
+        const float best = S.pval[0];
         a.peak_i[g] = S.pi[0];
         a.peak_j[g] = S.pj[0];
         if (a.near_tie) a.near_tie[g] = 0;
@@ -709,25 +730,39 @@ __global__ void __launch_bounds__(32 * kWarpFftWarps, kWarpFftCtas) k_corr_fft_w
       fa = (float)(da - rint(da));
       fb = (float)(db - rint(db));
     }
-    float na = 0.f, nb = 0.f;  // search: sums of squares
+    float va[8], vb[8], na = 0.f, nb = 0.f;  // search: sums of squares
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if constexpr (sizeof(X) == 8) {
+        va[k] = (float)(xa[k] - da);
+        vb[k] = (float)(xb[k] - db);
+      } else {
+        va[k] = less_mean<SEARCH>(xa[k], ma, fa);
+        vb[k] = less_mean<SEARCH>(xb[k], mb, fb);
+      }
+      if (!ok) va[k] = vb[k] = 0.f;
+      if (SEARCH) {
+        na = fmaf(va[k], va[k], na);
+        nb = fmaf(vb[k], vb[k], nb);
+      }
+    }
+    float scale_a = 1.f, scale_b = 1.f, gap = 0.f;
+    if constexpr (SEARCH) {
+      na = warp_sum(na);
+      nb = warp_sum(nb);
+      scale_a = search_scale(na);
+      scale_b = search_scale(nb);
+      gap = search_gap(na, nb, scale_a, scale_b);
+    }
     __syncwarp();  // the previous window's map has been read
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       const int e = lane + 32 * k, r = e / SS, c = e % SS;
-      float va, vb;
-      if constexpr (sizeof(X) == 8) {
-        va = (float)(xa[k] - da);
-        vb = (float)(xb[k] - db);
-      } else {
-        va = less_mean<SEARCH>(xa[k], ma, fa);
-        vb = less_mean<SEARCH>(xb[k], mb, fb);
-      }
-      if (!ok) va = vb = 0.f;
       if (SEARCH) {
-        na = fmaf(va, va, na);
-        nb = fmaf(vb, vb, nb);
+        va[k] *= scale_a;
+        vb[k] *= scale_b;
       }
-      buf[(PAD + r) * LD + PAD + c] = cmake<float>(va, vb);
+      buf[(PAD + r) * LD + PAD + c] = cmake<float>(va[k], vb[k]);
     }
     __syncwarp();
     Cplx<float> x[N];
@@ -801,7 +836,6 @@ __global__ void __launch_bounds__(32 * kWarpFftWarps, kWarpFftCtas) k_corr_fft_w
       }
     }
     if constexpr (SEARCH) {
-      const float gap = search_gap(warp_sum(na), warp_sum(nb));
       if (lane == 0) {
         a.peak_i[g] = top.at / N;
         a.peak_j[g] = top.at % N;
