@@ -211,7 +211,9 @@ PIV_D unsigned cluster_rank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
-// Barrier of every thread of the cluster; orders shared and global memory.
+// Barrier of every thread of the cluster; orders shared and global memory. A
+// kernel passes one before its first st_cluster: until then a CTA of the
+// cluster may not have started, and its shared memory is not there to write.
 PIV_D void cluster_barrier(int c) {
   if (c == 1) {
     __syncthreads();
@@ -730,7 +732,7 @@ k_gcv(int m, int n, int c, double rmn, const double* __restrict__ fd, double* __
   // again in float64 and the first minimum among them is kept (np.argmin).
   auto scan_point = [&](int k) { return fma((double)k * (1.0 / 9.0), pmax - pmin, pmin); };
   if (threadIdx.x < 10) sh_s[threadIdx.x] = pow(10.0, scan_point(threadIdx.x));
-  __syncthreads();
+  cluster_barrier(c);  // sh_s is complete, and every CTA of the cluster runs
   {
     // Points SETS k + set: sums of the residuals in acc[k], of 1 - gamma in
     // acc[PER + k].
@@ -1177,6 +1179,7 @@ k_smoothn_weighted(int m, int n, int c, const double* u_in, const double* v_in, 
     nf += fin ? 1.0 : 0.0;
     ws += wv;
   }
+  cluster_barrier(c);  // every CTA of the cluster runs
   sw_sums(x, nf, ws);
   nf = sh.sums[0];
   ws = sh.sums[1];
