@@ -271,6 +271,15 @@ static int plan_alloc_t(piv_plan* p, Ptr** ptr, size_t count) {
   return rc;
 }
 
+// A stream for a plan's set-up, which waits for no other stream and goes ahead
+// of queued work of lower priority.
+static int setup_stream(cudaStream_t* stream) {
+  int least = 0, greatest = 0;
+  cudaDeviceGetStreamPriorityRange(&least, &greatest);
+  const cudaError_t e = cudaStreamCreateWithPriority(stream, cudaStreamNonBlocking, greatest);
+  return e == cudaSuccess ? PIV_OK : set_cuda_error(e, "plan set-up stream");
+}
+
 static bool is_pow2(int v) { return v > 0 && (v & (v - 1)) == 0; }
 
 // A geometry the correlation reads windows with: positive sizes and every
@@ -417,6 +426,10 @@ int piv_plan_create(const piv_config* cfg, piv_plan** out) {
   if (cfg->mask) p->host_mask.assign(cfg->mask, cfg->mask + hw);
   p->st.resize(cfg->n_iters);
   size_t max_mn = 0;
+  // Everything that creation puts into device memory goes through a stream of
+  // its own: the caller's streams (the legacy stream among them, which every
+  // blocking stream waits for) are neither waited for nor held up.
+  cudaStream_t setup = nullptr;
   for (int k = 0; k < cfg->n_iters && rc == PIV_OK; ++k) {
     const piv_iteration& it = p->iters[k];
     IterState& s = p->st[k];
@@ -436,6 +449,7 @@ int piv_plan_create(const piv_config* cfg, piv_plan** out) {
     const size_t cnt = s.mn * P;
     if ((rc = plan_alloc(p, &s.u_corr, cnt * tsz))) break;
     if ((rc = plan_alloc(p, &s.v_corr, cnt * tsz))) break;
+    if (!setup && (rc = setup_stream(&setup))) break;
     if (k > 0) {
       if ((rc = plan_alloc_t(p, &s.up, cnt))) break;
       if ((rc = plan_alloc_t(p, &s.vp, cnt))) break;
@@ -447,7 +461,7 @@ int piv_plan_create(const piv_config* cfg, piv_plan** out) {
       if ((rc = plan_alloc_t(p, &s.v_out, cnt))) break;
       if (s.mn >= 2) {
         if ((rc = plan_alloc(p, &s.smooth_tables, smooth_tables_bytes(s.g.m, s.g.n)))) break;
-        if ((rc = smooth_tables_build(s.g.m, s.g.n, s.smooth_tables, nullptr))) break;
+        if ((rc = smooth_tables_build(s.g.m, s.g.n, s.smooth_tables, setup))) break;
       }
     } else {
       s.u_out = s.u_rep;
@@ -457,7 +471,7 @@ int piv_plan_create(const piv_config* cfg, piv_plan** out) {
     if ((rc = plan_alloc_t(p, &s.val, cnt))) break;
     if ((rc = plan_alloc_t(p, &s.smooth_p, (size_t)P))) break;
     if ((rc = plan_alloc_t(p, &s.smooth_flags, (size_t)P))) break;
-    cudaMemset(s.smooth_flags, 0, sizeof(int) * P);
+    cudaMemsetAsync(s.smooth_flags, 0, sizeof(int) * P, setup);
     if ((rc = plan_alloc_t(p, &s.peak_i, cnt))) break;
     if ((rc = plan_alloc_t(p, &s.peak_j, cnt))) break;
     if ((rc = plan_alloc_t(p, &s.near_tie, cnt))) break;
@@ -472,7 +486,7 @@ int piv_plan_create(const piv_config* cfg, piv_plan** out) {
           fm[(size_t)i * s.g.n + j] = cfg->mask[(size_t)y * W + x] ? 1 : 0;
         }
       if ((rc = plan_alloc_t(p, &s.field_mask, s.mn))) break;
-      cudaMemcpy(s.field_mask, fm.data(), s.mn, cudaMemcpyHostToDevice);
+      cudaMemcpyAsync(s.field_mask, fm.data(), s.mn, cudaMemcpyHostToDevice, setup);
     }
     const size_t cs = correlate_fft_scratch_bytes(it.fft_size, cfg->dtype);
     if (cs > p->corr_scratch_bytes) p->corr_scratch_bytes = cs;
@@ -487,7 +501,7 @@ int piv_plan_create(const piv_config* cfg, piv_plan** out) {
   if (rc == PIV_OK && p->any_cubic) rc = plan_alloc_t(p, &p->coef, 2 * (size_t)P * chw);
   if (rc == PIV_OK && cfg->mask) {
     rc = plan_alloc_t(p, &p->frame_mask, hw);
-    if (rc == PIV_OK) cudaMemcpy(p->frame_mask, cfg->mask, hw, cudaMemcpyHostToDevice);
+    if (rc == PIV_OK) cudaMemcpyAsync(p->frame_mask, cfg->mask, hw, cudaMemcpyHostToDevice, setup);
   }
   if (rc == PIV_OK) rc = plan_alloc(p, &p->corr_scratch, p->corr_scratch_bytes);
   if (rc == PIV_OK) rc = plan_alloc(p, &p->rep_scratch, replace_scratch_bytes(1, (int)max_mn, P));
@@ -500,11 +514,11 @@ int piv_plan_create(const piv_config* cfg, piv_plan** out) {
   if (rc == PIV_OK) rc = plan_alloc_t(p, &p->rms_stats, 4 * (size_t)P);
   if (rc == PIV_OK) {
     rc = plan_alloc_t(p, &p->status, 1);
-    if (rc == PIV_OK) cudaMemset(p->status, 0, sizeof(int));
+    if (rc == PIV_OK) cudaMemsetAsync(p->status, 0, sizeof(int), setup);
   }
   if (rc == PIV_OK) {
     rc = plan_alloc_t(p, &p->tie_counts, (size_t)cfg->n_iters);
-    if (rc == PIV_OK) cudaMemset(p->tie_counts, 0, sizeof(int) * cfg->n_iters);
+    if (rc == PIV_OK) cudaMemsetAsync(p->tie_counts, 0, sizeof(int) * cfg->n_iters, setup);
   }
   bool refine_buffers = cfg->dft_mode == PIV_DFT_TENSOR_REFINED;
   for (int k = 0; k < cfg->n_iters; ++k)  // the split form's 64-px passes take the refined path
@@ -523,10 +537,11 @@ int piv_plan_create(const piv_config* cfg, piv_plan** out) {
     if (rc == PIV_OK) rc = plan_alloc_t(p, &p->u_final, cnt);
     if (rc == PIV_OK) rc = plan_alloc_t(p, &p->v_final, cnt);
   }
-  // The smoothing tables are complete before a run on any stream reads them.
-  if (rc == PIV_OK && cfg->n_iters > 1) {
-    const cudaError_t e = cudaStreamSynchronize(nullptr);
-    if (e != cudaSuccess) rc = set_cuda_error(e, "plan tables");
+  // Tables, masks and zeros are complete before a run on any stream reads them.
+  if (setup) {
+    const cudaError_t e = cudaStreamSynchronize(setup);
+    if (rc == PIV_OK && e != cudaSuccess) rc = set_cuda_error(e, "plan set-up");
+    cudaStreamDestroy(setup);
   }
   if (rc != PIV_OK) {
     piv_plan_destroy(p);

@@ -168,9 +168,13 @@ static int build_tables(int m, int n, const SmoothTables& t, cudaStream_t stream
   const long long entries = (long long)m * m + (long long)n * n;
   const long long mat = (entries + kTabThreads - 1) / kTabThreads;
   const long long lam_cols = (n + kTabThreads - 1) / kTabThreads, lam_rows = (m + kLamRows - 1) / kLamRows;
-  k_smooth_tables<<<(unsigned)(mat + lam_cols * lam_rows), kTabThreads, 0, stream>>>(m, n, t, sc, (int)mat,
-                                                                                     (int)lam_cols);
-  return check("k_smooth_tables");
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(mat + lam_cols * lam_rows));
+  cfg.blockDim = dim3(kTabThreads);
+  cfg.stream = stream;
+  // The launch's own status: an error that the caller has left behind is not the tables'.
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, k_smooth_tables, m, n, t, sc, (int)mat, (int)lam_cols);
+  return e == cudaSuccess ? PIV_OK : set_cuda_error(e, "k_smooth_tables");
 }
 
 // Tables that a plan keeps (every table, whichever path its runs take).
