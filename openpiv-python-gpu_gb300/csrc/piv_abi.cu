@@ -809,8 +809,8 @@ static int run_post(piv_plan* p, int k, RunCtx& x, cudaStream_t s) {
   return PIV_OK;
 }
 
-// Device results of a run in one launch (four copies on the stream took 4 us
-// each, whatever their size).
+// Results of a run in memory of the plan's device in one launch (four copies on
+// the stream took 4 us each, whatever their size).
 __global__ void k_results(int count, const double* __restrict__ u, const double* __restrict__ v,
                           const uint8_t* __restrict__ val, const uint8_t* __restrict__ out, double* uo, double* vo,
                           uint8_t* valo, uint8_t* outo) {
@@ -820,6 +820,26 @@ __global__ void k_results(int count, const double* __restrict__ u, const double*
   vo[t] = v[t];
   if (valo) valo[t] = val[t];
   if (outo) outo[t] = out[t];
+}
+
+// Whether k_results may store to every output (NULL: none): fields on 8-byte
+// boundaries, in memory of the plan's device. Other memory (another device's,
+// which a kernel reaches only with peer access, pinned or managed memory) takes
+// copies.
+static bool results_on_device(const piv_plan* p, const double* u, const double* v, const uint8_t* val,
+                              const uint8_t* out) {
+  if (((uintptr_t)u | (uintptr_t)v) & 7) return false;
+  const void* ptrs[4] = {u, v, val, out};
+  for (const void* q : ptrs) {
+    cudaPointerAttributes at;
+    if (!q) continue;
+    if (cudaPointerGetAttributes(&at, q) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    if (!memory_of_device(at, p->device)) return false;
+  }
+  return true;
 }
 
 static int run_end(piv_plan* p, RunCtx& x, double* u, double* v, uint8_t* val_locations, uint8_t* outliers,
@@ -834,7 +854,7 @@ static int run_end(piv_plan* p, RunCtx& x, double* u, double* v, uint8_t* val_lo
     ru = p->u_final;
     rv = p->v_final;
   }
-  if (!outputs_on_host && (((uintptr_t)u | (uintptr_t)v) & 7) == 0) {
+  if (!outputs_on_host && results_on_device(p, u, v, val_locations, outliers)) {
     k_results<<<(unsigned)((cnt + 255) / 256), 256, 0, s>>>(cnt, ru, rv, last.val0, p->outliers, u, v, val_locations,
                                                            outliers);
     PIV_TRY(cuda_ok(cudaGetLastError(), "k_results"));

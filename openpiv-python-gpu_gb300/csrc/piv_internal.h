@@ -13,6 +13,11 @@ namespace piv {
 int set_error(int code, const char* fmt, ...);
 int set_cuda_error(cudaError_t e, const char* what);
 
+// Whether the memory that `at` describes is `device`'s own.
+inline bool memory_of_device(const cudaPointerAttributes& at, int device) {
+  return at.type == cudaMemoryTypeDevice && at.device == device;
+}
+
 // Arguments of one correlation pass over n_pairs frame pairs.
 // One frame geometry of a multi-geometry correlation launch: the windows of
 // n_pairs pairs of one frame size, global windows [win0, win0 + n_pairs m n)
