@@ -26,6 +26,7 @@
 
 #include "piv_common.cuh"
 #include "piv_internal.h"
+#include "piv_scratch_pool.h"
 
 namespace piv {
 
@@ -66,41 +67,32 @@ int sm_count() {
 // trimmed when a plan is destroyed and when a plan's allocation fails.
 // Allocations made while `s` is captured become the graph's own, as before.
 static constexpr unsigned long long kPoolKeep = 64ull << 20;
-static std::mutex g_pool_mu;
-static cudaMemPool_t g_pools[64] = {nullptr};
-
-static cudaMemPool_t scratch_pool() {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-  std::lock_guard<std::mutex> lock(g_pool_mu);
-  if (!g_pools[dev]) {
+struct PoolApi {
+  using Pool = cudaMemPool_t;
+  static bool device(int* dev) { return cudaGetDevice(dev) == cudaSuccess; }
+  static bool create(int dev, Pool* pool) {
     cudaMemPoolProps props = {};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = dev;
-    cudaMemPool_t pool = nullptr;
     unsigned long long keep = kPoolKeep;
-    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+    if (cudaMemPoolCreate(pool, &props) != cudaSuccess) {
       cudaGetLastError();
-      return nullptr;
+      return false;
     }
-    cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    g_pools[dev] = pool;
+    cudaMemPoolSetAttribute(*pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    return true;
   }
-  return g_pools[dev];
-}
-
-static void scratch_pool_trim() {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
-  std::lock_guard<std::mutex> lock(g_pool_mu);
-  if (g_pools[dev] && cudaMemPoolTrimTo(g_pools[dev], 0) != cudaSuccess) cudaGetLastError();
-}
+  static void trim(Pool pool) {
+    if (cudaMemPoolTrimTo(pool, 0) != cudaSuccess) cudaGetLastError();
+  }
+};
+static ScratchPools<PoolApi> g_pools;
 
 static cudaError_t scratch_alloc(void** ptr, size_t bytes, cudaStream_t s) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
-    cudaMemPool_t pool = scratch_pool();
+    cudaMemPool_t pool = g_pools.get();
     if (pool && cudaMallocFromPoolAsync(ptr, bytes, pool, s) == cudaSuccess) return cudaSuccess;
   }
   cudaGetLastError();
@@ -251,7 +243,7 @@ static int plan_alloc(piv_plan* p, void** ptr, size_t bytes) {
   cudaError_t e = cudaMalloc(ptr, bytes);
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
-    scratch_pool_trim();
+    g_pools.trim(p->device);
     e = cudaMalloc(ptr, bytes);
   }
   if (e != cudaSuccess) {
@@ -370,8 +362,8 @@ void piv_plan_destroy(piv_plan* p) {
   }
   for (auto e : p->event_pool) cudaEventDestroy(e);
   for (void* a : p->allocs) cudaFree(a);
+  g_pools.trim(p->device);
   delete p;
-  scratch_pool_trim();
 }
 
 int piv_plan_set_timing(piv_plan* p, int enable) {

@@ -1,0 +1,23 @@
+// Host-side harness of the scratch pools' bookkeeping (csrc/piv_scratch_pool.h)
+// with a fake runtime, for the CPU tests.
+#include "../openpiv-python-gpu_gb300/csrc/piv_scratch_pool.h"
+
+namespace {
+int g_device = 0, g_pools = 0, g_trimmed[64] = {0};
+bool g_fail = false;
+struct Fake {
+  using Pool = int;  // 1, 2, ... in the order of creation
+  static bool device(int* dev) { return *dev = g_device, true; }
+  static bool create(int, Pool* pool) { return g_fail ? false : (*pool = ++g_pools, true); }
+  static void trim(Pool pool) { ++g_trimmed[pool]; }
+};
+piv::ScratchPools<Fake> g_set;
+}  // namespace
+
+extern "C" {
+void fake_device(int dev) { g_device = dev; }
+void fake_fail(int fail) { g_fail = fail != 0; }
+int fake_trimmed(int pool) { return g_trimmed[pool]; }
+int pool_get() { return g_set.get(); }
+void pool_trim(int dev) { g_set.trim(dev); }
+}
