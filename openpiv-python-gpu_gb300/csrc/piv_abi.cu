@@ -61,16 +61,51 @@ int sm_count() {
 }
 
 // Scratch of the stage entry points, stream-ordered from a pool of this
-// library's own per device. The device's default pool gives its memory back at
-// every synchronisation, so each call after one mapped its scratch anew (250
-// us of a 360 us correlation). This pool keeps up to kPoolKeep bytes; it is
-// trimmed when a plan is destroyed and when a plan's allocation fails.
-// Allocations made while `s` is captured become the graph's own, as before.
+// library's own per device (per context: ScratchPools). The device's default
+// pool gives its memory back at every synchronisation, so each call after one
+// mapped its scratch anew (250 us of a 360 us correlation). This pool keeps up
+// to kPoolKeep bytes; it is trimmed when a plan is destroyed and when a plan's
+// allocation fails. Allocations made while `s` is captured become the graph's
+// own, as before.
 static constexpr unsigned long long kPoolKeep = 64ull << 20;
 struct PoolApi {
   using Pool = cudaMemPool_t;
-  static bool device(int* dev) { return cudaGetDevice(dev) == cudaSuccess; }
-  static bool create(int dev, Pool* pool) {
+  // Makes `dev` current while it lives.
+  struct OnDevice {
+    int before = 0;
+    bool moved = false;
+    explicit OnDevice(int dev) {
+      if (cudaGetDevice(&before) == cudaSuccess && before != dev) moved = cudaSetDevice(dev) == cudaSuccess;
+    }
+    ~OnDevice() {
+      if (moved) cudaSetDevice(before);
+    }
+  };
+  // Id of the current context, made current by the runtime if need be; 0: none.
+  static unsigned long long context() {
+    using GetId = int (*)(void*, unsigned long long*);  // cuCtxGetId
+    static const GetId get_id = [] {
+      void* f = nullptr;
+      cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+      if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+          found != cudaDriverEntryPointSuccess) {
+        cudaGetLastError();
+        f = nullptr;
+      }
+      return reinterpret_cast<GetId>(f);
+    }();
+    unsigned long long id = 0;
+    if (!get_id) return 0;
+    if (get_id(nullptr, &id) == 0) return id;
+    if (cudaFree(nullptr) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    return get_id(nullptr, &id) == 0 ? id : 0;
+  }
+  static bool create(Pool* pool) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
     cudaMemPoolProps props = {};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;

@@ -3,12 +3,17 @@
 #include "../openpiv-python-gpu_gb300/csrc/piv_scratch_pool.h"
 
 namespace {
-int g_device = 0, g_pools = 0, g_trimmed[64] = {0};
+int g_device = 0, g_resets[64] = {0}, g_pools = 0, g_trimmed[256] = {0};
 bool g_fail = false;
 struct Fake {
   using Pool = int;  // 1, 2, ... in the order of creation
-  static bool device(int* dev) { return *dev = g_device, true; }
-  static bool create(int, Pool* pool) { return g_fail ? false : (*pool = ++g_pools, true); }
+  struct OnDevice {
+    int before = g_device;
+    explicit OnDevice(int dev) { g_device = dev; }
+    ~OnDevice() { g_device = before; }
+  };
+  static unsigned long long context() { return 1 + g_device + 64ull * g_resets[g_device]; }
+  static bool create(Pool* pool) { return g_fail ? false : (*pool = ++g_pools, true); }
   static void trim(Pool pool) { ++g_trimmed[pool]; }
 };
 piv::ScratchPools<Fake> g_set;
@@ -16,6 +21,7 @@ piv::ScratchPools<Fake> g_set;
 
 extern "C" {
 void fake_device(int dev) { g_device = dev; }
+void fake_reset(int dev) { ++g_resets[dev]; }
 void fake_fail(int fail) { g_fail = fail != 0; }
 int fake_trimmed(int pool) { return g_trimmed[pool]; }
 int pool_get() { return g_set.get(); }

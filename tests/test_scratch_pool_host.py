@@ -39,3 +39,23 @@ def test_a_pool_per_device_and_its_own_trim(pools):
     pools.pool_trim(5)  # a device without a pool
     assert (pools.fake_trimmed(first), pools.fake_trimmed(other)) == (1, 1)
     assert pools.pool_get() == first
+
+
+def test_a_device_reset_ends_its_pool(pools):
+    first = pools.pool_get()
+    pools.fake_device(1)
+    other = pools.pool_get()
+    pools.fake_reset(0)
+    assert pools.pool_get() == other
+    pools.pool_trim(0)  # the old handle is gone with its context
+    assert pools.fake_trimmed(first) == 0
+    pools.fake_device(0)
+    second = pools.pool_get()
+    assert second not in (0, first, other) and pools.pool_get() == second
+    pools.pool_trim(0)
+    assert (pools.fake_trimmed(first), pools.fake_trimmed(second), pools.fake_trimmed(other)) == (0, 1, 0)
+    made = {first, other, second}
+    for _ in range(100):  # pools without end: none, which sends the call to the device's own pool
+        pools.fake_reset(0)
+        made.add(pools.pool_get())
+    assert 0 in made and len(made) == 64 + 1
