@@ -297,9 +297,10 @@ static constexpr int kDeformRows = 8;                       // image rows per CT
 // apart, and the last one has a point behind it. Sized by the spacing, not for
 // spacing 1 (18.6 KB a CTA): what is left over caches the taps (64 pairs of
 // 1024 x 1024, two passes of k_deform_cubic: 1081 -> 1054 us).
+static int deform_cols(int spacing) { return (kDeformThreads - 1) / spacing + 3; }
+static int deform_rows(int spacing) { return (kDeformRows - 1) / spacing + 3; }
 static size_t deform_smem(int spacing) {
-  const size_t cols = (kDeformThreads - 1) / spacing + 3, rows = (kDeformRows - 1) / spacing + 3;
-  return 2 * cols * rows * sizeof(float);
+  return 2 * (size_t)deform_cols(spacing) * deform_rows(spacing) * sizeof(float);
 }
 
 // One thread per pixel column of an 8-row x 256-pixel block; each thread
@@ -311,8 +312,8 @@ static size_t deform_smem(int spacing) {
 // Launch grid: x over row segments, y over blocks of rows, z over pairs.
 template <typename T>
 __global__ void __launch_bounds__(kDeformThreads) k_deform(DeformArgs a, AxisMap ax, AxisMap ay, T dta, T dtb,
-                                                           int do_a, int do_b) {
-  extern __shared__ float field_s[];  // u, then v: [nr][nc]
+                                                           int do_a, int do_b, int pitch, int plane) {
+  extern __shared__ float field_s[];  // u, then v: [nr][ld]
   __shared__ int s_klo, s_khi;
   const piv_geometry& g = a.geom;
   const int H = g.height, W = g.width;
@@ -329,13 +330,18 @@ __global__ void __launch_bounds__(kDeformThreads) k_deform(DeformArgs a, AxisMap
   const int k_lo = s_klo, k_hi = s_khi;
   const int nc = k_hi - k_lo + 1, nr = r_hi - r_lo + 1;
   float* su = field_s;
-  float* sv = field_s + nr * nc;
+  // Row pitch and size: those of the launch in float32, where they stay out of
+  // the registers (eight pairs of 1024 x 1024, one frame moved: bilinear 55.4 ->
+  // 54.5 us, cubic 79.4 -> 77.4 us); in float64 the CTA's own, which cost less
+  // there (51.5 us for 52.1, one cubic pair).
+  const int ld = sizeof(T) == 4 ? pitch : nc;
+  float* sv = field_s + (sizeof(T) == 4 ? plane : nr * nc);
   const long long fo = (long long)pair * g.m * g.n;
   for (int e = threadIdx.x; e < nr * nc; e += kDeformThreads) {
     const int r = e / nc, c = e % nc;
     const long long q = fo + (long long)(r_lo + r) * g.n + k_lo + c;
-    su[e] = (float)__ldg(a.up + q);
-    sv[e] = (float)__ldg(a.vp + q);
+    su[r * ld + c] = (float)__ldg(a.up + q);
+    sv[r * ld + c] = (float)__ldg(a.vp + q);
   }
   __syncthreads();
   if (j >= W) return;
@@ -360,7 +366,7 @@ __global__ void __launch_bounds__(kDeformThreads) k_deform(DeformArgs a, AxisMap
       continue;
     }
     const AxisWeight wy = axis_weight(i, ay);
-    const int y0r = (wy.i - r_lo) * nc, y1r = ((g.m < 2 ? wy.i : wy.i + 1) - r_lo) * nc;
+    const int y0r = (wy.i - r_lo) * ld, y1r = ((g.m < 2 ? wy.i : wy.i + 1) - r_lo) * ld;
     const float u0 = fmaf(wy.t, su[y1r + c0] - su[y0r + c0], su[y0r + c0]);
     const float u1 = fmaf(wy.t, su[y1r + c1] - su[y0r + c1], su[y0r + c1]);
     const float v0 = fmaf(wy.t, sv[y1r + c0] - sv[y0r + c0], sv[y0r + c0]);
@@ -646,8 +652,9 @@ int deform(const DeformArgs& a, cudaStream_t stream) {
   const AxisMap ax = axis_map(a.geom.search_size, a.geom.x_offset, a.geom.spacing, a.geom.n);
   const AxisMap ay = axis_map(a.geom.search_size, a.geom.y_offset, a.geom.spacing, a.geom.m);
   const size_t smem = deform_smem(a.geom.spacing);
+  const int pitch = deform_cols(a.geom.spacing), plane = pitch * deform_rows(a.geom.spacing);
   if (a.dtype == PIV_DTYPE_F64)
-    k_deform<double><<<grid, kDeformThreads, smem, stream>>>(a, ax, ay, dta, dtb, do_a, do_b);
+    k_deform<double><<<grid, kDeformThreads, smem, stream>>>(a, ax, ay, dta, dtb, do_a, do_b, pitch, plane);
   else if (a.order == 3 && do_a && do_b && a.coef_pad)
     k_deform_cubic<true><<<grid, kDeformThreads, smem, stream>>>(a, ax, ay, (float)dta, (float)dtb);
   else if (a.order == 3 && do_a && do_b)
@@ -667,7 +674,7 @@ int deform(const DeformArgs& a, cudaStream_t stream) {
         k_deform_bilinear<double><<<grid, kDeformThreads, smem, stream>>>(a, ax, ay, (float)dta, (float)dtb);
     }
   else
-    k_deform<float><<<grid, kDeformThreads, smem, stream>>>(a, ax, ay, (float)dta, (float)dtb, do_a, do_b);
+    k_deform<float><<<grid, kDeformThreads, smem, stream>>>(a, ax, ay, (float)dta, (float)dtb, do_a, do_b, pitch, plane);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? PIV_OK : set_cuda_error(e, "k_deform launch");
 }
