@@ -23,6 +23,7 @@
 
 #include <algorithm>
 
+#include "piv_corr_common.cuh"
 #include "piv_fft.cuh"
 #include "piv_internal.h"
 #include "twiddles.h"
@@ -297,30 +298,9 @@ PIV_D void corr_outputs(const CorrArgs& a, const Cplx<T>* buf, const CorrShared<
     const int i = S.pi[w], j = S.pj[w];
     T isp = (T)i, jsp = (T)j;
     if (i > 0 && i < N - 1 && j > 0 && j < N - 1) {
-      T c = corr_at<N, T>(wb, i, j, ss);
-      T cd = corr_at<N, T>(wb, i - 1, j, ss), cu = corr_at<N, T>(wb, i + 1, j, ss);
-      T cl = corr_at<N, T>(wb, i, j - 1, ss), cr = corr_at<N, T>(wb, i, j + 1, ss);
-      const T eps = (T)1e-7;
-      const T half = (T)0.5, two = (T)2;
-      if (a.subpixel == PIV_SUBPIXEL_GAUSSIAN) {
-        if (c > 0 && cd > 0 && cu > 0 && cl > 0 && cr > 0) {
-          c = log(c); cd = log(cd); cu = log(cu); cl = log(cl); cr = log(cr);
-          T di = div_rn(mul_rn(half, sub_rn(cd, cu)), add_rn(add_rn(sub_rn(cd, mul_rn(two, c)), cu), eps));
-          T dj = div_rn(mul_rn(half, sub_rn(cl, cr)), add_rn(add_rn(sub_rn(cl, mul_rn(two, c)), cr), eps));
-          isp = add_rn((T)i, di);
-          jsp = add_rn((T)j, dj);
-        }
-      } else if (a.subpixel == PIV_SUBPIXEL_PARABOLIC) {
-        T di = div_rn(mul_rn(half, sub_rn(cd, cu)), add_rn(add_rn(sub_rn(cd, mul_rn(two, c)), cu), eps));
-        T dj = div_rn(mul_rn(half, sub_rn(cl, cr)), add_rn(add_rn(sub_rn(cl, mul_rn(two, c)), cr), eps));
-        isp = add_rn((T)i, di);
-        jsp = add_rn((T)j, dj);
-      } else {
-        T di = div_rn(sub_rn(cu, cd), add_rn(add_rn(add_rn(cd, c), cu), eps));
-        T dj = div_rn(sub_rn(cr, cl), add_rn(add_rn(add_rn(cl, c), cr), eps));
-        isp = add_rn((T)i, di);
-        jsp = add_rn((T)j, dj);
-      }
+      subpixel_fit<T>(a.subpixel, i, j, corr_at<N, T>(wb, i, j, ss), corr_at<N, T>(wb, i - 1, j, ss),
+                      corr_at<N, T>(wb, i + 1, j, ss), corr_at<N, T>(wb, i, j - 1, ss),
+                      corr_at<N, T>(wb, i, j + 1, ss), isp, jsp);
     }
     T* uo = reinterpret_cast<T*>(a.u);
     T* vo = reinterpret_cast<T*>(a.v);

@@ -18,7 +18,6 @@
 // this): N = 32 136 -> 57 us, N = 64 139 -> 68 us, N = 128 174 -> 90 us.
 #pragma once
 
-#include "piv_corr_common.cuh"
 #include "piv_corr_fft.cuh"
 
 namespace piv {
