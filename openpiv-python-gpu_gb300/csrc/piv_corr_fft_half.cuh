@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(H::NT, H::MIN_CTAS) k_corr_fft_half(CorrArgs a
   for (long long slot = blockIdx.x; slot < total; slot += gridDim.x) {
     const long long g = a.win_list ? (long long)a.win_list[slot] : slot;
     long long base;
-    const bool ok = window_corner(a, g, base);
+    const bool ok = window_corner(a, g, base) || SEARCH;  // the search's passes have no mask
     // The window's pixels, PER per virtual thread, and the means.
     X xa[NV * PER], xb[NV * PER];
     auto elem = [&](int k) { return tid + (k / PER) * NT + (k % PER) * NT0; };
@@ -613,7 +613,7 @@ __global__ void __launch_bounds__(H::NT, H::MIN_CTAS) k_corr_fft_half(CorrArgs a
         a.peak_j[g] = S.pj[0];
         if (a.near_tie) a.near_tie[g] = 0;
         // The values that the window's candidates reach (open windows only).
-        cand_from = !ok || (!bad && best - S.means[0] > gap) ? INFINITY : (bad ? -INFINITY : best - gap);
+        cand_from = !bad && best - S.means[0] > gap ? INFINITY : (bad ? -INFINITY : best - gap);
         cand_n = 0;
       }
       __syncthreads();
@@ -686,7 +686,7 @@ __global__ void __launch_bounds__(32 * kWarpFftWarps, kWarpFftCtas) k_corr_fft_w
        slot += (long long)gridDim.x * kWarpFftWarps) {
     const long long g = a.win_list ? (long long)a.win_list[slot] : slot;
     long long base;
-    const bool ok = window_corner(a, g, base);
+    const bool ok = window_corner(a, g, base) || SEARCH;  // the search's passes have no mask
     // Pixels e = lane + 32 v + 128 q: the sums of the general kernel's 128
     // threads (pairs e, e + 128), then its four warps in order.
     X xa[8], xb[8];
@@ -840,7 +840,7 @@ __global__ void __launch_bounds__(32 * kWarpFftWarps, kWarpFftCtas) k_corr_fft_w
         a.peak_j[g] = top.at % N;
         if (a.near_tie) a.near_tie[g] = 0;
       }
-      if (ok && (bad || !(top.best - top.second > gap))) {
+      if (bad || !(top.best - top.second > gap)) {
         const float from = bad ? INFINITY : top.best - gap;
         int count = 0, at[kCandMax];
         // Candidates in map order, counted by every lane.

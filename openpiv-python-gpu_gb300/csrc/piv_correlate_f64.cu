@@ -186,11 +186,11 @@ __global__ void __launch_bounds__(32 * kFitWarps) k_resolve64(CorrArgs a) {
   }
 }
 
-// Fit and displacement of every window from its peak: each warp sums
-// kFitPerWarp windows, then one warp fits all of the CTA's, a window per lane
-// (a fit is some 500 float64 instructions, whose cost does not depend on how
-// many lanes take part: with one fit per warp the kernel took 81 us for 3,871
-// windows of 32 px, so it takes 33 us).
+// Fit and displacement of every window (none is masked) from its peak: each
+// warp sums kFitPerWarp windows, then one warp fits all of the CTA's, a window
+// per lane (a fit is some 500 float64 instructions, whose cost does not depend
+// on how many lanes take part: with one fit per warp the kernel took 81 us for
+// 3,871 windows of 32 px, so it takes 33 us).
 static constexpr int kFitPerWarp = 2;
 static_assert(kFitWarps * kFitPerWarp == 32, "one window per lane of the fitting warp");
 template <typename P>
@@ -211,8 +211,9 @@ __global__ void __launch_bounds__(32 * kFitWarps) k_fit64(CorrArgs a) {
     for (int k = 0; k < kFitPerWarp; ++k) {
       const int slot = warp * kFitPerWarp + k;
       const long long g = g0 + slot;
+      if (g >= total || !lags(g, di, dj)) continue;
       long long base;
-      if (g >= total || !window_corner(a, g, base) || !lags(g, di, dj)) continue;
+      window_corner(a, g, base);
       LagSums<P, 5> sums;
       lag_sums<P, 5>(reinterpret_cast<const P*>(a.frame_a) + base, reinterpret_cast<const P*>(a.frame_b) + base,
                      a.width, a.ss, di, dj, sums);
@@ -221,17 +222,16 @@ __global__ void __launch_bounds__(32 * kFitWarps) k_fit64(CorrArgs a) {
     __syncthreads();
     const long long g = g0 + lane;
     if (warp == 0 && g < total) {
-      long long base;
-      const bool ok = window_corner(a, g, base), inner = lags(g, di, dj);
+      const bool inner = lags(g, di, dj);
       const int pi = a.peak_i[g], pj = a.peak_j[g];
       double isp = (double)pi, jsp = (double)pj, c[5];
-      if (ok && inner) {
+      if (inner) {
 #pragma unroll
         for (int k = 0; k < 5; ++k) c[k] = sums_s[lane].value(k, a.ss, di[k], dj[k]);
         subpixel_fit<double>(a.subpixel, pi, pj, c[0], c[1], c[2], c[3], c[4], isp, jsp);
       }
-      reinterpret_cast<double*>(a.u)[g] = ok ? sub_rn(jsp, (double)(n / 2)) : NAN;
-      reinterpret_cast<double*>(a.v)[g] = ok ? sub_rn(isp, (double)(n / 2)) : NAN;
+      reinterpret_cast<double*>(a.u)[g] = sub_rn(jsp, (double)(n / 2));
+      reinterpret_cast<double*>(a.v)[g] = sub_rn(isp, (double)(n / 2));
     }
     __syncthreads();
   }
