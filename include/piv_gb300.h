@@ -144,7 +144,9 @@ int piv_plan_workspace_bytes(const piv_plan* plan, size_t* bytes);
  * memory are queued on `stream` and the call returns at once (the caller
  * synchronises the stream before reading them: lets a caller upload the next
  * batch while this one runs), otherwise (device outputs) it returns without
- * synchronising. */
+ * synchronising. Device outputs may lie in memory of another GPU or in pinned
+ * host memory: a kernel stores them only where all of them are memory of the
+ * plan's device, other memory is copied to. */
 int piv_plan_run(piv_plan* plan, int n_pairs, const void* frames_a, const void* frames_b, int frames_on_host,
                  double* u, double* v, uint8_t* val_locations, uint8_t* outliers, int outputs_on_host,
                  void* stream);

@@ -237,7 +237,7 @@ PIV_D void st_cluster(double* p, unsigned rank, double v) {
 // CTAs per pair: the largest power of two up to 8 (the portable cluster size)
 // that keeps every CTA on an SM of its own (with more pairs than that the
 // float64 pipes are busy anyway). Measured: one pair's two GCV searches of a
-// three-pass 1024 x 1024 run 396 -> 157 us with 8 CTAs, those of 64 pairs
+// three-pass 1024 x 1024 run 396 -> 139 us with 8 CTAs, those of 64 pairs
 // 230 -> 86 us with 2.
 static int cluster_size(int n_pairs) {
   int c = 1;
@@ -698,7 +698,7 @@ PIV_D int smooth_flags(bool is_auto, double p, double pmin, double pmax, bool la
 // float64 units of an SM work.
 // Bound by the float64 pipe and by the latency of the search's steps. One
 // score at a time on one CTA, with the scan in ten passes, took 396 us for
-// the 31 x 31 and 63 x 63 fields of one 1024 x 1024 pair; this takes 157 us.
+// the 31 x 31 and 63 x 63 fields of one 1024 x 1024 pair; this takes 139 us.
 template <int SETS>
 __global__ void __launch_bounds__(kVT)
 k_gcv(int m, int n, int c, double rmn, const double* __restrict__ fd, double* __restrict__ f2, float* __restrict__ f2f,
