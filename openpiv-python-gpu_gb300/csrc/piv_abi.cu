@@ -26,7 +26,7 @@
 
 #include "piv_common.cuh"
 #include "piv_internal.h"
-#include "piv_scratch_pool.h"
+#include "piv_per_context.h"
 
 namespace piv {
 
@@ -60,16 +60,8 @@ int sm_count() {
   return counts[dev];
 }
 
-// Scratch of the stage entry points, stream-ordered from a pool of this
-// library's own per device (per context: ScratchPools). The device's default
-// pool gives its memory back at every synchronisation, so each call after one
-// mapped its scratch anew (250 us of a 360 us correlation). This pool keeps up
-// to kPoolKeep bytes; it is trimmed when a plan is destroyed and when a plan's
-// allocation fails. Allocations made while `s` is captured become the graph's
-// own, as before.
-static constexpr unsigned long long kPoolKeep = 64ull << 20;
-struct PoolApi {
-  using Pool = cudaMemPool_t;
+// The contexts of this process's devices (PerContext).
+struct Contexts {
   // Makes `dev` current while it lives.
   struct OnDevice {
     int before = 0;
@@ -103,7 +95,19 @@ struct PoolApi {
     }
     return get_id(nullptr, &id) == 0 ? id : 0;
   }
-  static bool create(Pool* pool) {
+};
+
+// Scratch of the stage entry points, stream-ordered from a pool of this
+// library's own per device (per context: PerContext). The device's default
+// pool gives its memory back at every synchronisation, so each call after one
+// mapped its scratch anew (250 us of a 360 us correlation). This pool keeps up
+// to kPoolKeep bytes; it is trimmed when a plan is destroyed and when a plan's
+// allocation fails. Allocations made while `s` is captured become the graph's
+// own, as before.
+static constexpr unsigned long long kPoolKeep = 64ull << 20;
+struct PoolApi : Contexts {
+  using Value = cudaMemPool_t;
+  static bool create(Value* pool) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return false;
     cudaMemPoolProps props = {};
@@ -118,11 +122,15 @@ struct PoolApi {
     cudaMemPoolSetAttribute(*pool, cudaMemPoolAttrReleaseThreshold, &keep);
     return true;
   }
-  static void trim(Pool pool) {
-    if (cudaMemPoolTrimTo(pool, 0) != cudaSuccess) cudaGetLastError();
-  }
 };
-static ScratchPools<PoolApi> g_pools;
+static PerContext<PoolApi> g_pools;
+
+// Gives back the idle memory of device `dev`'s pool.
+static void scratch_pool_trim(int dev) {
+  g_pools.with(dev, [](cudaMemPool_t pool) {
+    if (cudaMemPoolTrimTo(pool, 0) != cudaSuccess) cudaGetLastError();
+  });
+}
 
 static cudaError_t scratch_alloc(void** ptr, size_t bytes, cudaStream_t s) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -278,7 +286,7 @@ static int plan_alloc(piv_plan* p, void** ptr, size_t bytes) {
   cudaError_t e = cudaMalloc(ptr, bytes);
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
-    g_pools.trim(p->device);
+    scratch_pool_trim(p->device);
     e = cudaMalloc(ptr, bytes);
   }
   if (e != cudaSuccess) {
@@ -298,14 +306,18 @@ static int plan_alloc_t(piv_plan* p, Ptr** ptr, size_t count) {
   return rc;
 }
 
-// A stream for a plan's set-up, which waits for no other stream and goes ahead
-// of queued work of lower priority.
-static int setup_stream(cudaStream_t* stream) {
-  int least = 0, greatest = 0;
-  cudaDeviceGetStreamPriorityRange(&least, &greatest);
-  const cudaError_t e = cudaStreamCreateWithPriority(stream, cudaStreamNonBlocking, greatest);
-  return e == cudaSuccess ? PIV_OK : set_cuda_error(e, "plan set-up stream");
-}
+// The stream of plans' set-up, which waits for no other stream and goes ahead
+// of queued work of lower priority. One per context, shared by all threads (one
+// made for every plan: 143 us to create a plan of one pass, with this 134 us).
+struct SetupApi : Contexts {
+  using Value = cudaStream_t;
+  static bool create(Value* stream) {
+    int least = 0, greatest = 0;
+    cudaDeviceGetStreamPriorityRange(&least, &greatest);
+    return cudaStreamCreateWithPriority(stream, cudaStreamNonBlocking, greatest) == cudaSuccess;
+  }
+};
+static PerContext<SetupApi> g_setup;
 
 static bool is_pow2(int v) { return v > 0 && (v & (v - 1)) == 0; }
 
@@ -397,7 +409,7 @@ void piv_plan_destroy(piv_plan* p) {
   }
   for (auto e : p->event_pool) cudaEventDestroy(e);
   for (void* a : p->allocs) cudaFree(a);
-  g_pools.trim(p->device);
+  scratch_pool_trim(p->device);
   delete p;
 }
 
@@ -453,10 +465,11 @@ int piv_plan_create(const piv_config* cfg, piv_plan** out) {
   if (cfg->mask) p->host_mask.assign(cfg->mask, cfg->mask + hw);
   p->st.resize(cfg->n_iters);
   size_t max_mn = 0;
-  // Everything that creation puts into device memory goes through a stream of
-  // its own: the caller's streams (the legacy stream among them, which every
+  // Everything that creation puts into device memory goes through the set-up
+  // stream: the caller's streams (the legacy stream among them, which every
   // blocking stream waits for) are neither waited for nor held up.
   cudaStream_t setup = nullptr;
+  bool own_setup = false;  // where no stream is kept for the context
   for (int k = 0; k < cfg->n_iters && rc == PIV_OK; ++k) {
     const piv_iteration& it = p->iters[k];
     IterState& s = p->st[k];
@@ -476,7 +489,10 @@ int piv_plan_create(const piv_config* cfg, piv_plan** out) {
     const size_t cnt = s.mn * P;
     if ((rc = plan_alloc(p, &s.u_corr, cnt * tsz))) break;
     if ((rc = plan_alloc(p, &s.v_corr, cnt * tsz))) break;
-    if (!setup && (rc = setup_stream(&setup))) break;
+    if (!setup && !(setup = g_setup.get())) {
+      own_setup = SetupApi::create(&setup);
+      if (!own_setup && (rc = set_cuda_error(cudaGetLastError(), "plan set-up stream"))) break;
+    }
     if (k > 0) {
       if ((rc = plan_alloc_t(p, &s.up, cnt))) break;
       if ((rc = plan_alloc_t(p, &s.vp, cnt))) break;
@@ -568,7 +584,7 @@ int piv_plan_create(const piv_config* cfg, piv_plan** out) {
   if (setup) {
     const cudaError_t e = cudaStreamSynchronize(setup);
     if (rc == PIV_OK && e != cudaSuccess) rc = set_cuda_error(e, "plan set-up");
-    cudaStreamDestroy(setup);
+    if (own_setup) cudaStreamDestroy(setup);
   }
   if (rc != PIV_OK) {
     piv_plan_destroy(p);

@@ -1,4 +1,5 @@
-"""Bookkeeping of the library's scratch pools, with a fake runtime (no GPU)."""
+"""Bookkeeping of the objects kept per context (scratch pools, set-up streams),
+with a fake runtime (no GPU)."""
 
 import ctypes
 import os
@@ -17,7 +18,7 @@ def pools(tmp_path):
         pytest.skip("nvcc not available")
     out = str(tmp_path / "libpools.so")
     r = subprocess.run([nvcc, "-std=c++17", "-shared", "-Xcompiler", "-fPIC",
-                        os.path.join(HERE, "scratch_pool_harness.cu"), "-o", out], capture_output=True, text=True)
+                        os.path.join(HERE, "per_context_harness.cu"), "-o", out], capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
     return ctypes.CDLL(out)
 
